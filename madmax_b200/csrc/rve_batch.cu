@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "rve_batch_kernel.cuh"
+#include "rve_modes_host.h"
 
 namespace sp {
 
@@ -214,7 +215,28 @@ struct sp_batch_s {
   size_t bytes = 0;
   TuneRecord tune;  // the autotuner's trial (tune.n == 0: shape fixed by the caller)
   int tune_slots = 0;  // work spaces allocated while the autotuner runs
+  // 512 x 1 FP32 stencil under affine conditions: RVEs the element-mode
+  // kernel takes, in one launch per class; `rest` keep k_batch
+  std::vector<MeshGeo> geo;      // per RVE
+  std::vector<int> cls;          // per RVE: element-mode class or -1
+  ModesPlan modes;
+  int nrest = 0;                 // RVEs of k_batch (d_rest: their order)
+  int *d_rest = nullptr, *d_mcount = nullptr;
+  unsigned *d_done = nullptr;
+  sp_solve_info *d_tinfo = nullptr;
+  ModesCommon mc;
 };
+
+// the shape whose FP32 affine stencil solves run the element-mode kernel
+static bool uses_modes(const sp_batch_opts &o, const Shape &s) {
+  return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op == SP_OP_STENCIL &&
+         o.precision == SP_PREC_MIXED;
+}
+
+static void split_rves(const sp_batch *b, const std::vector<int> &order, std::vector<int> *in,
+                       std::vector<int> *rest) {
+  for (int i : order) (b->cls[i] >= 0 ? in : rest)->push_back(i);
+}
 
 // Time every candidate shape on the same sample of the batch: 2 G RVEs, G
 // the largest candidate grid, taken at even steps through the largest-first
@@ -257,6 +279,40 @@ static int tune_trial(sp_batch *b, const std::vector<Shape> &cands, const std::v
     if (grid / cands[c].cluster > b->tune_slots) continue;  // work spaces sized for fewer
     BatchParams P = b->P;
     P.order = d_trial;
+    if (uses_modes(b->o, cands[c])) {
+      // the element-mode kernel on the RVEs it takes, k_batch on the rest
+      std::vector<int> in, rest;
+      ModesPlan mk;
+      split_rves(b, sample, &in, &rest);
+      std::stable_sort(in.begin(), in.end(),
+                       [&](int x, int y) { return b->geo[x].ndof > b->geo[y].ndof; });
+      rc = modes_plan(in, b->cls, b->geo, b->nrhs, d, &mk);
+      if (!rc) rc = modes_launch(mk, b->mc, b->d_mcount, s, true);
+      P.nrve = (int)rest.size();
+      if (!rc && !rest.empty() &&
+          (cudaMemcpyAsync(d_trial, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
+           cudaMemsetAsync(b->d_counter, 0, sizeof(int), s)))
+        rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: autotuner upload failed");
+      if (!rc && cudaEventRecord(e0, s))
+        rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: autotuner launch failed");
+      if (!rc) rc = modes_launch(mk, b->mc, b->d_mcount, s);
+      if (!rc && !rest.empty()) rc = launch_shape(fn, cands[c], grid, dyn, s, P);
+      float ms = 0.f;
+      if (!rc && (cudaEventRecord(e1, s) || cudaEventSynchronize(e1) || cudaEventElapsedTime(&ms, e0, e1)))
+        rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: autotuner timing failed");
+      modes_free(&mk);
+      if (!rc && cudaMemcpyAsync(d_trial, sample.data(), T * sizeof(int), cudaMemcpyHostToDevice, s))
+        rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: autotuner upload failed");
+      if (rc) break;
+      const int k = rec->n++;
+      rec->shape[k] = cands[c];
+      rec->rate[k] = wsum / std::max(ms, 1e-3f);
+      if (rec->rate[k] > best) {
+        best = rec->rate[k];
+        rec->best = k;
+      }
+      continue;
+    }
     if (cudaMemsetAsync(b->d_counter, 0, sizeof(int), s)) {
       rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: autotuner upload failed");
       break;
@@ -312,8 +368,10 @@ extern "C" int sp_batch_destroy(sp_batch *b) {
   if (!b) return SP_OK;
   void *bufs[] = {b->d_plans, b->d_rves, b->d_order, b->d_counter, b->d_vals, b->d_dinv,
                   b->d_etype, b->d_strains, b->d_mats, b->d_stress, b->d_strain, b->d_info,
-                  b->d_ws_u, b->d_ws_v, b->d_ws_dinv};
+                  b->d_ws_u, b->d_ws_v, b->d_ws_dinv, b->d_rest, b->d_mcount, b->d_done,
+                  b->d_tinfo};
   for (void *p : bufs) cudaFree(p);
+  modes_free(&b->modes);
   for (DevPlan *p : b->plans) plan_release(p);
   delete b;
   return SP_OK;
@@ -432,6 +490,8 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
     maxnp = std::max(maxnp, g.nn_pad);
     b->etype_off.push_back(r.etype_off);
     b->nelm.push_back(g.nelm);
+    b->geo.push_back(g);
+    b->cls.push_back(modes_class(g, descs[i].len));
   }
   // host-side classification into one pinned staging buffer
   uint8_t *et = nullptr;
@@ -515,12 +575,28 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
   if (!rc) rc = dmalloc((void **)&b->d_stress, (size_t)nrve * nrhs * 6 * sizeof(double), acct);
   if (!rc) rc = dmalloc((void **)&b->d_strain, (size_t)nrve * nrhs * 6 * sizeof(double), acct);
   if (!rc) rc = dmalloc((void **)&b->d_info, (size_t)nrve * sizeof(sp_solve_info), acct);
+  const Shape wide{512, 1, 1, kernel_op(o)};
+  const bool modes = uses_modes(o, wide) && o.cluster <= 1 &&
+                     (trial || (o.threads == 512 && o.ctas_per_sm == 1));
+  if (!rc && modes) {
+    rc = dmalloc((void **)&b->d_rest, nrve * sizeof(int), acct);
+    if (!rc) rc = dmalloc((void **)&b->d_mcount, 256, acct);
+    if (!rc) rc = dmalloc((void **)&b->d_done, nrve * sizeof(unsigned), acct);
+    if (!rc) rc = dmalloc((void **)&b->d_tinfo, (size_t)nrve * nrhs * sizeof(sp_solve_info), acct);
+    if (!rc && cudaMemset(b->d_done, 0, nrve * sizeof(unsigned)))
+      rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
+  }
+  // with a fixed 512 x 1 shape k_batch needs work spaces only for the RVEs
+  // the element-mode kernel does not take
+  std::vector<int> in, rest;
+  if (!rc) split_rves(b, order, &in, &rest);
+  const bool idle = modes && !trial && rest.empty();
   // one work space per cluster (for the largest candidate grid while tuning)
   const size_t slots = (size_t)std::max(b->grid / o.cluster, b->tune_slots);
-  if (!rc) rc = dmalloc((void **)&b->d_ws_u, slots * stride * sizeof(double), acct);
-  if (!rc) rc = dmalloc(&b->d_ws_v, slots * 4 * stride * tsz, acct);
+  if (!rc && !idle) rc = dmalloc((void **)&b->d_ws_u, slots * stride * sizeof(double), acct);
+  if (!rc && !idle) rc = dmalloc(&b->d_ws_v, slots * 4 * stride * tsz, acct);
   // stencil: one Jacobi diagonal [3][max nn_pad] per work space
-  if (!rc && !ell) rc = dmalloc(&b->d_ws_dinv, slots * drm_stride * tsz, acct);
+  if (!rc && !ell && !idle) rc = dmalloc(&b->d_ws_dinv, slots * drm_stride * tsz, acct);
   if (!rc) {
     // default inputs: unit strains e_0..e_{nrhs-1}, materials of the descriptors
     std::vector<double> eps((size_t)nrve * nrhs * 6, 0.0), mats((size_t)nrve * 4);
@@ -569,6 +645,9 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
   P.inner_rtol = o.inner_rtol;
   P.max_outer = o.max_outer;
   P.max_inner = o.max_inner;
+  b->mc = ModesCommon{b->d_plans, b->d_rves, nrhs, b->d_etype, b->d_strains, b->d_mats,
+                      b->d_stress, b->d_strain, b->d_info, b->d_tinfo, b->d_done,
+                      o.rtol, o.inner_rtol, o.max_outer, o.max_inner};
   if (trial) {
     rc = tune_trial(b, cands, order, work, d, &b->tune);
     if (!rc) {
@@ -583,7 +662,9 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
       g_tune_cache[tkey] = b->tune;
     }
     // keep only the work spaces the chosen grid uses
-    const size_t keep = (size_t)(b->grid / b->o.cluster);
+    const bool none = uses_modes(b->o, {b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)}) &&
+                      rest.empty();
+    const size_t keep = none ? 0 : (size_t)(b->grid / b->o.cluster);
     if (!rc && keep < slots) {
       cudaFree(b->d_ws_u);
       cudaFree(b->d_ws_v);
@@ -591,14 +672,26 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
       b->d_ws_u = nullptr;
       b->d_ws_v = b->d_ws_dinv = nullptr;
       b->bytes -= slots * (stride * sizeof(double) + 4 * stride * tsz + (ell ? 0 : drm_stride * tsz));
-      if (!rc) rc = dmalloc((void **)&b->d_ws_u, keep * stride * sizeof(double), acct);
-      if (!rc) rc = dmalloc(&b->d_ws_v, keep * 4 * stride * tsz, acct);
-      if (!rc && !ell) rc = dmalloc(&b->d_ws_dinv, keep * drm_stride * tsz, acct);
+      if (!rc && keep) rc = dmalloc((void **)&b->d_ws_u, keep * stride * sizeof(double), acct);
+      if (!rc && keep) rc = dmalloc(&b->d_ws_v, keep * 4 * stride * tsz, acct);
+      if (!rc && !ell && keep) rc = dmalloc(&b->d_ws_dinv, keep * drm_stride * tsz, acct);
       P.ws_u = b->d_ws_u;
       P.ws_v = b->d_ws_v;
       P.ws_dinv = b->d_ws_dinv;
     }
     b->tune_slots = 0;
+    if (rc) {
+      sp_batch_destroy(b);
+      return rc;
+    }
+  }
+  if (uses_modes(b->o, {b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)})) {
+    b->nrest = (int)rest.size();
+    rc = modes_plan(in, b->cls, b->geo, nrhs, d, &b->modes);
+    if (!rc && b->nrest &&
+        cudaMemcpy(b->d_rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice))
+      rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
+    for (const ModesBucket &m : b->modes.buckets) b->bytes += m.bytes;
     if (rc) {
       sp_batch_destroy(b);
       return rc;
@@ -656,6 +749,19 @@ extern "C" int sp_batch_launch(sp_batch *b, void *stream) {
   cudaStream_t s = pick_stream(stream, d);
   Shape sh{b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)};
   BatchFn fn = pick(b->o.precision, b->nrhs, sh);
+  if (uses_modes(b->o, sh)) {
+    SP_TRY(modes_launch(b->modes, b->mc, b->d_mcount, s));
+    b->last_launches = (int)b->modes.buckets.size();
+    if (b->nrest) {
+      BatchParams P = b->P;
+      P.order = b->d_rest;
+      P.nrve = b->nrest;
+      SP_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(int), s));
+      SP_TRY(launch_shape(fn, sh, b->grid, b->dyn_smem, s, P));
+      b->last_launches++;
+    }
+    return SP_OK;
+  }
   SP_CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(int), s));
   SP_TRY(launch_shape(fn, sh, b->grid, b->dyn_smem, s, b->P));
   b->last_launches = 1;

@@ -1,0 +1,165 @@
+// rve_modes.cu -- host side of the element-mode batch kernel.
+#include <algorithm>
+
+#include "rve_modes_host.h"
+
+namespace sp {
+
+SP_MODES_CLASSES(SP_MODES_EXTERN)
+
+struct ModesClass {
+  int threads, minb;
+  bool qs;
+  ModesFn fn[2];  // box elements, cubes
+};
+
+static const ModesClass kClasses[] = {
+#define SP_MODES_ROW(NT, MINB, QS) \
+  {NT, MINB, QS, {k_modes<NT, MINB, false, QS>, k_modes<NT, MINB, true, QS>}},
+    SP_MODES_CLASSES(SP_MODES_ROW)
+#undef SP_MODES_ROW
+};
+constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
+
+// shared memory of one SM and what a block holds beside its dynamic part
+constexpr int SP_MODES_SM_BYTES = 228 * 1024, SP_MODES_BLOCK_MAX = 227 * 1024;
+constexpr int SP_MODES_RESERVED = 1024;
+
+// dynamic shared memory a CTA of a class may use
+static int class_room(const ModesClass &k) {
+  return (std::min(SP_MODES_SM_BYTES / k.minb, SP_MODES_BLOCK_MAX + 1024) - SP_MODES_RESERVED) / 16 * 16;
+}
+
+// An RVE runs on the smallest class whose threads hold one element column
+// each and whose shared memory holds its vectors beside the
+// class's other CTAs; it needs an interior node on every axis and at most 31
+// element layers (a column's materials are one 32-bit mask).  Larger RVEs
+// keep the solve_rve kernel.
+int modes_class(const MeshGeo &g, const double *len) {
+  if (g.nex < 2 || g.ney < 2 || g.nez < 2 || g.nez > SP_MODES_MAX_NEZ) return -1;
+  if ((long long)g.nex * g.ney > 640) return -1;
+  const ModesGeo G(g.nex, g.ney, g.nez);
+  const double hx = len[0] / g.nex, hy = len[1] / g.ney, hz = len[2] / g.nez;
+  const int cube = hx == hy && hx == hz;
+  for (int c = 0; c < kNumClasses; c++) {
+    const ModesClass &k = kClasses[c];
+    if (G.warps() * 32 <= k.threads && G.smem(k.qs) <= class_room(k)) return 2 * c + cube;
+  }
+  return -1;
+}
+
+int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
+               const std::vector<MeshGeo> &geo, int nrhs, const Device *d,
+               ModesPlan *out) {
+  // classes with the largest RVEs first
+  for (int c = 2 * kNumClasses - 1; c >= 0; c--) {
+    std::vector<int> ord;
+    for (int i : ids)
+      if (cls[i] == c) ord.push_back(i);
+    if (ord.empty()) continue;
+    const ModesClass &k = kClasses[c / 2];
+    out->buckets.push_back(ModesBucket());
+    ModesBucket &b = out->buckets.back();
+    b.fn = k.fn[c & 1];
+    b.nrve = (int)ord.size();
+    int ntot = 0, wlen = 0;
+    for (int i : ord) {
+      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez);
+      b.threads = std::max(b.threads, G.warps() * 32);
+      b.smem = std::max(b.smem, G.smem(k.qs));
+      ntot = std::max(ntot, G.ntot);
+      wlen = std::max(wlen, G.wlen());
+    }
+    b.w_stride = ((size_t)3 * wlen + 15) / 16 * 16;
+    b.v_stride = ((size_t)3 * ntot + 15) / 16 * 16;
+    // the class's largest, the same for every batch: the attribute is the
+    // function's, not the launch's
+    if (cudaFuncSetAttribute((const void *)b.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             class_room(k)) != cudaSuccess) {
+      cudaGetLastError();
+      return sp_set_error(SP_ERR_CUDA, "sp_batch_create: %d bytes of dynamic shared memory refused",
+                          class_room(k));
+    }
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, (const void *)b.fn, b.threads, b.smem) !=
+            cudaSuccess ||
+        nb < 1) {
+      cudaGetLastError();
+      return sp_set_error(SP_ERR_CUDA, "sp_batch_create: %d-thread CTAs cannot be resident", b.threads);
+    }
+    b.grid = (int)std::min<long long>((long long)d->nsm * nb, (long long)b.nrve * nrhs);
+    SP_TRY(dmalloc((void **)&b.d_order, ord.size() * sizeof(int), &b.bytes));
+    SP_TRY(dmalloc((void **)&b.ws_w, b.grid * b.w_stride * sizeof(double), &b.bytes));
+    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (k.qs ? 2 : 3) * b.v_stride * sizeof(float2), &b.bytes));
+    if (cudaMemcpy(b.d_order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice))
+      return sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
+  }
+  for (size_t i = 1; i < out->buckets.size(); i++) {
+    cudaStream_t st;
+    cudaEvent_t ev;
+    SP_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    out->side.push_back(st);
+    SP_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    out->joined.push_back(ev);
+  }
+  if (!out->side.empty())
+    SP_CUDA_TRY(cudaEventCreateWithFlags(&out->forked, cudaEventDisableTiming));
+  return SP_OK;
+}
+
+void modes_free(ModesPlan *m) {
+  for (ModesBucket &k : m->buckets) {
+    cudaFree(k.d_order);
+    cudaFree(k.ws_w);
+    cudaFree(k.ws_v);
+  }
+  for (cudaStream_t s : m->side) cudaStreamDestroy(s);
+  for (cudaEvent_t e : m->joined) cudaEventDestroy(e);
+  if (m->forked) cudaEventDestroy(m->forked);
+  *m = ModesPlan();
+}
+
+int modes_launch(const ModesPlan &m, const ModesCommon &c, int *counters, cudaStream_t s,
+                 bool empty) {
+  const std::vector<ModesBucket> &b = m.buckets;
+  if (b.empty()) return SP_OK;
+  SP_CUDA_TRY(cudaMemsetAsync(counters, 0, b.size() * sizeof(int), s));
+  if (b.size() > 1) SP_CUDA_TRY(cudaEventRecord(m.forked, s));
+  for (size_t i = 0; i < b.size(); i++) {
+    const ModesBucket &k = b[i];
+    ModesParams P;
+    P.plans = c.plans;
+    P.rves = c.rves;
+    P.order = k.d_order;
+    P.nrhs = c.nrhs;
+    P.ntask = empty ? 0 : k.nrve * c.nrhs;
+    P.etype = c.etype;
+    P.strains = c.strains;
+    P.mats = c.mats;
+    P.out_stress = c.out_stress;
+    P.out_strain = c.out_strain;
+    P.out_info = c.out_info;
+    P.task_info = c.task_info;
+    P.done = c.done;
+    P.counter = counters + i;
+    P.ws_w = k.ws_w;
+    P.ws_v = k.ws_v;
+    P.w_stride = k.w_stride;
+    P.v_stride = k.v_stride;
+    P.rtol = c.rtol;
+    P.inner_rtol = c.inner_rtol;
+    P.max_outer = c.max_outer;
+    P.max_inner = c.max_inner;
+    cudaStream_t st = i ? m.side[i - 1] : s;
+    if (i) SP_CUDA_TRY(cudaStreamWaitEvent(st, m.forked, 0));
+    k.fn<<<k.grid, k.threads, k.smem, st>>>(P);
+    SP_CUDA_TRY(cudaGetLastError());
+    if (i) SP_CUDA_TRY(cudaEventRecord(m.joined[i - 1], st));
+  }
+  for (size_t i = 1; i < b.size(); i++) {
+    SP_CUDA_TRY(cudaStreamWaitEvent(s, m.joined[i - 1], 0));
+  }
+  return SP_OK;
+}
+
+}  // namespace sp

@@ -1,0 +1,936 @@
+// rve_modes_kernel.cuh -- the batched FP32 stencil solve, one load case of
+// one RVE per CTA at a time, on the element-mode operator (rve_modes.cuh).
+//
+// The load cases of an RVE are independent systems.  Solved one by one, the
+// search direction p and the product q = A p of an RVE of up to about 20^3
+// elements stay in one SM's shared memory (6 load cases at once are 2.7 MB of
+// vectors at n = 20, which stream from HBM in every CG iteration); r and x,
+// 16 bytes a node component, stream from L2 once per iteration.  A load case
+// leaves when it has converged, not when the slowest of its RVE has.
+//
+// What a CTA runs is the solve of rve_solve.cuh for K = 1: FP64 residual of
+// u = eps.x + w (here marched in element modes too), FP32 Jacobi-PCG
+// corrections as reliable updates, w += x in FP64, volume averages in FP64.
+#pragma once
+
+#include "rve_batch_kernel.cuh"
+#include "rve_modes.cuh"
+
+namespace sp {
+
+struct ModesParams {
+  const BatchPlan *plans;
+  const BatchRve *rves;
+  const int *order;  // RVEs of this launch, largest first
+  int ntask, nrhs;   // tasks: (RVE, load case)
+  const uint8_t *etype;
+  const double *strains;  // [nrve][nrhs][6]
+  const double *mats;     // [nrve][4]
+  double *out_stress, *out_strain;
+  sp_solve_info *out_info;
+  sp_solve_info *task_info;  // [nrve][nrhs]
+  unsigned *done;            // [nrve] finished load cases (0 between launches)
+  int *counter;
+  double *ws_w;    // per CTA [3][wlen]
+  float2 *ws_v;    // per CTA r, x and (q not in shared memory) q: [3][ntot] pairs each
+  size_t w_stride, v_stride;  // v_stride: of one of them
+  double rtol, inner_rtol;
+  int max_outer, max_inner;
+};
+
+constexpr int SP_MODES_MAX_NEZ = 31;  // a column's materials are one 32-bit mask
+constexpr int SP_MODES_MAX_WARPS = 20;
+
+// What the CTA shares while it solves one load case; the first thing in its
+// dynamic shared memory.
+struct ModesShared {
+  double cd[2][MC_N];    // mode coefficients of the two materials
+  float2 c32[4][MC_N];   // FP32 pairs: materials of the (lower, upper) layer
+  float4 dl[9];          // Jacobi diagonal by the number of fibre elements around a node
+  double kd2[9];         // sum over components of the squared diagonal
+  double A[9];           // first-order modes of eps.x: [component][axis]
+  double E[9];           // eps as a 3x3 matrix
+  double len[3], hx[3], a[3];  // box, element edges and their inverses
+  double lame[2][2];     // lambda, mu of the two materials
+  double red[2 * SP_MODES_MAX_WARPS * 10];
+  double cc[2][CC_N];    // cube: lambda, mu, 2 mu, lambda/3, mu/3, (lambda + 4 mu)/9, times c0 a^2
+  float2 c6[4][CC_N];    // ... as FP32 pairs: materials of the (lower, upper) layer
+  unsigned col[SP_MODES_MAX_WARPS * 32];  // per column: bit e = material of layer e
+  int nex, ney, nez, nface, mz, h, ntot, wlen;
+  int job, rid, k, outer, inner, wcols, qoff, cntoff;  // qoff, cntoff: bytes from p on
+};
+static_assert(sizeof(ModesShared) % 16 == 0, "vectors follow on a 16-byte boundary");
+
+// sizes of one RVE's march
+struct ModesGeo {
+  int nex, ney, nez, nface, mz, h, ntot;
+  __host__ __device__ ModesGeo(int ex, int ey, int ez)
+      : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(ez - 1), h(ez / 2),
+        ntot((ez / 2) * ex * ey + ex + 2) {}
+  __host__ __device__ int wlen() const { return mz * nface + nex + 2; }
+  // columns of a warp: 32 where rows start at lane 0 (a row's first node is a
+  // boundary node, which needs no share from the lane below), else 31 and a
+  // repeated one
+  __host__ __device__ int wcols() const { return 32 % nex == 0 ? 32 : 31; }
+  __host__ __device__ int warps() const { return (nface + wcols() - 1) / wcols(); }
+  // Dynamic shared memory: tables, p, then (QS) q, whose place the FP64
+  // residual's face state and exchange planes take too, or (no q) two
+  // exchange planes and the state in p's place; material counts.
+  __host__ __device__ int state() const { return 32 * warps() * 8; }
+  __host__ __device__ int pbytes(bool qs) const {
+    const int a = ntot * 24, b = qs ? 0 : 25 * state();
+    return a > b ? a : b;
+  }
+  __host__ __device__ int qbytes(bool qs) const {
+    const int a = qs ? ntot * 24 : 0, b = 2 * nface * 24 + (qs ? 13 * state() : 0);
+    return a > b ? a : b;
+  }
+  __host__ __device__ int smem(bool qs) const {
+    return (int)sizeof(ModesShared) + pbytes(qs) + qbytes(qs) + (h * nface + 15) / 16 * 16;
+  }
+};
+
+extern __shared__ __align__(16) unsigned char s_modes[];
+__device__ __forceinline__ ModesShared &msh() { return *reinterpret_cast<ModesShared *>(s_modes); }
+__device__ __forceinline__ F2 *mp() { return reinterpret_cast<F2 *>(s_modes + sizeof(ModesShared)); }
+// q, or the exchange planes
+__device__ __forceinline__ F2 *mq() {
+  return reinterpret_cast<F2 *>(reinterpret_cast<char *>(mp()) + msh().qoff);
+}
+__device__ __forceinline__ uint8_t *mcnt() {
+  return reinterpret_cast<uint8_t *>(mp()) + msh().cntoff;
+}
+
+// Sum NV doubles over the CTA in a fixed order; every thread gets the
+// totals.  One barrier: red holds two buffers, used in turn.
+template <int NV>
+__device__ __forceinline__ void cta_sum(double (&v)[NV], int &ph) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double *r = msh().red + ph * (SP_MODES_MAX_WARPS * 10);
+#pragma unroll
+  for (int q = 0; q < NV; q++)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < NV; q++) r[warp * NV + q] = v[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    v[q] = lane < nw ? r[lane * NV + q] : 0.0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+  }
+  ph ^= 1;
+}
+
+// A thread's place in the march.  f: its element column (face); the repeated
+// lanes and the padding threads of the last warp write nothing.
+struct ModesLane {
+  int f;
+  bool warp_on;  // the warp has a column
+  bool column;   // the thread has one
+  bool owner;    // ... and its node (ex, ey) is an interior one
+  int threads;   // of all warps that have a column
+  __device__ __forceinline__ ModesLane() {
+    const ModesShared &sh = msh();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rep = 32 - sh.wcols;
+    const int i = warp * sh.wcols + lane - rep;
+    warp_on = warp * sh.wcols < sh.nface;
+    column = lane >= rep && i < sh.nface;
+    f = min(max(i, 0), sh.nface - 1);
+    owner = column && f >= sh.nex && f % sh.nex != 0;
+    threads = (sh.nface + sh.wcols - 1) / sh.wcols * 32;
+  }
+};
+
+// Barrier over the warps that have columns
+__device__ __forceinline__ void plane_sync(int threads) {
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+// q = A p: p, q in shared memory ([slot][3] pairs), q in qg ([3][ntot]) when
+// QS is false; returns the thread's share of p.q.
+template <bool CUBE, bool QS>
+__device__ __noinline__ double march_apply(float2 *qg) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  const unsigned mats = sh.col[T.f];
+  const int nface = sh.nface, nf3 = 3 * nface, h = sh.h, ntot = sh.ntot;
+  const int up = 3 * sh.nex;
+  const F2 *pf = mp() + 3 * T.f;  // corner (0, 0) of slot 0
+  F2 *const qf = mq() + 3 * T.f;
+  const bool odd = (sh.mz & 1) != 0;
+  F2 raw[3][4], Fa[3][4], Fb[3][4], acc[3][4];
+  auto load = [&](const F2 *a) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      raw[c][0] = a[c];
+      raw[c][1] = a[3 + c];
+      raw[c][2] = a[up + c];
+      raw[c][3] = a[up + 3 + c];
+    }
+  };
+  // values of step s: slot s; above slot h - 1 lies plane h (lower half), the
+  // boundary plane (upper half)
+  auto next = [&](int s) {
+    load(s < h ? pf + s * nf3 : pf);
+    if (s >= h) {
+      __syncwarp();  // a branch: predicated, the moves would be issued every step
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) raw[c][m] = mk2(raw[c][m].v.y, 0.f);
+    }
+  };
+  if (T.warp_on) {
+    // below slot 0: the boundary plane (lower half), plane h - 1 (upper half)
+    load(pf + (h - 1) * nf3);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        raw[c][m] = mk2(0.f, raw[c][m].v.x);
+        acc[c][m] = mk2(0.f, 0.f);
+      }
+    face_modes(raw, Fa);
+    if (QS) next(0);
+  }
+  if (!T.warp_on) return 0.0;
+  double pq = 0.0;
+  // one step: F0 the modes of the face below, F1 takes those above (two steps
+  // a trip, so that the faces change places without copies)
+  auto step = [&](int s, F2 (&F0)[3][4], F2 (&F1)[3][4]) {
+    F2 low[3];
+    if (T.warp_on) {
+      F2 S[3][3], D[3][4], high[3];
+      if (!QS) next(s);
+      face_modes(raw, F1);
+      layer_modes(F0, F1, S, D);
+      const unsigned ma = (mats >> s) & 1u, mb = (mats >> (s + h)) & 1u;
+      if constexpr (CUBE) {
+        const float2 *ct = sh.c6[ma + 2 * mb];
+        modes_cube(S, D, [ct](int i) { return F2{ct[i]}; });
+      } else {
+        const float2 *ct = sh.c32[ma + 2 * mb];
+        modes_box(S, D, [ct](int i) { return F2{ct[i]}; });
+      }
+      layer_back(S, D, acc, low, high);
+      // the upper row's share waits where that row's q goes (QS), or in the
+      // exchange planes in turn
+      F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3 + up;
+      if (T.column && s > 0 && T.f + sh.nex < nface)
+#pragma unroll
+        for (int c = 0; c < 3; c++) e[c] = high[c];
+      // with registers to spare, the next slot's values before the barrier
+      if (QS) next(s + 1);
+    }
+    if (s > 0) {
+      plane_sync(T.threads);
+      if (T.owner) {
+        F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3;
+        const F2 *ps = pf + (s - 1) * nf3;
+        F2 t = mk2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          low[c] = low[c] + e[c];
+          if (odd && s == h) low[c].v.y = 0.f;  // no plane there
+          if constexpr (QS)
+            e[c] = low[c];
+          else
+            __stcg(qg + (size_t)c * ntot + (s - 1) * nface + T.f, low[c].v);
+          t = mad(low[c], ps[c], t);
+        }
+        pq += (double)(t.v.x + t.v.y);
+      }
+    }
+  };
+#pragma unroll 1
+  for (int s = 0; s <= h; s++) {
+    step(s, Fa, Fb);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) Fa[c][m] = Fb[c][m];
+  }
+  return pq;
+}
+
+// b = -K (eps.x + w) on the interior nodes in FP64: rounded to FP32 into rg;
+// returns the thread's shares of |b|^2 and r.z.  The running plane's forces
+// (and, at 96 registers a thread, the face's modes) wait in shared memory
+// between layers: in registers they spill, and a spill goes to L2, since the
+// vectors leave L1 next to nothing (n = 20: 285k cycles an evaluation with
+// spills, 80k without).
+template <bool CUBE, bool QS>
+__device__ __noinline__ double2 march_residual(const double *w, float *rg) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  const unsigned mats = sh.col[T.f];
+  const int nface = sh.nface, nex = sh.nex, wl = sh.wlen, mz = sh.mz, h = sh.h;
+  double *const ex = reinterpret_cast<double *>(mq());  // two exchange planes
+  const uint8_t *const cnt = mcnt();
+  // [c][m] of the running forces at 4 c + m, of the face's modes 12 further;
+  // an odd number of doubles a thread (no bank conflicts)
+  double *const state = (QS ? ex + 6 * nface : reinterpret_cast<double *>(mp())) +
+                        (T.warp_on ? threadIdx.x : 0) * (QS ? 13 : 25);
+  double n2 = 0.0, rz = 0.0;
+  double F0[3][4] = {};  // (QS)
+  double raw[3][4];
+  auto load = [&](int pl) {
+    const double *a = w + (pl * nface + T.f);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      raw[c][0] = a[c * wl];
+      raw[c][1] = a[c * wl + 1];
+      raw[c][2] = a[c * wl + nex];
+      raw[c][3] = a[c * wl + nex + 1];
+    }
+  };
+  if (T.warp_on) {
+#pragma unroll
+    for (int j = 0; j < (QS ? 12 : 24); j++) state[j] = 0.0;
+    load(0);
+  }
+  if (!T.warp_on) return make_double2(0.0, 0.0);
+#pragma unroll 1
+  for (int s = 0; s <= mz; s++) {
+    double low[3];
+    double *const exs = ex + (s & 1) * 3 * nface;
+    if (T.warp_on) {
+      double S[3][3], D[3][4];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double s0 = raw[c][1] + raw[c][0], d0 = raw[c][1] - raw[c][0];
+        const double s1 = raw[c][3] + raw[c][2], d1 = raw[c][3] - raw[c][2];
+        const double F1[4] = {s1 + s0, d1 + d0, s1 - s0, d1 - d0};
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const double v = QS ? F0[c][m] : state[12 + 4 * c + m];
+          if (m > 0) S[c][m - 1] = F1[m] + v;
+          D[c][m] = F1[m] - v;
+          if (QS)
+            F0[c][m] = F1[m];
+          else
+            state[12 + 4 * c + m] = F1[m];
+        }
+        S[c][0] += sh.A[3 * c];
+        S[c][1] += sh.A[3 * c + 1];
+        D[c][0] += sh.A[3 * c + 2];
+      }
+      if constexpr (CUBE) {
+        const double *ct = sh.cc[(mats >> s) & 1u];
+        modes_cube(S, D, [ct](int i) { return ct[i]; });
+      } else {
+        const double *ct = sh.cd[(mats >> s) & 1u];
+        modes_box(S, D, [ct](int i) { return ct[i]; });
+      }
+      double *e = exs + 3 * T.f;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        double *const ac = state + 4 * c;
+        const double t0 = ac[0] - D[c][0];
+        const double t1 = ac[1] + (S[c][0] - D[c][1]);
+        const double t2 = ac[2] + (S[c][1] - D[c][2]);
+        const double t3 = ac[3] + (S[c][2] - D[c][3]);
+        ac[0] = D[c][0];
+        ac[1] = S[c][0] + D[c][1];
+        ac[2] = S[c][1] + D[c][2];
+        ac[3] = S[c][2] + D[c][3];
+        double high;
+        plane_back(t0, t1, t2, t3, low[c], high);
+        if (T.column) e[c] = high;
+      }
+    }
+    if (s + 1 < mz) {
+      load(s + 1);
+    } else {
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) raw[c][m] = 0.0;
+    }
+    if (s > 0) {
+      plane_sync(T.threads);
+      if (T.owner) {
+        const double *e = exs + 3 * (T.f - nex);
+        const bool hi = s - 1 >= h;
+        const int i = (hi ? s - 1 - h : s - 1) * nface + T.f;
+        const unsigned cv = cnt[i];
+        const float4 dl = sh.dl[hi ? cv >> 4 : cv & 15u];
+        const float dz[3] = {dl.x, dl.y, dl.z};
+        float *ro = rg + 2 * i + (hi ? 1 : 0);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double b = -(low[c] + e[c]);
+          const float bf = (float)b;
+          ro[2 * c * sh.ntot] = bf;
+          n2 += b * b;
+          rz += (double)bf * (double)(dz[c] * bf);
+        }
+      }
+    }
+  }
+  return make_double2(n2, rz);
+}
+
+// Integrals over the fibre elements of the fluctuation's gradient, up to the
+// factor element volume / 4 and the edge lengths: m[3 c + d] = sum of the
+// first-order mode along d of component c, as a sum over nodes -- a node's
+// weight is the number of fibre elements below it along d less the number
+// above.  (Over all elements the weights vanish: the mean strain is eps.)
+// m[9]: the number of fibre elements.
+// Summed over the CTA; thread 0 gets the totals.
+__device__ __noinline__ inline int march_average(const double *w, int ph) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  double m[10];
+#pragma unroll
+  for (int q = 0; q < 10; q++) m[q] = 0.0;
+  if (T.column) m[9] = (double)__popc(sh.col[T.f]);
+  if (T.owner) {
+    const int wl = sh.wlen, mz = sh.mz, nface = sh.nface;
+    const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f - 1], c1 = sh.col[T.f - sh.nex],
+                   c0 = sh.col[T.f - sh.nex - 1];
+#pragma unroll 4
+    for (int pl = 0; pl < mz; pl++) {
+      const unsigned b0 = (c0 >> pl) & 3u, b1 = (c1 >> pl) & 3u, b2 = (c2 >> pl) & 3u,
+                     b3 = (c3 >> pl) & 3u;
+      const int n0 = __popc(b0), n1 = __popc(b1), n2 = __popc(b2), n3 = __popc(b3);
+      const int lower = (b0 & 1) + (b1 & 1) + (b2 & 1) + (b3 & 1);
+      const double k[3] = {(double)(n0 + n2 - n1 - n3), (double)(n0 + n1 - n2 - n3),
+                           (double)(2 * lower - (n0 + n1 + n2 + n3))};
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double v = w[c * wl + pl * nface + T.f];
+#pragma unroll
+        for (int d = 0; d < 3; d++) m[3 * c + d] = fma(k[d], v, m[3 * c + d]);
+      }
+    }
+  }
+  cta_sum<10>(m, ph);
+  __syncthreads();
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int q = 0; q < 10; q++) msh().red[q] = m[q];  // for thread 0 alone
+  return ph;
+}
+
+// Jacobi diagonal of a slot's two nodes
+template <bool CUBE>
+__device__ __forceinline__ void dinv_pairs(int i, F2 (&dz)[3]) {
+  const ModesShared &sh = msh();
+  const unsigned cv = mcnt()[i];
+  if (CUBE) {  // the three components' diagonals are equal
+    dz[0] = dz[1] = dz[2] = mk2(sh.dl[cv & 15u].x, sh.dl[cv >> 4].x);
+    return;
+  }
+  const float4 da = sh.dl[cv & 15u], db = sh.dl[cv >> 4];
+  dz[0] = mk2(da.x, db.x);
+  dz[1] = mk2(da.y, db.y);
+  dz[2] = mk2(da.z, db.z);
+}
+
+// One group of up to U slots of update_xr: all loads before the stores, one L2
+// round trip for the group.
+template <bool CUBE, bool QS, int U>
+__device__ __forceinline__ void xr_slots(int s0, int f, float2 *rg, float2 *xg, const float2 *qg,
+                                         F2 al, F2 nal, bool first, double &vz, double &vr) {
+  const ModesShared &sh = msh();
+  const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
+  F2 *const p = mp();
+  F2 r[U][3], q[U][3];
+#pragma unroll
+  for (int j = 0; j < U; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const int o = c * ntot + min(s0 + j, h - 1) * nface + f;
+      r[j][c].v = __ldcg(rg + o);
+      if (!QS) q[j][c].v = __ldcg(qg + o);
+    }
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    if (s0 + j >= h) break;
+    const int i = (s0 + j) * nface + f;
+    F2 dz[3];
+    dinv_pairs<CUBE>(i, dz);
+    F2 sz = mk2(0.f, 0.f), sr = mk2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const int o = c * ntot + i;
+      const F2 rn = mad(nal, QS ? p[3 * (ntot + i) + c] : q[j][c], r[j][c]);
+      const F2 dx = al * p[3 * i + c];
+      __stcg(rg + o, rn.v);
+      if (first)
+        __stcg(xg + o, dx.v);
+      else
+        atomicAdd(xg + o, dx.v);  // (no value back: nothing waits for it)
+      if constexpr (QS) p[3 * (ntot + i) + c] = rn;
+      sz = mad(rn, dz[c] * rn, sz);
+      sr = mad(rn, rn, sr);
+    }
+    vz += (double)(sz.v.x + sz.v.y);
+    vr += (double)(sr.v.x + sr.v.y);
+  }
+}
+
+// x += alpha p, r -= alpha q over the thread's column (x = alpha p in a
+// correction's first step); returns its shares of r.z and r.r.  x is added to
+// in L2: only this thread touches its entries.  q's slots take the new r for
+// the direction update.
+template <bool CUBE, bool QS>
+__device__ __noinline__ double2 update_xr(float2 *rg, float2 *xg, const float2 *qg, float alpha,
+                                          bool first) {
+  const ModesLane T;
+  if (!T.owner) return make_double2(0.0, 0.0);
+  const int h = msh().h;
+  const F2 al = mk2(alpha, alpha), nal = mk2(-alpha, -alpha);
+  double vz = 0.0, vr = 0.0;
+  constexpr int U = QS ? 5 : 3;
+#pragma unroll 1
+  for (int s = 0; s < h; s += U) xr_slots<CUBE, QS, U>(s, T.f, rg, xg, qg, al, nal, first, vz, vr);
+  return make_double2(vz, vr);
+}
+
+// p = D^-1 r + beta p over the thread's column; r in q's slots (LOCAL) or in
+// rg.  beta = 0 starts afresh without reading p.
+template <bool CUBE, bool LOCAL, int U>
+__device__ __forceinline__ void p_slots(int s0, int f, const float2 *rg, F2 be, bool fresh) {
+  const ModesShared &sh = msh();
+  const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
+  F2 *const p = mp();
+  F2 r[U][3], pv[U][3];
+#pragma unroll
+  for (int j = 0; j < U; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const int i = min(s0 + j, h - 1) * nface + f;
+      if constexpr (LOCAL)
+        r[j][c] = p[3 * (ntot + i) + c];
+      else
+        r[j][c].v = __ldcg(rg + (c * ntot + i));
+      pv[j][c] = p[3 * i + c];
+    }
+#pragma unroll
+  for (int j = 0; j < U; j++) {
+    if (s0 + j >= h) break;
+    const int i = (s0 + j) * nface + f;
+    F2 dz[3];
+    dinv_pairs<CUBE>(i, dz);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const F2 z = dz[c] * r[j][c];
+      p[3 * i + c] = fresh ? z : mad(be, pv[j][c], z);
+    }
+  }
+}
+
+template <bool CUBE, bool LOCAL>
+__device__ __noinline__ void update_p(const float2 *rg, float beta) {
+  const ModesLane T;
+  if (!T.owner) return;
+  const int h = msh().h;
+  const F2 be = mk2(beta, beta);
+  constexpr int U = LOCAL ? 3 : 5;
+#pragma unroll 1
+  for (int s = 0; s < h; s += U) p_slots<CUBE, LOCAL, U>(s, T.f, rg, be, beta == 0.f);
+}
+
+// w += x in FP64 over the thread's column
+__device__ __noinline__ inline void update_w(const float2 *xg, double *w) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  if (!T.owner) return;
+  const int nface = sh.nface, ntot = sh.ntot, h = sh.h, mz = sh.mz, wl = sh.wlen;
+#pragma unroll 1
+  for (int s = 0; s < h; s++) {
+    const int i = s * nface + T.f;
+    float2 x[3];
+    double w0[3], w1[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      x[c] = __ldcg(xg + (c * ntot + i));
+      w0[c] = w[c * wl + i];
+      w1[c] = s + h < mz ? w[c * wl + i + h * nface] : 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      w[c * wl + i] = w0[c] + (double)x[c].x;
+      if (s + h < mz) w[c * wl + i + h * nface] = w1[c] + (double)x[c].y;
+    }
+  }
+}
+
+// The residual's face state takes p's place when q is not in shared memory:
+// every column's p waits in q's global work space meanwhile, the padding is
+// zeroed anew.
+__device__ __noinline__ inline void save_p(float2 *qg) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  if (T.owner)
+    for (int s = 0; s < sh.h; s++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const int i = s * sh.nface + T.f;
+        __stcg(qg + (c * sh.ntot + i), mp()[3 * i + c].v);
+      }
+  __syncthreads();
+}
+__device__ __noinline__ inline void restore_p(const float2 *qg, bool saved) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  for (int i = threadIdx.x; i < 3 * sh.ntot; i += blockDim.x) mp()[i] = mk2(0.f, 0.f);
+  __syncthreads();
+  if (T.owner && saved)
+    for (int s = 0; s < sh.h; s++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const int i = s * sh.nface + T.f;
+        mp()[3 * i + c].v = __ldcg(qg + (c * sh.ntot + i));
+      }
+}
+
+// the tables, materials and start vectors of one load case
+template <bool QS>
+__device__ __noinline__ void modes_setup(const double *len, const double *mat,
+                                         const uint8_t *etype, const double *eps, double *w,
+                                         float2 *rg) {
+  ModesShared &sh = msh();
+  const int t = threadIdx.x;
+  const ModesLane T;
+  const int nface = sh.nface, nex = sh.nex, wl = sh.wlen;
+  if (t < 3) {
+    const int n = t == 0 ? sh.nex : (t == 1 ? sh.ney : sh.nez);
+    sh.len[t] = len[t];
+    sh.hx[t] = len[t] / n;
+    sh.a[t] = n / len[t];
+  }
+  if (t < 2) {
+    const double E = mat[2 * t], nu = mat[2 * t + 1];
+    sh.lame[t][0] = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
+    sh.lame[t][1] = E / (2.0 * (1.0 + nu));
+  }
+  if (t >= 3 && t < 12) {
+    const int i = (t - 3) / 3, j = (t - 3) % 3;
+    // Voigt entry of (i, j): xx yy zz xy yz xz, shears halved
+    const int v = i == j ? i : (i + j == 1 ? 3 : (i + j == 3 ? 4 : 5));
+    sh.E[t - 3] = i == j ? eps[v] : eps[v] / 2;
+  }
+  unsigned mats = 0;
+  const uint8_t *et = etype + T.f;
+  if (T.warp_on)
+    for (int e = 0; e < sh.nez; e++) mats |= (unsigned)__ldg(et + e * nface) << e;
+  if (T.column) sh.col[T.f] = mats;
+  {
+    float4 *p = reinterpret_cast<float4 *>(mp());  // (3 ntot pairs, rounded down to 16 bytes)
+    for (int i = t; i < 3 * sh.ntot / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t == 0) mp()[3 * sh.ntot - 1] = mk2(0.f, 0.f);
+  }
+  // w's padding: the columns without an interior node and the row past the end
+  if (T.column && !T.owner)
+    for (int c = 0; c < 3; c++)
+      for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = 0.0;
+  for (int i = t; i < 3 * (nex + 2); i += blockDim.x)
+    w[(i / (nex + 2)) * wl + sh.mz * nface + i % (nex + 2)] = 0.0;
+  __syncthreads();
+  if (t < 2 * MC_N)
+    sh.cd[t / MC_N][t % MC_N] = mode_coef(t % MC_N, sh.lame[t / MC_N][0], sh.lame[t / MC_N][1],
+                                          sh.hx[0] * sh.hx[1] * sh.hx[2] / 16.0, sh.a);
+  if (t < 9) sh.A[t] = 4.0 * sh.hx[t % 3] * sh.E[t];
+  // fibre elements around the column's nodes; start of the right-hand side's
+  // own residual: w = -eps.x inside, i.e. u = 0 inside
+  if (T.owner) {
+    const unsigned m0 = mats, m1 = sh.col[T.f - 1], m2 = sh.col[T.f - nex],
+                   m3 = sh.col[T.f - nex - 1];
+    auto count = [&](int pl) {
+      return __popc((m0 >> pl) & 3u) + __popc((m1 >> pl) & 3u) + __popc((m2 >> pl) & 3u) +
+             __popc((m3 >> pl) & 3u);
+    };
+    for (int s = 0; s < sh.h; s++)
+      mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (count(s + sh.h) << 4));
+    const double X = (T.f % nex) * sh.hx[0], Y = (T.f / nex) * sh.hx[1];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const double xy = sh.E[3 * c] * X + sh.E[3 * c + 1] * Y, ez = sh.E[3 * c + 2] * sh.hx[2];
+      for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
+      // a slot without an upper plane keeps a zero there
+      rg[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
+    }
+  }
+  __syncthreads();
+  if (t >= 32 && t < 34) {
+    const double *C = sh.cd[t - 32];
+    double *k = sh.cc[t - 32];
+    k[CC_LAM] = C[MC_BXY];
+    k[CC_MU] = C[MC_MXX];
+    k[CC_MU2] = 2.0 * C[MC_MXX];
+    k[CC_LAM3] = C[MC_B3XY];
+    k[CC_MU3] = C[MC_M3XY];
+    k[CC_K9] = C[MC_U111];
+  }
+  for (int i = t; i < 4 * MC_N; i += blockDim.x) {
+    const int m = i / MC_N, c = i % MC_N;
+    sh.c32[m][c] = make_float2((float)sh.cd[m & 1][c], (float)sh.cd[m >> 1][c]);
+  }
+  __syncthreads();
+  if (t < 24) {
+    const int m = t / 6, i = t % 6;
+    sh.c6[m][i] =
+        make_float2((float)sh.cc[m & 1][i], (float)sh.cc[m >> 1][i]);
+  }
+  if (t < 9) {
+    double s2 = 0.0, d[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      d[c] = (8 - t) * mode_diag(sh.cd[0], c) + t * mode_diag(sh.cd[1], c);
+      s2 += d[c] * d[c];
+    }
+    sh.dl[t] = make_float4((float)(1.0 / d[0]), (float)(1.0 / d[1]), (float)(1.0 / d[2]), 0.f);
+    sh.kd2[t] = s2;
+  }
+  __syncthreads();
+}
+
+// Averages from the fibre's integrals m (march_average), by one thread: <strain> = eps, <stress> = D_0 eps + (D_1 -
+// D_0) f, f = the strain's integral over the fibre / volume.
+__device__ __noinline__ inline void modes_output(const double *m, double *stress, double *strain) {
+  const ModesShared &sh = msh();
+  const double nel = (double)sh.nface * sh.nez;
+  const double sc = 0.25 / nel, vf = m[9] / nel;
+  const double *a = sh.a, *E = sh.E;
+  const double e[6] = {E[0], E[4], E[8], 2.0 * E[1], 2.0 * E[5], 2.0 * E[2]};
+  const double f[6] = {vf * e[0] + sc * a[0] * m[0],
+                       vf * e[1] + sc * a[1] * m[4],
+                       vf * e[2] + sc * a[2] * m[8],
+                       vf * e[3] + sc * (a[1] * m[1] + a[0] * m[3]),
+                       vf * e[4] + sc * (a[2] * m[5] + a[1] * m[7]),
+                       vf * e[5] + sc * (a[2] * m[2] + a[0] * m[6])};
+  const double l0 = sh.lame[0][0], m0 = sh.lame[0][1], l1 = sh.lame[1][0], m1 = sh.lame[1][1];
+  const double tf = f[0] + f[1] + f[2], tm = e[0] + e[1] + e[2] - tf;
+#pragma unroll
+  for (int i = 0; i < 6; i++) {
+    const double g = e[i] - f[i];
+    if (strain) strain[i] = e[i];
+    stress[i] = i < 3 ? (l0 * tm + 2.0 * m0 * g) + (l1 * tf + 2.0 * m1 * f[i])
+                      : m0 * g + m1 * f[i];
+  }
+}
+
+// The CTA's work spaces.  Formed anew at every use (hidden from the
+// compiler's view of the loop), so that no pointer holds registers across the
+// marches.
+template <bool QS>
+struct ModesSpace {
+  double *w;
+  float2 *r, *x, *q;
+  __device__ __forceinline__ explicit ModesSpace(const ModesParams &P) {
+    unsigned b = blockIdx.x;
+    asm volatile("" : "+r"(b));
+    w = P.ws_w + (size_t)b * P.w_stride;
+    r = P.ws_v + (size_t)b * (QS ? 2 : 3) * P.v_stride;
+    x = r + P.v_stride;
+    q = QS ? nullptr : x + P.v_stride;
+  }
+};
+
+// norm of the right-hand side (u = 0 inside, as modes_setup left w) from its
+// square and the column's share; one at the round-off level of its own
+// cancelling terms is zero, and its load case is solved with u = 0.  Else
+// w = 0: the affine field starts.
+__device__ __noinline__ inline double rhs_norm(double n2, double *w, int ph) {
+  const ModesShared &sh = msh();
+  const ModesLane T;
+  double v[2] = {n2, 0.0};
+  if (T.owner)
+    for (int s = 0; s < sh.h; s++) {
+      const unsigned cv = mcnt()[s * sh.nface + T.f];
+      v[1] += sh.kd2[cv & 15u];
+      if (s + sh.h < sh.mz) v[1] += sh.kd2[cv >> 4];
+    }
+  cta_sum<2>(v, ph);
+  double um = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    um = fmax(um, fabs(sh.E[3 * c]) * sh.len[0] + fabs(sh.E[3 * c + 1]) * sh.len[1] +
+                      fabs(sh.E[3 * c + 2]) * sh.len[2]);
+  double rn0 = sqrt(v[0]);
+  if (rn0 <= SP_RHS_FLOOR * sqrt(v[1]) * um) rn0 = 0.0;
+  if (rn0 > 0.0 && T.owner)
+    for (int c = 0; c < 3; c++)
+      for (int pl = 0; pl < sh.mz; pl++) w[c * sh.wlen + pl * sh.nface + T.f] = 0.0;
+  __syncthreads();
+  return rn0;
+}
+
+// The RVE's last load case to finish reports for all of them: the worst
+// status and residual, the most refinement steps and CG iterations.  One
+// thread.
+__device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_solve_info *ti, int k,
+                                                 int nrhs, unsigned *done, sp_solve_info *out) {
+  ti[k] = in;
+  __threadfence();
+  if (atomicAdd(done, 1u) == (unsigned)nrhs - 1) {
+    __threadfence();
+    sp_solve_info all = {};
+    for (int i = 0; i < nrhs; i++) {
+      const volatile sp_solve_info *c = ti + i;
+      if (c->status > all.status) all.status = c->status;
+      if (c->outer_its > all.outer_its) all.outer_its = c->outer_its;
+      if (c->inner_its > all.inner_its) all.inner_its = c->inner_its;
+      all.relres = fmax(all.relres, c->relres);
+    }
+    *out = all;
+    *done = 0;
+  }
+}
+
+// NT threads at most, MINB CTAs per SM; CUBE: equal element edges; QS: q in
+// shared memory
+template <int NT, int MINB, bool CUBE, bool QS>
+__global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
+  ModesShared &sh = msh();
+  if (dynamic_smem_bytes() < sizeof(ModesShared)) return;
+  int ph = 0;  // the reduction buffer in turn
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int task = atomicAdd(P.counter, 1);
+      sh.job = task < P.ntask ? 1 : 0;
+      if (task < P.ntask) {
+        sh.rid = P.order[task / P.nrhs];
+        sh.k = task % P.nrhs;
+        const MeshGeo &mg = P.plans[P.rves[sh.rid].plan].geo;
+        const ModesGeo G(mg.nex, mg.ney, mg.nez);
+        if (dynamic_smem_bytes() < (unsigned)G.smem(QS) || G.warps() * 32 > blockDim.x ||
+            G.warps() > SP_MODES_MAX_WARPS || G.nez > SP_MODES_MAX_NEZ)
+          sh.job = 2;  // launched with less than this RVE needs
+        sh.nex = G.nex;
+        sh.ney = G.ney;
+        sh.nez = G.nez;
+        sh.nface = G.nface;
+        sh.mz = G.mz;
+        sh.h = G.h;
+        sh.ntot = G.ntot;
+        sh.wlen = G.wlen();
+        sh.wcols = G.wcols();
+        sh.qoff = G.pbytes(QS);
+        sh.cntoff = G.pbytes(QS) + G.qbytes(QS);
+        sh.outer = sh.inner = 0;
+      }
+    }
+    __syncthreads();
+    if (sh.job == 0) break;
+    double relres = 0.0;
+    if (sh.job == 1) {
+      // 1. tables
+      {
+        const ModesSpace<QS> ws(P);
+        const BatchRve &rv = P.rves[sh.rid];
+        modes_setup<QS>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
+                        P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r);
+      }
+      // 2. the right-hand side's norm
+      double rn0;
+      {
+        const ModesSpace<QS> ws(P);
+        rn0 = rhs_norm(march_residual<CUBE, QS>(ws.w, reinterpret_cast<float *>(ws.r)).x,
+                       ws.w, ph);
+        ph ^= 1;
+      }
+      // 3. refinement
+      double rho = 0.0;
+      int outer = 0;
+      for (;;) {
+        double v[2];
+        {
+          const ModesSpace<QS> ws(P);
+          if (!QS && rho != 0.0) save_p(ws.q);
+          const double2 d = march_residual<CUBE, QS>(ws.w, reinterpret_cast<float *>(ws.r));
+          v[0] = d.x;
+          v[1] = d.y;
+          cta_sum<2>(v, ph);
+        }
+        relres = rn0 > 0.0 ? sqrt(v[0]) / rn0 : 0.0;
+        if (!(rn0 > 0.0 && sqrt(v[0]) > P.rtol * rn0) || outer >= P.max_outer) break;
+        const double fin = SP_FINAL_MARGIN * P.rtol * rn0;
+        const double thr = fmax(P.inner_rtol * P.inner_rtol * v[0], fin * fin);
+        // a reliable update: r is the true residual, the search direction
+        // goes on with beta = r.z / rho of the last step
+        {
+          const ModesSpace<QS> ws(P);
+          if (!QS) restore_p(ws.q, rho != 0.0);
+          update_p<CUBE, false>(ws.r, rho != 0.0 ? (float)(v[1] / rho) : 0.f);
+        }
+        rho = v[1];
+        __syncthreads();
+        int it = 0;
+        while (it < P.max_inner) {
+          {
+            const ModesSpace<QS> ws(P);
+            v[0] = march_apply<CUBE, QS>(ws.q);
+          }
+          double d[1] = {v[0]};
+          cta_sum<1>(d, ph);
+          {
+            const ModesSpace<QS> ws(P);
+            const double2 u =
+                update_xr<CUBE, QS>(ws.r, ws.x, ws.q, d[0] != 0.0 ? (float)(rho / d[0]) : 0.f, it == 0);
+            v[0] = u.x;
+            v[1] = u.y;
+          }
+          cta_sum<2>(v, ph);
+          it++;
+          if (v[1] <= thr) break;
+          {
+            const ModesSpace<QS> ws(P);
+            update_p<CUBE, QS>(ws.r, rho != 0.0 ? (float)(v[0] / rho) : 0.f);
+          }
+          rho = v[0];
+          __syncthreads();
+        }
+        if (it > 0) {
+          const ModesSpace<QS> ws(P);
+          update_w(ws.x, ws.w);
+        }
+        outer++;
+        if (threadIdx.x == 0) {
+          sh.inner += it;
+          sh.outer = outer;
+        }
+        __syncthreads();
+      }
+      // 4. averages
+      {
+        const ModesSpace<QS> ws(P);
+        ph = march_average(ws.w, ph);
+      }
+      if (threadIdx.x == 0) {
+        const size_t o = ((size_t)sh.rid * P.nrhs + sh.k) * 6;
+        modes_output(sh.red, P.out_stress + o, P.out_strain ? P.out_strain + o : nullptr);
+      }
+    }
+    if (threadIdx.x == 0) {
+      sp_solve_info in = {};
+      in.relres = relres;
+      in.status = sh.job != 1 ? SP_ERR_STATE : (relres <= P.rtol ? SP_OK : SP_ERR_NOCONV);
+      in.outer_its = sh.outer;
+      in.inner_its = sh.inner;
+      modes_report(in, P.task_info + (size_t)sh.rid * P.nrhs, sh.k, P.nrhs, P.done + sh.rid,
+                   P.out_info + sh.rid);
+    }
+    __syncthreads();
+  }
+}
+
+using ModesFn = void (*)(ModesParams);
+
+// the instantiated classes (threads, CTAs per SM, q in shared memory): the
+// largest blocks of which 6, 3, 2 and 1 fit an SM's register file
+#define SP_MODES_CLASSES(X) \
+  X(64, 8, true) X(160, 3, true) X(256, 2, true) X(512, 1, true) X(640, 1, false)
+#define SP_MODES_EXTERN(NT, MINB, QS) \
+  extern template __global__ void k_modes<NT, MINB, true, QS>(ModesParams); \
+  extern template __global__ void k_modes<NT, MINB, false, QS>(ModesParams);
+
+}  // namespace sp
