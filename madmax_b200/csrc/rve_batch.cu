@@ -215,7 +215,7 @@ struct sp_batch_s {
   size_t bytes = 0;
   TuneRecord tune;  // the autotuner's trial (tune.n == 0: shape fixed by the caller)
   int tune_slots = 0;  // work spaces allocated while the autotuner runs
-  // 512 x 1 FP32 stencil under affine conditions: RVEs the element-mode
+  // 512 x 1 FP32 stencil: RVEs the element-mode
   // kernel takes, in one launch per class; `rest` keep k_batch
   std::vector<MeshGeo> geo;      // per RVE
   std::vector<int> cls;          // per RVE: element-mode class or -1
@@ -227,9 +227,9 @@ struct sp_batch_s {
   ModesCommon mc;
 };
 
-// the shape whose FP32 affine stencil solves run the element-mode kernel
+// the shape whose FP32 stencil solves run the element-mode kernel
 static bool uses_modes(const sp_batch_opts &o, const Shape &s) {
-  return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op == SP_OP_STENCIL &&
+  return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op != SP_OP_ELL &&
          o.precision == SP_PREC_MIXED;
 }
 
@@ -286,7 +286,7 @@ static int tune_trial(sp_batch *b, const std::vector<Shape> &cands, const std::v
       split_rves(b, sample, &in, &rest);
       std::stable_sort(in.begin(), in.end(),
                        [&](int x, int y) { return b->geo[x].ndof > b->geo[y].ndof; });
-      rc = modes_plan(in, b->cls, b->geo, b->nrhs, d, &mk);
+      rc = modes_plan(in, b->cls, b->geo, b->nrhs, b->o.bc == SP_BC_PERIODIC, d, &mk);
       if (!rc) rc = modes_launch(mk, b->mc, b->d_mcount, s, true);
       P.nrve = (int)rest.size();
       if (!rc && !rest.empty() &&
@@ -491,7 +491,7 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
     b->etype_off.push_back(r.etype_off);
     b->nelm.push_back(g.nelm);
     b->geo.push_back(g);
-    b->cls.push_back(modes_class(g, descs[i].len));
+    b->cls.push_back(modes_class(g, descs[i].len, o.bc == SP_BC_PERIODIC));
   }
   // host-side classification into one pinned staging buffer
   uint8_t *et = nullptr;
@@ -687,7 +687,7 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
   }
   if (uses_modes(b->o, {b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)})) {
     b->nrest = (int)rest.size();
-    rc = modes_plan(in, b->cls, b->geo, nrhs, d, &b->modes);
+    rc = modes_plan(in, b->cls, b->geo, nrhs, o.bc == SP_BC_PERIODIC, d, &b->modes);
     if (!rc && b->nrest &&
         cudaMemcpy(b->d_rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice))
       rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");

@@ -10,12 +10,14 @@ SP_MODES_CLASSES(SP_MODES_EXTERN)
 struct ModesClass {
   int threads, minb;
   bool qs;
-  ModesFn fn[2];  // box elements, cubes
+  ModesFn fn[2][2];  // [periodic][box elements, cubes]
 };
 
 static const ModesClass kClasses[] = {
 #define SP_MODES_ROW(NT, MINB, QS) \
-  {NT, MINB, QS, {k_modes<NT, MINB, false, QS>, k_modes<NT, MINB, true, QS>}},
+  {NT, MINB, QS, \
+   {{k_modes<NT, MINB, false, QS, false>, k_modes<NT, MINB, true, QS, false>}, \
+    {k_modes<NT, MINB, false, QS, true>, k_modes<NT, MINB, true, QS, true>}}},
     SP_MODES_CLASSES(SP_MODES_ROW)
 #undef SP_MODES_ROW
 };
@@ -33,12 +35,14 @@ static int class_room(const ModesClass &k) {
 // An RVE runs on the smallest class whose threads hold one element column
 // each and whose shared memory holds its vectors beside the
 // class's other CTAs; it needs an interior node on every axis and at most 31
-// element layers (a column's materials are one 32-bit mask).  Larger RVEs
+// element layers, 30 under periodic conditions (a column's materials are one
+// 32-bit mask, which repeats two layers then).  Larger RVEs
 // keep the solve_rve kernel.
-int modes_class(const MeshGeo &g, const double *len) {
-  if (g.nex < 2 || g.ney < 2 || g.nez < 2 || g.nez > SP_MODES_MAX_NEZ) return -1;
+int modes_class(const MeshGeo &g, const double *len, bool per) {
+  if (g.nex < 2 || g.ney < 2 || g.nez < 2) return -1;
+  if (g.nez > (per ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ)) return -1;
   if ((long long)g.nex * g.ney > 640) return -1;
-  const ModesGeo G(g.nex, g.ney, g.nez);
+  const ModesGeo G(g.nex, g.ney, g.nez, per);
   const double hx = len[0] / g.nex, hy = len[1] / g.ney, hz = len[2] / g.nez;
   const int cube = hx == hy && hx == hz;
   for (int c = 0; c < kNumClasses; c++) {
@@ -49,7 +53,7 @@ int modes_class(const MeshGeo &g, const double *len) {
 }
 
 int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
-               const std::vector<MeshGeo> &geo, int nrhs, const Device *d,
+               const std::vector<MeshGeo> &geo, int nrhs, bool per, const Device *d,
                ModesPlan *out) {
   // classes with the largest RVEs first
   for (int c = 2 * kNumClasses - 1; c >= 0; c--) {
@@ -60,11 +64,11 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     const ModesClass &k = kClasses[c / 2];
     out->buckets.push_back(ModesBucket());
     ModesBucket &b = out->buckets.back();
-    b.fn = k.fn[c & 1];
+    b.fn = k.fn[per][c & 1];
     b.nrve = (int)ord.size();
     int ntot = 0, wlen = 0;
     for (int i : ord) {
-      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez);
+      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez, per);
       b.threads = std::max(b.threads, G.warps() * 32);
       b.smem = std::max(b.smem, G.smem(k.qs));
       ntot = std::max(ntot, G.ntot);

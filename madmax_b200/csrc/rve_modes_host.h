@@ -44,10 +44,10 @@ struct ModesCommon {
 };
 
 // The kernel class of an RVE (-1: none, the solve_rve kernel takes it)
-int modes_class(const MeshGeo &g, const double *len);
+int modes_class(const MeshGeo &g, const double *len, bool periodic);
 // Launches for the RVEs `ids` (largest first), every one of a class >= 0
 int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
-               const std::vector<MeshGeo> &geo, int nrhs, const Device *d,
+               const std::vector<MeshGeo> &geo, int nrhs, bool periodic, const Device *d,
                ModesPlan *out);
 void modes_free(ModesPlan *m);
 // counters: one per bucket, on the device

@@ -1,0 +1,9 @@
+// rve_modes_inst_box_per.cu -- instantiations of the element-mode batch kernel
+// (rve_modes_kernel.cuh) for box elements, periodic conditions.
+#include "rve_modes_kernel.cuh"
+
+namespace sp {
+#define SP_MODES_DEFINE(NT, MINB, QS) \
+  template __global__ void k_modes<NT, MINB, false, QS, true>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE)
+}  // namespace sp

@@ -4,6 +4,6 @@
 
 namespace sp {
 #define SP_MODES_DEFINE(NT, MINB, QS) \
-  template __global__ void k_modes<NT, MINB, true, QS>(ModesParams);
+  template __global__ void k_modes<NT, MINB, true, QS, false>(ModesParams);
 SP_MODES_CLASSES(SP_MODES_DEFINE)
 }  // namespace sp

@@ -56,23 +56,29 @@ struct ModesShared {
   double cc[2][CC_N];    // cube: lambda, mu, 2 mu, lambda/3, mu/3, (lambda + 4 mu)/9, times c0 a^2
   float2 c6[4][CC_N];    // ... as FP32 pairs: materials of the (lower, upper) layer
   unsigned col[SP_MODES_MAX_WARPS * 32];  // per column: bit e = material of layer e
-  int nex, ney, nez, nface, mz, h, ntot, wlen;
-  int job, rid, k, outer, inner, wcols, qoff, cntoff;  // qoff, cntoff: bytes from p on
+  int nex, ney, nez, nface, mz, h, ntot, wlen, threads;
+  int job, rid, k, outer, inner, wcols, qoff, cntoff, pad[3];  // qoff, cntoff: bytes from p on
 };
 static_assert(sizeof(ModesShared) % 16 == 0, "vectors follow on a 16-byte boundary");
 
-// sizes of one RVE's march
+// Sizes of one RVE's march.  Affine conditions: the interior planes, a row's
+// first node and a plane's first row being the boundary's zeros.  Periodic
+// conditions: every node of the periodic grid, neighbours wrapped; a row's
+// columns are preceded by a repetition of its last one, the left neighbour of
+// its first.
 struct ModesGeo {
-  int nex, ney, nez, nface, mz, h, ntot;
-  __host__ __device__ ModesGeo(int ex, int ey, int ez)
-      : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(ez - 1), h(ez / 2),
-        ntot((ez / 2) * ex * ey + ex + 2) {}
-  __host__ __device__ int wlen() const { return mz * nface + nex + 2; }
-  // columns of a warp: 32 where rows start at lane 0 (a row's first node is a
-  // boundary node, which needs no share from the lane below), else 31 and a
-  // repeated one
-  __host__ __device__ int wcols() const { return 32 % nex == 0 ? 32 : 31; }
-  __host__ __device__ int warps() const { return (nface + wcols() - 1) / wcols(); }
+  int nex, ney, nez, nface, mz, h, ntot, per;
+  __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic)
+      : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(periodic ? ez : ez - 1), h((mz + 1) / 2),
+        ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic) {}
+  __host__ __device__ int wlen() const { return mz * nface + (per ? 0 : nex + 2); }
+  // lanes of a row, of all rows, and of a warp: 32 where rows start at lane 0
+  // (whose left neighbour is the boundary, or its own repetition), else 31
+  // and a repetition of the last lane of the previous warp
+  __host__ __device__ int rowlanes() const { return per ? nex + 1 : nex; }
+  __host__ __device__ int lanes() const { return rowlanes() * ney; }
+  __host__ __device__ int wcols() const { return 32 % rowlanes() == 0 ? 32 : 31; }
+  __host__ __device__ int warps() const { return (lanes() + wcols() - 1) / wcols(); }
   // Dynamic shared memory: tables, p, then (QS) q, whose place the FP64
   // residual's face state and exchange planes take too, or (no q) two
   // exchange planes and the state in p's place; material counts.
@@ -126,23 +132,43 @@ __device__ __forceinline__ void cta_sum(double (&v)[NV], int &ph) {
 
 // A thread's place in the march.  f: its element column (face); the repeated
 // lanes and the padding threads of the last warp write nothing.
+template <bool PER>
 struct ModesLane {
   int f;
+  int dx, dy;    // from f to the columns at x + 1 and y + 1
   bool warp_on;  // the warp has a column
   bool column;   // the thread has one
-  bool owner;    // ... and its node (ex, ey) is an interior one
-  int threads;   // of all warps that have a column
+  bool owner;    // ... and its node (ex, ey) is an unknown
   __device__ __forceinline__ ModesLane() {
     const ModesShared &sh = msh();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rep = 32 - sh.wcols;
-    const int i = warp * sh.wcols + lane - rep;
-    warp_on = warp * sh.wcols < sh.nface;
-    column = lane >= rep && i < sh.nface;
-    f = min(max(i, 0), sh.nface - 1);
-    owner = column && f >= sh.nex && f % sh.nex != 0;
-    threads = (sh.nface + sh.wcols - 1) / sh.wcols * 32;
+    const int i = warp * sh.wcols + lane - rep, row = PER ? sh.nex + 1 : sh.nex;
+    const int n = row * sh.ney, ic = min(max(i, 0), n - 1);
+    warp_on = warp * sh.wcols < n;
+    column = lane >= rep && i < n;
+    if (PER) {
+      const int y = ic / row, v = ic - y * row, x = v ? v - 1 : sh.nex - 1;
+      f = y * sh.nex + x;
+      dx = x == sh.nex - 1 ? 1 - sh.nex : 1;
+      dy = y == sh.ney - 1 ? sh.nex - sh.nface : sh.nex;
+      column = column && v != 0;
+      owner = column;
+    } else {
+      f = ic;
+      dx = 1;
+      dy = sh.nex;
+      owner = column && f >= sh.nex && f % sh.nex != 0;
+    }
   }
 };
+
+// the columns at x - 1 and y - 1 of an owner's column
+template <bool PER>
+__device__ __forceinline__ void modes_below(int f, int &left, int &down) {
+  const ModesShared &sh = msh();
+  left = PER && f % sh.nex == 0 ? sh.nex - 1 : -1;
+  down = PER && f < sh.nex ? sh.nface - sh.nex : -sh.nex;
+}
 
 // Barrier over the warps that have columns
 __device__ __forceinline__ void plane_sync(int threads) {
@@ -152,13 +178,13 @@ __device__ __forceinline__ void plane_sync(int threads) {
 
 // q = A p: p, q in shared memory ([slot][3] pairs), q in qg ([3][ntot]) when
 // QS is false; returns the thread's share of p.q.
-template <bool CUBE, bool QS>
+template <bool CUBE, bool QS, bool PER>
 __device__ __noinline__ double march_apply(float2 *qg) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   const unsigned mats = sh.col[T.f];
   const int nface = sh.nface, nf3 = 3 * nface, h = sh.h, ntot = sh.ntot;
-  const int up = 3 * sh.nex;
+  const int right = PER ? 3 * T.dx : 3, up = 3 * T.dy;
   const F2 *pf = mp() + 3 * T.f;  // corner (0, 0) of slot 0
   F2 *const qf = mq() + 3 * T.f;
   const bool odd = (sh.mz & 1) != 0;
@@ -167,13 +193,14 @@ __device__ __noinline__ double march_apply(float2 *qg) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       raw[c][0] = a[c];
-      raw[c][1] = a[3 + c];
+      raw[c][1] = a[right + c];
       raw[c][2] = a[up + c];
-      raw[c][3] = a[up + 3 + c];
+      raw[c][3] = a[up + right + c];
     }
   };
-  // values of step s: slot s; above slot h - 1 lies plane h (lower half), the
-  // boundary plane (upper half)
+  // values of step s: slot s; above slot h - 1 lies plane h (lower half) and
+  // the boundary plane (upper half), or plane 0 under periodic conditions
+  // (for an odd number of planes, already at slot h - 1)
   auto next = [&](int s) {
     load(s < h ? pf + s * nf3 : pf);
     if (s >= h) {
@@ -181,17 +208,35 @@ __device__ __noinline__ double march_apply(float2 *qg) {
 #pragma unroll
       for (int c = 0; c < 3; c++)
 #pragma unroll
-        for (int m = 0; m < 4; m++) raw[c][m] = mk2(raw[c][m].v.y, 0.f);
+        for (int m = 0; m < 4; m++) raw[c][m] = mk2(raw[c][m].v.y, PER ? raw[c][m].v.x : 0.f);
+    }
+    if (PER && odd && s == h - 1) {
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        raw[c][0].v.y = pf[c].v.x;
+        raw[c][1].v.y = pf[right + c].v.x;
+        raw[c][2].v.y = pf[up + c].v.x;
+        raw[c][3].v.y = pf[up + right + c].v.x;
+      }
     }
   };
   if (T.warp_on) {
-    // below slot 0: the boundary plane (lower half), plane h - 1 (upper half)
+    // below slot 0: the boundary plane, or the last one (lower half); plane
+    // h - 1 (upper half)
+    if (PER) {
+      load(pf + (odd ? h - 2 : h - 1) * nf3);
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) acc[c][m].v.x = raw[c][m].v.y;
+    }
     load(pf + (h - 1) * nf3);
 #pragma unroll
     for (int c = 0; c < 3; c++)
 #pragma unroll
       for (int m = 0; m < 4; m++) {
-        raw[c][m] = mk2(0.f, raw[c][m].v.x);
+        raw[c][m] = mk2(PER ? acc[c][m].v.x : 0.f, raw[c][m].v.x);
         acc[c][m] = mk2(0.f, 0.f);
       }
     face_modes(raw, Fa);
@@ -220,14 +265,14 @@ __device__ __noinline__ double march_apply(float2 *qg) {
       // the upper row's share waits where that row's q goes (QS), or in the
       // exchange planes in turn
       F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3 + up;
-      if (T.column && s > 0 && T.f + sh.nex < nface)
+      if (T.column && s > 0 && (PER || T.f + sh.nex < nface))
 #pragma unroll
         for (int c = 0; c < 3; c++) e[c] = high[c];
       // with registers to spare, the next slot's values before the barrier
       if (QS) next(s + 1);
     }
     if (s > 0) {
-      plane_sync(T.threads);
+      plane_sync(sh.threads);
       if (T.owner) {
         F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3;
         const F2 *ps = pf + (s - 1) * nf3;
@@ -236,6 +281,7 @@ __device__ __noinline__ double march_apply(float2 *qg) {
         for (int c = 0; c < 3; c++) {
           low[c] = low[c] + e[c];
           if (odd && s == h) low[c].v.y = 0.f;  // no plane there
+          if (PER && s == 1 && T.f == 0) low[c].v.x = 0.f;  // the fixed node
           if constexpr (QS)
             e[c] = low[c];
           else
@@ -263,12 +309,12 @@ __device__ __noinline__ double march_apply(float2 *qg) {
 // between layers: in registers they spill, and a spill goes to L2, since the
 // vectors leave L1 next to nothing (n = 20: 285k cycles an evaluation with
 // spills, 80k without).
-template <bool CUBE, bool QS>
+template <bool CUBE, bool QS, bool PER>
 __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   const unsigned mats = sh.col[T.f];
-  const int nface = sh.nface, nex = sh.nex, wl = sh.wlen, mz = sh.mz, h = sh.h;
+  const int nface = sh.nface, right = PER ? T.dx : 1, up = T.dy, wl = sh.wlen, mz = sh.mz, h = sh.h;
   double *const ex = reinterpret_cast<double *>(mq());  // two exchange planes
   const uint8_t *const cnt = mcnt();
   // [c][m] of the running forces at 4 c + m, of the face's modes 12 further;
@@ -283,17 +329,29 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       raw[c][0] = a[c * wl];
-      raw[c][1] = a[c * wl + 1];
-      raw[c][2] = a[c * wl + nex];
-      raw[c][3] = a[c * wl + nex + 1];
+      raw[c][1] = a[c * wl + right];
+      raw[c][2] = a[c * wl + up];
+      raw[c][3] = a[c * wl + up + right];
     }
   };
-  if (T.warp_on) {
-#pragma unroll
-    for (int j = 0; j < (QS ? 12 : 24); j++) state[j] = 0.0;
-    load(0);
-  }
   if (!T.warp_on) return make_double2(0.0, 0.0);
+#pragma unroll
+  for (int j = 0; j < (QS ? 12 : 24); j++) state[j] = 0.0;
+  if (PER) {  // below plane 0 lies the last one
+    load(mz - 1);
+    double F[3][4];
+    face_modes(raw, F);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        if (QS)
+          F0[c][m] = F[c][m];
+        else
+          state[12 + 4 * c + m] = F[c][m];
+      }
+  }
+  load(0);
 #pragma unroll 1
   for (int s = 0; s <= mz; s++) {
     double low[3];
@@ -326,7 +384,8 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
         const double *ct = sh.cd[(mats >> s) & 1u];
         modes_box(S, D, [ct](int i) { return ct[i]; });
       }
-      double *e = exs + 3 * T.f;
+      double *e = exs + 3 * (T.f + up);
+      const bool put = T.column && (PER || T.f + up < nface);
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         double *const ac = state + 4 * c;
@@ -340,11 +399,11 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
         ac[3] = S[c][2] + D[c][3];
         double high;
         plane_back(t0, t1, t2, t3, low[c], high);
-        if (T.column) e[c] = high;
+        if (put) e[c] = high;
       }
     }
-    if (s + 1 < mz) {
-      load(s + 1);
+    if (PER || s + 1 < mz) {
+      load(PER && s + 1 >= mz ? 0 : s + 1);
     } else {
       __syncwarp();
 #pragma unroll
@@ -353,9 +412,9 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
         for (int m = 0; m < 4; m++) raw[c][m] = 0.0;
     }
     if (s > 0) {
-      plane_sync(T.threads);
+      plane_sync(sh.threads);
       if (T.owner) {
-        const double *e = exs + 3 * (T.f - nex);
+        const double *e = exs + 3 * T.f;
         const bool hi = s - 1 >= h;
         const int i = (hi ? s - 1 - h : s - 1) * nface + T.f;
         const unsigned cv = cnt[i];
@@ -364,7 +423,8 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
         float *ro = rg + 2 * i + (hi ? 1 : 0);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          const double b = -(low[c] + e[c]);
+          double b = -(low[c] + e[c]);
+          if (PER && s == 1 && T.f == 0) b = 0.0;  // the fixed node
           const float bf = (float)b;
           ro[2 * c * sh.ntot] = bf;
           n2 += b * b;
@@ -383,17 +443,20 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
 // above.  (Over all elements the weights vanish: the mean strain is eps.)
 // m[9]: the number of fibre elements.
 // Summed over the CTA; thread 0 gets the totals.
-__device__ __noinline__ inline int march_average(const double *w, int ph) {
+template <bool PER>
+__device__ __noinline__ int march_average(const double *w, int ph) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   double m[10];
 #pragma unroll
   for (int q = 0; q < 10; q++) m[q] = 0.0;
-  if (T.column) m[9] = (double)__popc(sh.col[T.f]);
+  if (T.column) m[9] = (double)__popc(sh.col[T.f] & ~(PER ? (1u | 2u << sh.nez) : 0u));
   if (T.owner) {
     const int wl = sh.wlen, mz = sh.mz, nface = sh.nface;
-    const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f - 1], c1 = sh.col[T.f - sh.nex],
-                   c0 = sh.col[T.f - sh.nex - 1];
+    int left, down;
+    modes_below<PER>(T.f, left, down);
+    const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f + left], c1 = sh.col[T.f + down],
+                   c0 = sh.col[T.f + left + down];
 #pragma unroll 4
     for (int pl = 0; pl < mz; pl++) {
       const unsigned b0 = (c0 >> pl) & 3u, b1 = (c1 >> pl) & 3u, b2 = (c2 >> pl) & 3u,
@@ -480,10 +543,10 @@ __device__ __forceinline__ void xr_slots(int s0, int f, float2 *rg, float2 *xg, 
 // correction's first step); returns its shares of r.z and r.r.  x is added to
 // in L2: only this thread touches its entries.  q's slots take the new r for
 // the direction update.
-template <bool CUBE, bool QS>
+template <bool CUBE, bool QS, bool PER>
 __device__ __noinline__ double2 update_xr(float2 *rg, float2 *xg, const float2 *qg, float alpha,
                                           bool first) {
-  const ModesLane T;
+  const ModesLane<PER> T;
   if (!T.owner) return make_double2(0.0, 0.0);
   const int h = msh().h;
   const F2 al = mk2(alpha, alpha), nal = mk2(-alpha, -alpha);
@@ -527,9 +590,9 @@ __device__ __forceinline__ void p_slots(int s0, int f, const float2 *rg, F2 be, 
   }
 }
 
-template <bool CUBE, bool LOCAL>
+template <bool CUBE, bool LOCAL, bool PER>
 __device__ __noinline__ void update_p(const float2 *rg, float beta) {
-  const ModesLane T;
+  const ModesLane<PER> T;
   if (!T.owner) return;
   const int h = msh().h;
   const F2 be = mk2(beta, beta);
@@ -539,9 +602,10 @@ __device__ __noinline__ void update_p(const float2 *rg, float beta) {
 }
 
 // w += x in FP64 over the thread's column
-__device__ __noinline__ inline void update_w(const float2 *xg, double *w) {
+template <bool PER>
+__device__ __noinline__ void update_w(const float2 *xg, double *w) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   if (!T.owner) return;
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h, mz = sh.mz, wl = sh.wlen;
 #pragma unroll 1
@@ -566,9 +630,10 @@ __device__ __noinline__ inline void update_w(const float2 *xg, double *w) {
 // The residual's face state takes p's place when q is not in shared memory:
 // every column's p waits in q's global work space meanwhile, the padding is
 // zeroed anew.
-__device__ __noinline__ inline void save_p(float2 *qg) {
+template <bool PER>
+__device__ __noinline__ void save_p(float2 *qg) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   if (T.owner)
     for (int s = 0; s < sh.h; s++)
 #pragma unroll
@@ -578,9 +643,10 @@ __device__ __noinline__ inline void save_p(float2 *qg) {
       }
   __syncthreads();
 }
-__device__ __noinline__ inline void restore_p(const float2 *qg, bool saved) {
+template <bool PER>
+__device__ __noinline__ void restore_p(const float2 *qg, bool saved) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   for (int i = threadIdx.x; i < 3 * sh.ntot; i += blockDim.x) mp()[i] = mk2(0.f, 0.f);
   __syncthreads();
   if (T.owner && saved)
@@ -593,13 +659,13 @@ __device__ __noinline__ inline void restore_p(const float2 *qg, bool saved) {
 }
 
 // the tables, materials and start vectors of one load case
-template <bool QS>
+template <bool QS, bool PER>
 __device__ __noinline__ void modes_setup(const double *len, const double *mat,
                                          const uint8_t *etype, const double *eps, double *w,
                                          float2 *rg) {
   ModesShared &sh = msh();
   const int t = threadIdx.x;
-  const ModesLane T;
+  const ModesLane<PER> T;
   const int nface = sh.nface, nex = sh.nex, wl = sh.wlen;
   if (t < 3) {
     const int n = t == 0 ? sh.nex : (t == 1 ? sh.ney : sh.nez);
@@ -622,6 +688,9 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
   const uint8_t *et = etype + T.f;
   if (T.warp_on)
     for (int e = 0; e < sh.nez; e++) mats |= (unsigned)__ldg(et + e * nface) << e;
+  // bit s: the layer below plane s.  Periodic: layer s - 1, and the first
+  // ones again past the last
+  if (PER) mats = mats << 1 | mats >> (sh.nez - 1) | (mats & 1u) << (sh.nez + 1);
   if (T.column) sh.col[T.f] = mats;
   {
     float4 *p = reinterpret_cast<float4 *>(mp());  // (3 ntot pairs, rounded down to 16 bytes)
@@ -629,21 +698,24 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
     if (t == 0) mp()[3 * sh.ntot - 1] = mk2(0.f, 0.f);
   }
   // w's padding: the columns without an interior node and the row past the end
-  if (T.column && !T.owner)
+  if (T.column && (PER || !T.owner))
     for (int c = 0; c < 3; c++)
       for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = 0.0;
-  for (int i = t; i < 3 * (nex + 2); i += blockDim.x)
-    w[(i / (nex + 2)) * wl + sh.mz * nface + i % (nex + 2)] = 0.0;
+  if (!PER)
+    for (int i = t; i < 3 * (nex + 2); i += blockDim.x)
+      w[(i / (nex + 2)) * wl + sh.mz * nface + i % (nex + 2)] = 0.0;
   __syncthreads();
-  if (t < 2 * MC_N)
-    sh.cd[t / MC_N][t % MC_N] = mode_coef(t % MC_N, sh.lame[t / MC_N][0], sh.lame[t / MC_N][1],
+  for (int i = t; i < 2 * MC_N; i += blockDim.x)
+    sh.cd[i / MC_N][i % MC_N] = mode_coef(i % MC_N, sh.lame[i / MC_N][0], sh.lame[i / MC_N][1],
                                           sh.hx[0] * sh.hx[1] * sh.hx[2] / 16.0, sh.a);
   if (t < 9) sh.A[t] = 4.0 * sh.hx[t % 3] * sh.E[t];
-  // fibre elements around the column's nodes; start of the right-hand side's
-  // own residual: w = -eps.x inside, i.e. u = 0 inside
+  // fibre elements around the column's nodes; affine conditions: start of the
+  // right-hand side's own residual, w = -eps.x inside, i.e. u = 0 inside
   if (T.owner) {
-    const unsigned m0 = mats, m1 = sh.col[T.f - 1], m2 = sh.col[T.f - nex],
-                   m3 = sh.col[T.f - nex - 1];
+    int left, down;
+    modes_below<PER>(T.f, left, down);
+    const unsigned m0 = mats, m1 = sh.col[T.f + left], m2 = sh.col[T.f + down],
+                   m3 = sh.col[T.f + left + down];
     auto count = [&](int pl) {
       return __popc((m0 >> pl) & 3u) + __popc((m1 >> pl) & 3u) + __popc((m2 >> pl) & 3u) +
              __popc((m3 >> pl) & 3u);
@@ -654,15 +726,16 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double xy = sh.E[3 * c] * X + sh.E[3 * c + 1] * Y, ez = sh.E[3 * c + 2] * sh.hx[2];
-      for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
+      if (!PER)
+        for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
       // a slot without an upper plane keeps a zero there
       rg[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
     }
   }
   __syncthreads();
-  if (t >= 32 && t < 34) {
-    const double *C = sh.cd[t - 32];
-    double *k = sh.cc[t - 32];
+  if (t < 2) {
+    const double *C = sh.cd[t];
+    double *k = sh.cc[t];
     k[CC_LAM] = C[MC_BXY];
     k[CC_MU] = C[MC_MXX];
     k[CC_MU2] = 2.0 * C[MC_MXX];
@@ -735,13 +808,15 @@ struct ModesSpace {
   }
 };
 
-// norm of the right-hand side (u = 0 inside, as modes_setup left w) from its
-// square and the column's share; one at the round-off level of its own
-// cancelling terms is zero, and its load case is solved with u = 0.  Else
+// Norm of the right-hand side from the thread's share of its square (affine
+// conditions: of u = 0 inside, as modes_setup left w; periodic ones: of the
+// zero fluctuation, w = 0); one at the round-off level of its own
+// cancelling terms is zero, and its load case is solved with that.  Else
 // w = 0: the affine field starts.
-__device__ __noinline__ inline double rhs_norm(double n2, double *w, int ph) {
+template <bool PER>
+__device__ __noinline__ double rhs_norm(double n2, double *w, int ph) {
   const ModesShared &sh = msh();
-  const ModesLane T;
+  const ModesLane<PER> T;
   double v[2] = {n2, 0.0};
   if (T.owner)
     for (int s = 0; s < sh.h; s++) {
@@ -757,7 +832,7 @@ __device__ __noinline__ inline double rhs_norm(double n2, double *w, int ph) {
                       fabs(sh.E[3 * c + 2]) * sh.len[2]);
   double rn0 = sqrt(v[0]);
   if (rn0 <= SP_RHS_FLOOR * sqrt(v[1]) * um) rn0 = 0.0;
-  if (rn0 > 0.0 && T.owner)
+  if (!PER && rn0 > 0.0 && T.owner)
     for (int c = 0; c < 3; c++)
       for (int pl = 0; pl < sh.mz; pl++) w[c * sh.wlen + pl * sh.nface + T.f] = 0.0;
   __syncthreads();
@@ -787,8 +862,8 @@ __device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_sol
 }
 
 // NT threads at most, MINB CTAs per SM; CUBE: equal element edges; QS: q in
-// shared memory
-template <int NT, int MINB, bool CUBE, bool QS>
+// shared memory; PER: periodic conditions
+template <int NT, int MINB, bool CUBE, bool QS, bool PER>
 __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
   ModesShared &sh = msh();
   if (dynamic_smem_bytes() < sizeof(ModesShared)) return;
@@ -801,9 +876,10 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.rid = P.order[task / P.nrhs];
         sh.k = task % P.nrhs;
         const MeshGeo &mg = P.plans[P.rves[sh.rid].plan].geo;
-        const ModesGeo G(mg.nex, mg.ney, mg.nez);
+        const ModesGeo G(mg.nex, mg.ney, mg.nez, PER);
         if (dynamic_smem_bytes() < (unsigned)G.smem(QS) || G.warps() * 32 > blockDim.x ||
-            G.warps() > SP_MODES_MAX_WARPS || G.nez > SP_MODES_MAX_NEZ)
+            G.warps() > SP_MODES_MAX_WARPS || G.nez > (PER ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ) ||
+            G.nface > SP_MODES_MAX_WARPS * 32)
           sh.job = 2;  // launched with less than this RVE needs
         sh.nex = G.nex;
         sh.ney = G.ney;
@@ -814,6 +890,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.ntot = G.ntot;
         sh.wlen = G.wlen();
         sh.wcols = G.wcols();
+        sh.threads = 32 * G.warps();
         sh.qoff = G.pbytes(QS);
         sh.cntoff = G.pbytes(QS) + G.qbytes(QS);
         sh.outer = sh.inner = 0;
@@ -827,15 +904,15 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       {
         const ModesSpace<QS> ws(P);
         const BatchRve &rv = P.rves[sh.rid];
-        modes_setup<QS>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
+        modes_setup<QS, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
                         P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r);
       }
       // 2. the right-hand side's norm
       double rn0;
       {
         const ModesSpace<QS> ws(P);
-        rn0 = rhs_norm(march_residual<CUBE, QS>(ws.w, reinterpret_cast<float *>(ws.r)).x,
-                       ws.w, ph);
+        rn0 = rhs_norm<PER>(
+            march_residual<CUBE, QS, PER>(ws.w, reinterpret_cast<float *>(ws.r)).x, ws.w, ph);
         ph ^= 1;
       }
       // 3. refinement
@@ -845,8 +922,8 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         double v[2];
         {
           const ModesSpace<QS> ws(P);
-          if (!QS && rho != 0.0) save_p(ws.q);
-          const double2 d = march_residual<CUBE, QS>(ws.w, reinterpret_cast<float *>(ws.r));
+          if (!QS && rho != 0.0) save_p<PER>(ws.q);
+          const double2 d = march_residual<CUBE, QS, PER>(ws.w, reinterpret_cast<float *>(ws.r));
           v[0] = d.x;
           v[1] = d.y;
           cta_sum<2>(v, ph);
@@ -859,8 +936,8 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         // goes on with beta = r.z / rho of the last step
         {
           const ModesSpace<QS> ws(P);
-          if (!QS) restore_p(ws.q, rho != 0.0);
-          update_p<CUBE, false>(ws.r, rho != 0.0 ? (float)(v[1] / rho) : 0.f);
+          if (!QS) restore_p<PER>(ws.q, rho != 0.0);
+          update_p<CUBE, false, PER>(ws.r, rho != 0.0 ? (float)(v[1] / rho) : 0.f);
         }
         rho = v[1];
         __syncthreads();
@@ -868,14 +945,14 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         while (it < P.max_inner) {
           {
             const ModesSpace<QS> ws(P);
-            v[0] = march_apply<CUBE, QS>(ws.q);
+            v[0] = march_apply<CUBE, QS, PER>(ws.q);
           }
           double d[1] = {v[0]};
           cta_sum<1>(d, ph);
           {
             const ModesSpace<QS> ws(P);
             const double2 u =
-                update_xr<CUBE, QS>(ws.r, ws.x, ws.q, d[0] != 0.0 ? (float)(rho / d[0]) : 0.f, it == 0);
+                update_xr<CUBE, QS, PER>(ws.r, ws.x, ws.q, d[0] != 0.0 ? (float)(rho / d[0]) : 0.f, it == 0);
             v[0] = u.x;
             v[1] = u.y;
           }
@@ -884,14 +961,14 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
           if (v[1] <= thr) break;
           {
             const ModesSpace<QS> ws(P);
-            update_p<CUBE, QS>(ws.r, rho != 0.0 ? (float)(v[0] / rho) : 0.f);
+            update_p<CUBE, QS, PER>(ws.r, rho != 0.0 ? (float)(v[0] / rho) : 0.f);
           }
           rho = v[0];
           __syncthreads();
         }
         if (it > 0) {
           const ModesSpace<QS> ws(P);
-          update_w(ws.x, ws.w);
+          update_w<PER>(ws.x, ws.w);
         }
         outer++;
         if (threadIdx.x == 0) {
@@ -903,7 +980,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       // 4. averages
       {
         const ModesSpace<QS> ws(P);
-        ph = march_average(ws.w, ph);
+        ph = march_average<PER>(ws.w, ph);
       }
       if (threadIdx.x == 0) {
         const size_t o = ((size_t)sh.rid * P.nrhs + sh.k) * 6;
@@ -930,7 +1007,9 @@ using ModesFn = void (*)(ModesParams);
 #define SP_MODES_CLASSES(X) \
   X(64, 8, true) X(160, 3, true) X(256, 2, true) X(512, 1, true) X(640, 1, false)
 #define SP_MODES_EXTERN(NT, MINB, QS) \
-  extern template __global__ void k_modes<NT, MINB, true, QS>(ModesParams); \
-  extern template __global__ void k_modes<NT, MINB, false, QS>(ModesParams);
+  extern template __global__ void k_modes<NT, MINB, true, QS, false>(ModesParams); \
+  extern template __global__ void k_modes<NT, MINB, false, QS, false>(ModesParams); \
+  extern template __global__ void k_modes<NT, MINB, true, QS, true>(ModesParams); \
+  extern template __global__ void k_modes<NT, MINB, false, QS, true>(ModesParams);
 
 }  // namespace sp

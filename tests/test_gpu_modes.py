@@ -54,6 +54,57 @@ def test_edges_match_oracle(cube):
         assert np.allclose(strain[i], eps[i], rtol=0, atol=1e-15), MESHES[i]
 
 
+@pytest.mark.parametrize("periodic", [False, True])
+def test_one_warp_launch(periodic):
+    """A launch whose largest RVE needs one warp (the tables are filled by as
+    few threads), affine and periodic, against the oracles."""
+    from oracle import periodic as PER
+    d = mb.rve_desc(4, 0.3, (1e9, 3e10), (0.31, 0.22))
+    s, _, info = mb.Batch([d], rtol=1e-10, threads=512, ctas_per_sm=1,
+                          bc=mb.SP_BC_PERIODIC if periodic else mb.SP_BC_AFFINE).homogenize()
+    m = O.cube_mesh(4)
+    et = O.fiber_types(m, [1, 1], d.radius)
+    if periodic:
+        _, st, _ = PER.homogenize_periodic(m, et, tuple(d.E), tuple(d.nu), np.eye(6))
+    else:
+        _, st, _, _ = O.homogenize(m, et, tuple(d.E), tuple(d.nu), np.eye(6), rtol=1e-12,
+                                   lin_rtol=1e-13)
+    assert info[0].status == 0
+    assert np.abs(s[0] - st).max() <= 1e-8 * np.abs(st).max()
+
+
+PER_MESHES = [(2, 2, 2), (3, 2, 3), (2, 5, 4), (7, 7, 5), (15, 4, 6), (8, 8, 7), (31, 3, 2),
+              (17, 17, 3), (4, 3, 30), (4, 3, 31), (24, 24, 2), (25, 25, 2)]
+
+
+@pytest.mark.parametrize("cube", [True, False])
+def test_periodic_edges_match_fp64(cube):
+    """Periodic conditions: rows that start at lane 0 or straddle warps, odd
+    and even plane counts (the halves' seams), 30 and 31 layers, the largest
+    classes, on random voxel materials; against the FP64 periodic batch (which
+    is tested against the periodic oracle), both solved to 1e-10."""
+    rng = np.random.default_rng(41 + cube)
+    descs, ets = [], []
+    for n in PER_MESHES:
+        edge = rng.uniform(0.05, 0.2, 3)
+        ln = [n[k] / 8.0 if cube else n[k] * edge[k] for k in range(3)]
+        descs.append(mb.rve_desc(n, 0.2, (1e9, 1e9 * float(rng.uniform(2, 100))), (0.3, 0.25), ln))
+        ets.append((rng.random(n[0] * n[1] * n[2]) < 0.4).astype(np.uint8))
+    eps = rng.normal(0, 1e-3, (len(descs), 3, 6))
+    out = []
+    for kw in ({"threads": 512, "ctas_per_sm": 1}, {"precision": mb.SP_PREC_FP64, "threads": 512,
+                                                    "ctas_per_sm": 2}):
+        b = mb.Batch(descs, nrhs=3, rtol=1e-10, bc=mb.SP_BC_PERIODIC, **kw)
+        for i, et in enumerate(ets):
+            b.set_etype(i, et)
+        s, strain, info = b.homogenize(np.ascontiguousarray(eps))
+        assert (mb.info_array(info)["status"] == 0).all()
+        assert np.allclose(strain, eps, rtol=0, atol=1e-14)
+        out.append(s)
+    for i in range(len(descs)):
+        assert np.abs(out[0][i] - out[1][i]).max() <= 1e-8 * np.abs(out[1][i]).max(), PER_MESHES[i]
+
+
 def test_trivial_load_cases():
     """A zero strain gives zero stress, and a homogeneous RVE is solved by the
     affine start: no CG iteration, stress = D strain."""
