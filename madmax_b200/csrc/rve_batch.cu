@@ -215,7 +215,7 @@ struct sp_batch_s {
   size_t bytes = 0;
   TuneRecord tune;  // the autotuner's trial (tune.n == 0: shape fixed by the caller)
   int tune_slots = 0;  // work spaces allocated while the autotuner runs
-  // 512 x 1 FP32 stencil: RVEs the element-mode
+  // 512 x 1 stencil: RVEs the element-mode
   // kernel takes, in one launch per class; `rest` keep k_batch
   std::vector<MeshGeo> geo;      // per RVE
   std::vector<int> cls;          // per RVE: element-mode class or -1
@@ -227,10 +227,9 @@ struct sp_batch_s {
   ModesCommon mc;
 };
 
-// the shape whose FP32 stencil solves run the element-mode kernel
-static bool uses_modes(const sp_batch_opts &o, const Shape &s) {
-  return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op != SP_OP_ELL &&
-         o.precision == SP_PREC_MIXED;
+// the shape whose stencil solves run the element-mode kernel
+static bool uses_modes(const Shape &s) {
+  return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op != SP_OP_ELL;
 }
 
 static void split_rves(const sp_batch *b, const std::vector<int> &order, std::vector<int> *in,
@@ -279,14 +278,15 @@ static int tune_trial(sp_batch *b, const std::vector<Shape> &cands, const std::v
     if (grid / cands[c].cluster > b->tune_slots) continue;  // work spaces sized for fewer
     BatchParams P = b->P;
     P.order = d_trial;
-    if (uses_modes(b->o, cands[c])) {
+    if (uses_modes(cands[c])) {
       // the element-mode kernel on the RVEs it takes, k_batch on the rest
       std::vector<int> in, rest;
       ModesPlan mk;
       split_rves(b, sample, &in, &rest);
       std::stable_sort(in.begin(), in.end(),
                        [&](int x, int y) { return b->geo[x].ndof > b->geo[y].ndof; });
-      rc = modes_plan(in, b->cls, b->geo, b->nrhs, b->o.bc == SP_BC_PERIODIC, d, &mk);
+      rc = modes_plan(in, b->cls, b->geo, b->nrhs, b->o.bc == SP_BC_PERIODIC,
+                      b->o.precision == SP_PREC_FP64, d, &mk);
       if (!rc) rc = modes_launch(mk, b->mc, b->d_mcount, s, true);
       P.nrve = (int)rest.size();
       if (!rc && !rest.empty() &&
@@ -491,7 +491,8 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
     b->etype_off.push_back(r.etype_off);
     b->nelm.push_back(g.nelm);
     b->geo.push_back(g);
-    b->cls.push_back(modes_class(g, descs[i].len, o.bc == SP_BC_PERIODIC));
+    b->cls.push_back(modes_class(g, descs[i].len, o.bc == SP_BC_PERIODIC,
+                                  o.precision == SP_PREC_FP64));
   }
   // host-side classification into one pinned staging buffer
   uint8_t *et = nullptr;
@@ -576,7 +577,7 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
   if (!rc) rc = dmalloc((void **)&b->d_strain, (size_t)nrve * nrhs * 6 * sizeof(double), acct);
   if (!rc) rc = dmalloc((void **)&b->d_info, (size_t)nrve * sizeof(sp_solve_info), acct);
   const Shape wide{512, 1, 1, kernel_op(o)};
-  const bool modes = uses_modes(o, wide) && o.cluster <= 1 &&
+  const bool modes = uses_modes(wide) && o.cluster <= 1 &&
                      (trial || (o.threads == 512 && o.ctas_per_sm == 1));
   if (!rc && modes) {
     rc = dmalloc((void **)&b->d_rest, nrve * sizeof(int), acct);
@@ -662,7 +663,7 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
       g_tune_cache[tkey] = b->tune;
     }
     // keep only the work spaces the chosen grid uses
-    const bool none = uses_modes(b->o, {b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)}) &&
+    const bool none = uses_modes({b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)}) &&
                       rest.empty();
     const size_t keep = none ? 0 : (size_t)(b->grid / b->o.cluster);
     if (!rc && keep < slots) {
@@ -685,9 +686,10 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
       return rc;
     }
   }
-  if (uses_modes(b->o, {b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)})) {
+  if (uses_modes({b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)})) {
     b->nrest = (int)rest.size();
-    rc = modes_plan(in, b->cls, b->geo, nrhs, o.bc == SP_BC_PERIODIC, d, &b->modes);
+    rc = modes_plan(in, b->cls, b->geo, nrhs, o.bc == SP_BC_PERIODIC, o.precision == SP_PREC_FP64, d,
+                    &b->modes);
     if (!rc && b->nrest &&
         cudaMemcpy(b->d_rest, rest.data(), rest.size() * sizeof(int), cudaMemcpyHostToDevice))
       rc = sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
@@ -749,7 +751,7 @@ extern "C" int sp_batch_launch(sp_batch *b, void *stream) {
   cudaStream_t s = pick_stream(stream, d);
   Shape sh{b->o.threads, b->o.ctas_per_sm, b->o.cluster, kernel_op(b->o)};
   BatchFn fn = pick(b->o.precision, b->nrhs, sh);
-  if (uses_modes(b->o, sh)) {
+  if (uses_modes(sh)) {
     SP_TRY(modes_launch(b->modes, b->mc, b->d_mcount, s));
     b->last_launches = (int)b->modes.buckets.size();
     if (b->nrest) {

@@ -5,21 +5,24 @@
 
 namespace sp {
 
-SP_MODES_CLASSES(SP_MODES_EXTERN)
+SP_MODES_CLASSES(SP_MODES_EXTERN, F2)
+SP_MODES_CLASSES(SP_MODES_EXTERN, double)
 
 struct ModesClass {
   int threads, minb;
   bool qs;
-  ModesFn fn[2][2];  // [periodic][box elements, cubes]
+  ModesFn fn[2][2][2];  // [FP64][periodic][cubes]
 };
 
 static const ModesClass kClasses[] = {
-#define SP_MODES_ROW(NT, MINB, QS) \
-  {NT, MINB, QS, \
-   {{k_modes<NT, MINB, false, QS, false>, k_modes<NT, MINB, true, QS, false>}, \
-    {k_modes<NT, MINB, false, QS, true>, k_modes<NT, MINB, true, QS, true>}}},
-    SP_MODES_CLASSES(SP_MODES_ROW)
+#define SP_MODES_FNS(V, NT, MINB, QS) \
+  {{k_modes<V, NT, MINB, false, QS, false>, k_modes<V, NT, MINB, true, QS, false>}, \
+   {k_modes<V, NT, MINB, false, QS, true>, k_modes<V, NT, MINB, true, QS, true>}}
+#define SP_MODES_ROW(V, NT, MINB, QS) \
+  {NT, MINB, QS, {SP_MODES_FNS(V, NT, MINB, QS), SP_MODES_FNS(double, NT, MINB, QS)}},
+    SP_MODES_CLASSES(SP_MODES_ROW, F2)
 #undef SP_MODES_ROW
+#undef SP_MODES_FNS
 };
 constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
 
@@ -38,11 +41,11 @@ static int class_room(const ModesClass &k) {
 // element layers, 30 under periodic conditions (a column's materials are one
 // 32-bit mask, which repeats two layers then).  Larger RVEs
 // keep the solve_rve kernel.
-int modes_class(const MeshGeo &g, const double *len, bool per) {
+int modes_class(const MeshGeo &g, const double *len, bool per, bool f64) {
   if (g.nex < 2 || g.ney < 2 || g.nez < 2) return -1;
   if (g.nez > (per ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ)) return -1;
   if ((long long)g.nex * g.ney > 640) return -1;
-  const ModesGeo G(g.nex, g.ney, g.nez, per);
+  const ModesGeo G(g.nex, g.ney, g.nez, per, f64);
   const double hx = len[0] / g.nex, hy = len[1] / g.ney, hz = len[2] / g.nez;
   const int cube = hx == hy && hx == hz;
   for (int c = 0; c < kNumClasses; c++) {
@@ -53,7 +56,7 @@ int modes_class(const MeshGeo &g, const double *len, bool per) {
 }
 
 int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
-               const std::vector<MeshGeo> &geo, int nrhs, bool per, const Device *d,
+               const std::vector<MeshGeo> &geo, int nrhs, bool per, bool f64, const Device *d,
                ModesPlan *out) {
   // classes with the largest RVEs first
   for (int c = 2 * kNumClasses - 1; c >= 0; c--) {
@@ -64,11 +67,11 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     const ModesClass &k = kClasses[c / 2];
     out->buckets.push_back(ModesBucket());
     ModesBucket &b = out->buckets.back();
-    b.fn = k.fn[per][c & 1];
+    b.fn = k.fn[f64][per][c & 1];
     b.nrve = (int)ord.size();
     int ntot = 0, wlen = 0;
     for (int i : ord) {
-      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez, per);
+      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez, per, f64);
       b.threads = std::max(b.threads, G.warps() * 32);
       b.smem = std::max(b.smem, G.smem(k.qs));
       ntot = std::max(ntot, G.ntot);
@@ -94,7 +97,7 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     b.grid = (int)std::min<long long>((long long)d->nsm * nb, (long long)b.nrve * nrhs);
     SP_TRY(dmalloc((void **)&b.d_order, ord.size() * sizeof(int), &b.bytes));
     SP_TRY(dmalloc((void **)&b.ws_w, b.grid * b.w_stride * sizeof(double), &b.bytes));
-    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (k.qs ? 2 : 3) * b.v_stride * sizeof(float2), &b.bytes));
+    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (k.qs ? 2 : 3) * b.v_stride * sizeof(double), &b.bytes));
     if (cudaMemcpy(b.d_order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice))
       return sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
   }

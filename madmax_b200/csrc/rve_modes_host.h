@@ -14,7 +14,7 @@ struct ModesBucket {
   int threads = 0, grid = 0, smem = 0, nrve = 0;
   int *d_order = nullptr;
   double *ws_w = nullptr;
-  float2 *ws_v = nullptr;
+  void *ws_v = nullptr;
   size_t w_stride = 0, v_stride = 0, bytes = 0;
 };
 
@@ -44,10 +44,10 @@ struct ModesCommon {
 };
 
 // The kernel class of an RVE (-1: none, the solve_rve kernel takes it)
-int modes_class(const MeshGeo &g, const double *len, bool periodic);
+int modes_class(const MeshGeo &g, const double *len, bool periodic, bool f64);
 // Launches for the RVEs `ids` (largest first), every one of a class >= 0
 int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
-               const std::vector<MeshGeo> &geo, int nrhs, bool periodic, const Device *d,
+               const std::vector<MeshGeo> &geo, int nrhs, bool periodic, bool f64, const Device *d,
                ModesPlan *out);
 void modes_free(ModesPlan *m);
 // counters: one per bucket, on the device

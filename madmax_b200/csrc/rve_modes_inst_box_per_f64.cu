@@ -1,0 +1,9 @@
+// rve_modes_inst_box_per_f64.cu -- instantiations of the element-mode batch kernel
+// (rve_modes_kernel.cuh) for box elements, periodic conditions, FP64.
+#include "rve_modes_kernel.cuh"
+
+namespace sp {
+#define SP_MODES_DEFINE(V, NT, MINB, QS) \
+  template __global__ void k_modes<V, NT, MINB, false, QS, true>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE, double)
+}  // namespace sp

@@ -3,7 +3,7 @@
 #include "rve_modes_kernel.cuh"
 
 namespace sp {
-#define SP_MODES_DEFINE(NT, MINB, QS) \
-  template __global__ void k_modes<NT, MINB, true, QS, true>(ModesParams);
-SP_MODES_CLASSES(SP_MODES_DEFINE)
+#define SP_MODES_DEFINE(V, NT, MINB, QS) \
+  template __global__ void k_modes<V, NT, MINB, true, QS, true>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE, F2)
 }  // namespace sp

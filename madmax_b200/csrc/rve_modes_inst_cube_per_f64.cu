@@ -1,0 +1,9 @@
+// rve_modes_inst_cube_per_f64.cu -- instantiations of the element-mode batch kernel
+// (rve_modes_kernel.cuh) for cubic elements, periodic conditions, FP64.
+#include "rve_modes_kernel.cuh"
+
+namespace sp {
+#define SP_MODES_DEFINE(V, NT, MINB, QS) \
+  template __global__ void k_modes<V, NT, MINB, true, QS, true>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE, double)
+}  // namespace sp

@@ -32,7 +32,7 @@ struct ModesParams {
   unsigned *done;            // [nrve] finished load cases (0 between launches)
   int *counter;
   double *ws_w;    // per CTA [3][wlen]
-  float2 *ws_v;    // per CTA r, x and (q not in shared memory) q: [3][ntot] pairs each
+  void *ws_v;      // per CTA r, x and (q not in shared memory) q: [3][ntot] 8-byte values each
   size_t w_stride, v_stride;  // v_stride: of one of them
   double rtol, inner_rtol;
   int max_outer, max_inner;
@@ -46,7 +46,8 @@ constexpr int SP_MODES_MAX_WARPS = 20;
 struct ModesShared {
   double cd[2][MC_N];    // mode coefficients of the two materials
   float2 c32[4][MC_N];   // FP32 pairs: materials of the (lower, upper) layer
-  float4 dl[9];          // Jacobi diagonal by the number of fibre elements around a node
+  double dl64[9][4];     // Jacobi diagonal by the number of fibre elements around a node
+  float4 dl[9];          // ... in FP32
   double kd2[9];         // sum over components of the squared diagonal
   double A[9];           // first-order modes of eps.x: [component][axis]
   double E[9];           // eps as a 3x3 matrix
@@ -66,11 +67,13 @@ static_assert(sizeof(ModesShared) % 16 == 0, "vectors follow on a 16-byte bounda
 // conditions: every node of the periodic grid, neighbours wrapped; a row's
 // columns are preceded by a repetition of its last one, the left neighbour of
 // its first.
+// FP32 vectors have a slot for each pair of planes, FP64 ones for each plane;
+// a value is 8 bytes either way.
 struct ModesGeo {
   int nex, ney, nez, nface, mz, h, ntot, per;
-  __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic)
-      : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(periodic ? ez : ez - 1), h((mz + 1) / 2),
-        ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic) {}
+  __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic, bool f64)
+      : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(periodic ? ez : ez - 1),
+        h(f64 ? mz : (mz + 1) / 2), ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic) {}
   __host__ __device__ int wlen() const { return mz * nface + (per ? 0 : nex + 2); }
   // lanes of a row, of all rows, and of a warp: 32 where rows start at lane 0
   // (whose left neighbour is the boundary, or its own repetition), else 31
@@ -98,14 +101,42 @@ struct ModesGeo {
 
 extern __shared__ __align__(16) unsigned char s_modes[];
 __device__ __forceinline__ ModesShared &msh() { return *reinterpret_cast<ModesShared *>(s_modes); }
-__device__ __forceinline__ F2 *mp() { return reinterpret_cast<F2 *>(s_modes + sizeof(ModesShared)); }
+template <typename V>
+__device__ __forceinline__ V *mp() {
+  return reinterpret_cast<V *>(s_modes + sizeof(ModesShared));
+}
 // q, or the exchange planes
-__device__ __forceinline__ F2 *mq() {
-  return reinterpret_cast<F2 *>(reinterpret_cast<char *>(mp()) + msh().qoff);
+template <typename V>
+__device__ __forceinline__ V *mq() {
+  return reinterpret_cast<V *>(mp<char>() + msh().qoff);
 }
-__device__ __forceinline__ uint8_t *mcnt() {
-  return reinterpret_cast<uint8_t *>(mp()) + msh().cntoff;
-}
+__device__ __forceinline__ uint8_t *mcnt() { return mp<uint8_t>() + msh().cntoff; }
+
+// FP32 pairs or FP64 values: their memory type and the type of their scalars
+template <typename V>
+struct ModesType;
+template <>
+struct ModesType<F2> {
+  static constexpr bool F64 = false;
+  using Mem = float2;
+  using S = float;
+  __device__ static F2 ld(const float2 *a) { return F2{__ldcg(a)}; }
+  __device__ static void st(float2 *a, F2 v) { __stcg(a, v.v); }
+  __device__ static void add(float2 *a, F2 v) { atomicAdd(a, v.v); }
+  __device__ static F2 splat(float s) { return mk2(s, s); }
+  __device__ static double sum(F2 v) { return (double)(v.v.x + v.v.y); }
+};
+template <>
+struct ModesType<double> {
+  static constexpr bool F64 = true;
+  using Mem = double;
+  using S = double;
+  __device__ static double ld(const double *a) { return __ldcg(a); }
+  __device__ static void st(double *a, double v) { __stcg(a, v); }
+  __device__ static void add(double *a, double v) { atomicAdd(a, v); }
+  __device__ static double splat(double s) { return s; }
+  __device__ static double sum(double v) { return v; }
+};
 
 // Sum NV doubles over the CTA in a fixed order; every thread gets the
 // totals.  One barrier: red holds two buffers, used in turn.
@@ -178,18 +209,22 @@ __device__ __forceinline__ void plane_sync(int threads) {
 
 // q = A p: p, q in shared memory ([slot][3] pairs), q in qg ([3][ntot]) when
 // QS is false; returns the thread's share of p.q.
-template <bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double march_apply(float2 *qg) {
+template <typename V, bool CUBE, bool QS, bool PER>
+__device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
+  using MT = ModesType<V>;
+  constexpr bool F64 = MT::F64;
+  // registers to spare for the next slot's values (FP64 has none)
+  constexpr bool AHEAD = QS && !F64;
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
   const unsigned mats = sh.col[T.f];
   const int nface = sh.nface, nf3 = 3 * nface, h = sh.h, ntot = sh.ntot;
   const int right = PER ? 3 * T.dx : 3, up = 3 * T.dy;
-  const F2 *pf = mp() + 3 * T.f;  // corner (0, 0) of slot 0
-  F2 *const qf = mq() + 3 * T.f;
-  const bool odd = (sh.mz & 1) != 0;
-  F2 raw[3][4], Fa[3][4], Fb[3][4], acc[3][4];
-  auto load = [&](const F2 *a) {
+  const V *pf = mp<V>() + 3 * T.f;  // corner (0, 0) of slot 0
+  V *const qf = mq<V>() + 3 * T.f;
+  const bool odd = !F64 && (sh.mz & 1) != 0;
+  V raw[3][4], Fa[3][4], Fb[3][4], acc[3][4];
+  auto load = [&](const V *a) {
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       raw[c][0] = a[c];
@@ -203,92 +238,125 @@ __device__ __noinline__ double march_apply(float2 *qg) {
   // (for an odd number of planes, already at slot h - 1)
   auto next = [&](int s) {
     load(s < h ? pf + s * nf3 : pf);
-    if (s >= h) {
+    if (s >= h && !(F64 && PER)) {
       __syncwarp();  // a branch: predicated, the moves would be issued every step
 #pragma unroll
       for (int c = 0; c < 3; c++)
 #pragma unroll
-        for (int m = 0; m < 4; m++) raw[c][m] = mk2(raw[c][m].v.y, PER ? raw[c][m].v.x : 0.f);
+        for (int m = 0; m < 4; m++) {
+          if constexpr (F64)
+            raw[c][m] = 0.0;
+          else
+            raw[c][m] = mk2(raw[c][m].v.y, PER ? raw[c][m].v.x : 0.f);
+        }
     }
-    if (PER && odd && s == h - 1) {
-      __syncwarp();
+    if constexpr (PER && !F64) {
+      if (odd && s == h - 1) {
+        __syncwarp();
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        raw[c][0].v.y = pf[c].v.x;
-        raw[c][1].v.y = pf[right + c].v.x;
-        raw[c][2].v.y = pf[up + c].v.x;
-        raw[c][3].v.y = pf[up + right + c].v.x;
+        for (int c = 0; c < 3; c++) {
+          raw[c][0].v.y = pf[c].v.x;
+          raw[c][1].v.y = pf[right + c].v.x;
+          raw[c][2].v.y = pf[up + c].v.x;
+          raw[c][3].v.y = pf[up + right + c].v.x;
+        }
       }
     }
   };
   if (T.warp_on) {
     // below slot 0: the boundary plane, or the last one (lower half); plane
     // h - 1 (upper half)
-    if (PER) {
-      load(pf + (odd ? h - 2 : h - 1) * nf3);
+    if constexpr (F64) {
+      if (PER) load(pf + (h - 1) * nf3);
 #pragma unroll
       for (int c = 0; c < 3; c++)
 #pragma unroll
-        for (int m = 0; m < 4; m++) acc[c][m].v.x = raw[c][m].v.y;
-    }
-    load(pf + (h - 1) * nf3);
+        for (int m = 0; m < 4; m++) {
+          if (!PER) raw[c][m] = 0.0;
+          acc[c][m] = 0.0;
+        }
+    } else {
+      if (PER) {
+        load(pf + (odd ? h - 2 : h - 1) * nf3);
 #pragma unroll
-    for (int c = 0; c < 3; c++)
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-      for (int m = 0; m < 4; m++) {
-        raw[c][m] = mk2(PER ? acc[c][m].v.x : 0.f, raw[c][m].v.x);
-        acc[c][m] = mk2(0.f, 0.f);
+          for (int m = 0; m < 4; m++) acc[c][m].v.x = raw[c][m].v.y;
       }
+      load(pf + (h - 1) * nf3);
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          raw[c][m] = mk2(PER ? acc[c][m].v.x : 0.f, raw[c][m].v.x);
+          acc[c][m] = mk2(0.f, 0.f);
+        }
+    }
     face_modes(raw, Fa);
-    if (QS) next(0);
+    if (AHEAD) next(0);
   }
   if (!T.warp_on) return 0.0;
   double pq = 0.0;
   // one step: F0 the modes of the face below, F1 takes those above (two steps
   // a trip, so that the faces change places without copies)
-  auto step = [&](int s, F2 (&F0)[3][4], F2 (&F1)[3][4]) {
-    F2 low[3];
+  auto step = [&](int s, V (&F0)[3][4], V (&F1)[3][4]) {
+    V low[3];
     if (T.warp_on) {
-      F2 S[3][3], D[3][4], high[3];
-      if (!QS) next(s);
+      V S[3][3], D[3][4], high[3];
+      if (!AHEAD) next(s);
       face_modes(raw, F1);
       layer_modes(F0, F1, S, D);
-      const unsigned ma = (mats >> s) & 1u, mb = (mats >> (s + h)) & 1u;
-      if constexpr (CUBE) {
-        const float2 *ct = sh.c6[ma + 2 * mb];
-        modes_cube(S, D, [ct](int i) { return F2{ct[i]}; });
+      const unsigned ma = (mats >> s) & 1u;
+      if constexpr (F64) {
+        if constexpr (CUBE) {
+          const double *ct = sh.cc[ma];
+          modes_cube(S, D, [ct](int i) { return ct[i]; });
+        } else {
+          const double *ct = sh.cd[ma];
+          modes_box(S, D, [ct](int i) { return ct[i]; });
+        }
       } else {
-        const float2 *ct = sh.c32[ma + 2 * mb];
-        modes_box(S, D, [ct](int i) { return F2{ct[i]}; });
+        const unsigned mb = (mats >> (s + h)) & 1u;
+        if constexpr (CUBE) {
+          const float2 *ct = sh.c6[ma + 2 * mb];
+          modes_cube(S, D, [ct](int i) { return F2{ct[i]}; });
+        } else {
+          const float2 *ct = sh.c32[ma + 2 * mb];
+          modes_box(S, D, [ct](int i) { return F2{ct[i]}; });
+        }
       }
       layer_back(S, D, acc, low, high);
       // the upper row's share waits where that row's q goes (QS), or in the
       // exchange planes in turn
-      F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3 + up;
+      V *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3 + up;
       if (T.column && s > 0 && (PER || T.f + sh.nex < nface))
 #pragma unroll
         for (int c = 0; c < 3; c++) e[c] = high[c];
-      // with registers to spare, the next slot's values before the barrier
-      if (QS) next(s + 1);
+      // the next slot's values before the barrier
+      if (AHEAD) next(s + 1);
     }
     if (s > 0) {
       plane_sync(sh.threads);
       if (T.owner) {
-        F2 *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3;
-        const F2 *ps = pf + (s - 1) * nf3;
-        F2 t = mk2(0.f, 0.f);
+        V *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3;
+        const V *ps = pf + (s - 1) * nf3;
+        V t = zero_of(V());
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           low[c] = low[c] + e[c];
-          if (odd && s == h) low[c].v.y = 0.f;  // no plane there
-          if (PER && s == 1 && T.f == 0) low[c].v.x = 0.f;  // the fixed node
+          if constexpr (F64) {
+            if (PER && s == 1 && T.f == 0) low[c] = 0.0;  // the fixed node
+          } else {
+            if (odd && s == h) low[c].v.y = 0.f;  // no plane there
+            if (PER && s == 1 && T.f == 0) low[c].v.x = 0.f;  // the fixed node
+          }
           if constexpr (QS)
             e[c] = low[c];
           else
-            __stcg(qg + (size_t)c * ntot + (s - 1) * nface + T.f, low[c].v);
+            MT::st(qg + (size_t)c * ntot + (s - 1) * nface + T.f, low[c]);
           t = mad(low[c], ps[c], t);
         }
-        pq += (double)(t.v.x + t.v.y);
+        pq += MT::sum(t);
       }
     }
   };
@@ -303,23 +371,24 @@ __device__ __noinline__ double march_apply(float2 *qg) {
   return pq;
 }
 
-// b = -K (eps.x + w) on the interior nodes in FP64: rounded to FP32 into rg;
+// b = -K (eps.x + w) on the interior nodes in FP64: rounded to V into rv;
 // returns the thread's shares of |b|^2 and r.z.  The running plane's forces
 // (and, at 96 registers a thread, the face's modes) wait in shared memory
 // between layers: in registers they spill, and a spill goes to L2, since the
 // vectors leave L1 next to nothing (n = 20: 285k cycles an evaluation with
 // spills, 80k without).
-template <bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double2 march_residual(const double *w, float *rg) {
+template <typename V, bool CUBE, bool QS, bool PER>
+__device__ __noinline__ double2 march_residual(const double *w, typename ModesType<V>::Mem *rv) {
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
   const unsigned mats = sh.col[T.f];
   const int nface = sh.nface, right = PER ? T.dx : 1, up = T.dy, wl = sh.wlen, mz = sh.mz, h = sh.h;
-  double *const ex = reinterpret_cast<double *>(mq());  // two exchange planes
+  constexpr bool F64 = ModesType<V>::F64;
+  double *const ex = mq<double>();  // two exchange planes
   const uint8_t *const cnt = mcnt();
   // [c][m] of the running forces at 4 c + m, of the face's modes 12 further;
   // an odd number of doubles a thread (no bank conflicts)
-  double *const state = (QS ? ex + 6 * nface : reinterpret_cast<double *>(mp())) +
+  double *const state = (QS ? ex + 6 * nface : mp<double>()) +
                         (T.warp_on ? threadIdx.x : 0) * (QS ? 13 : 25);
   double n2 = 0.0, rz = 0.0;
   double F0[3][4] = {};  // (QS)
@@ -415,20 +484,22 @@ __device__ __noinline__ double2 march_residual(const double *w, float *rg) {
       plane_sync(sh.threads);
       if (T.owner) {
         const double *e = exs + 3 * T.f;
-        const bool hi = s - 1 >= h;
+        const bool hi = !F64 && s - 1 >= h;
         const int i = (hi ? s - 1 - h : s - 1) * nface + T.f;
-        const unsigned cv = cnt[i];
-        const float4 dl = sh.dl[hi ? cv >> 4 : cv & 15u];
-        const float dz[3] = {dl.x, dl.y, dl.z};
-        float *ro = rg + 2 * i + (hi ? 1 : 0);
+        const unsigned cv = hi ? cnt[i] >> 4 : cnt[i] & 15u;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           double b = -(low[c] + e[c]);
           if (PER && s == 1 && T.f == 0) b = 0.0;  // the fixed node
-          const float bf = (float)b;
-          ro[2 * c * sh.ntot] = bf;
           n2 += b * b;
-          rz += (double)bf * (double)(dz[c] * bf);
+          if constexpr (F64) {
+            rv[c * sh.ntot + i] = b;
+            rz += b * (sh.dl64[cv][c] * b);
+          } else {
+            const float bf = (float)b;
+            reinterpret_cast<float *>(rv + c * sh.ntot + i)[hi] = bf;
+            rz += (double)bf * (double)(reinterpret_cast<const float *>(&sh.dl[cv])[c] * bf);
+          }
         }
       }
     }
@@ -481,12 +552,12 @@ __device__ __noinline__ int march_average(const double *w, int ph) {
   return ph;
 }
 
-// Jacobi diagonal of a slot's two nodes
+// Jacobi diagonal of a slot's nodes (in a cube the components' are equal)
 template <bool CUBE>
-__device__ __forceinline__ void dinv_pairs(int i, F2 (&dz)[3]) {
+__device__ __forceinline__ void slot_dinv(int i, F2 (&dz)[3]) {
   const ModesShared &sh = msh();
   const unsigned cv = mcnt()[i];
-  if (CUBE) {  // the three components' diagonals are equal
+  if (CUBE) {
     dz[0] = dz[1] = dz[2] = mk2(sh.dl[cv & 15u].x, sh.dl[cv >> 4].x);
     return;
   }
@@ -495,47 +566,56 @@ __device__ __forceinline__ void dinv_pairs(int i, F2 (&dz)[3]) {
   dz[1] = mk2(da.y, db.y);
   dz[2] = mk2(da.z, db.z);
 }
+template <bool CUBE>
+__device__ __forceinline__ void slot_dinv(int i, double (&dz)[3]) {
+  const double *d = msh().dl64[mcnt()[i] & 15u];
+#pragma unroll
+  for (int c = 0; c < 3; c++) dz[c] = d[CUBE ? 0 : c];
+}
 
 // One group of up to U slots of update_xr: all loads before the stores, one L2
 // round trip for the group.
-template <bool CUBE, bool QS, int U>
-__device__ __forceinline__ void xr_slots(int s0, int f, float2 *rg, float2 *xg, const float2 *qg,
-                                         F2 al, F2 nal, bool first, double &vz, double &vr) {
+template <typename V, bool CUBE, bool QS, int U>
+__device__ __forceinline__ void xr_slots(int s0, int f, typename ModesType<V>::Mem *rg,
+                                         typename ModesType<V>::Mem *xg,
+                                         const typename ModesType<V>::Mem *qg, V al, V nal,
+                                         bool first, double &vz, double &vr) {
+  using MT = ModesType<V>;
   const ModesShared &sh = msh();
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
-  F2 *const p = mp();
-  F2 r[U][3], q[U][3];
+  V *const p = mp<V>();
+  V r[U][3], q[U][3];
 #pragma unroll
   for (int j = 0; j < U; j++)
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const int o = c * ntot + min(s0 + j, h - 1) * nface + f;
-      r[j][c].v = __ldcg(rg + o);
-      if (!QS) q[j][c].v = __ldcg(qg + o);
+      r[j][c] = MT::ld(rg + o);
+      if (!QS) q[j][c] = MT::ld(qg + o);
     }
 #pragma unroll
   for (int j = 0; j < U; j++) {
     if (s0 + j >= h) break;
     const int i = (s0 + j) * nface + f;
-    F2 dz[3];
-    dinv_pairs<CUBE>(i, dz);
-    F2 sz = mk2(0.f, 0.f), sr = mk2(0.f, 0.f);
+    V dz[3];
+    slot_dinv<CUBE>(i, dz);
+    V sz = zero_of(V()), sr = zero_of(V());
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const int o = c * ntot + i;
-      const F2 rn = mad(nal, QS ? p[3 * (ntot + i) + c] : q[j][c], r[j][c]);
-      const F2 dx = al * p[3 * i + c];
-      __stcg(rg + o, rn.v);
+      const V rn = mad(nal, QS ? p[3 * (ntot + i) + c] : q[j][c], r[j][c]);
+      const V dx = al * p[3 * i + c];
+      MT::st(rg + o, rn);
       if (first)
-        __stcg(xg + o, dx.v);
+        MT::st(xg + o, dx);
       else
-        atomicAdd(xg + o, dx.v);  // (no value back: nothing waits for it)
+        MT::add(xg + o, dx);  // (no value back: nothing waits for it)
       if constexpr (QS) p[3 * (ntot + i) + c] = rn;
       sz = mad(rn, dz[c] * rn, sz);
       sr = mad(rn, rn, sr);
     }
-    vz += (double)(sz.v.x + sz.v.y);
-    vr += (double)(sr.v.x + sr.v.y);
+    vz += MT::sum(sz);
+    vr += MT::sum(sr);
   }
 }
 
@@ -543,28 +623,33 @@ __device__ __forceinline__ void xr_slots(int s0, int f, float2 *rg, float2 *xg, 
 // correction's first step); returns its shares of r.z and r.r.  x is added to
 // in L2: only this thread touches its entries.  q's slots take the new r for
 // the direction update.
-template <bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double2 update_xr(float2 *rg, float2 *xg, const float2 *qg, float alpha,
+template <typename V, bool CUBE, bool QS, bool PER>
+__device__ __noinline__ double2 update_xr(typename ModesType<V>::Mem *rg,
+                                          typename ModesType<V>::Mem *xg,
+                                          const typename ModesType<V>::Mem *qg, double alpha,
                                           bool first) {
   const ModesLane<PER> T;
   if (!T.owner) return make_double2(0.0, 0.0);
   const int h = msh().h;
-  const F2 al = mk2(alpha, alpha), nal = mk2(-alpha, -alpha);
+  const typename ModesType<V>::S a = (typename ModesType<V>::S)alpha;
+  const V al = ModesType<V>::splat(a), nal = ModesType<V>::splat(-a);
   double vz = 0.0, vr = 0.0;
   constexpr int U = QS ? 5 : 3;
 #pragma unroll 1
-  for (int s = 0; s < h; s += U) xr_slots<CUBE, QS, U>(s, T.f, rg, xg, qg, al, nal, first, vz, vr);
+  for (int s = 0; s < h; s += U)
+    xr_slots<V, CUBE, QS, U>(s, T.f, rg, xg, qg, al, nal, first, vz, vr);
   return make_double2(vz, vr);
 }
 
 // p = D^-1 r + beta p over the thread's column; r in q's slots (LOCAL) or in
 // rg.  beta = 0 starts afresh without reading p.
-template <bool CUBE, bool LOCAL, int U>
-__device__ __forceinline__ void p_slots(int s0, int f, const float2 *rg, F2 be, bool fresh) {
+template <typename V, bool CUBE, bool LOCAL, int U>
+__device__ __forceinline__ void p_slots(int s0, int f, const typename ModesType<V>::Mem *rg, V be,
+                                        bool fresh) {
   const ModesShared &sh = msh();
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
-  F2 *const p = mp();
-  F2 r[U][3], pv[U][3];
+  V *const p = mp<V>();
+  V r[U][3], pv[U][3];
 #pragma unroll
   for (int j = 0; j < U; j++)
 #pragma unroll
@@ -573,37 +658,38 @@ __device__ __forceinline__ void p_slots(int s0, int f, const float2 *rg, F2 be, 
       if constexpr (LOCAL)
         r[j][c] = p[3 * (ntot + i) + c];
       else
-        r[j][c].v = __ldcg(rg + (c * ntot + i));
+        r[j][c] = ModesType<V>::ld(rg + (c * ntot + i));
       pv[j][c] = p[3 * i + c];
     }
 #pragma unroll
   for (int j = 0; j < U; j++) {
     if (s0 + j >= h) break;
     const int i = (s0 + j) * nface + f;
-    F2 dz[3];
-    dinv_pairs<CUBE>(i, dz);
+    V dz[3];
+    slot_dinv<CUBE>(i, dz);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      const F2 z = dz[c] * r[j][c];
+      const V z = dz[c] * r[j][c];
       p[3 * i + c] = fresh ? z : mad(be, pv[j][c], z);
     }
   }
 }
 
-template <bool CUBE, bool LOCAL, bool PER>
-__device__ __noinline__ void update_p(const float2 *rg, float beta) {
+template <typename V, bool CUBE, bool LOCAL, bool PER>
+__device__ __noinline__ void update_p(const typename ModesType<V>::Mem *rg, double beta) {
   const ModesLane<PER> T;
   if (!T.owner) return;
   const int h = msh().h;
-  const F2 be = mk2(beta, beta);
+  const typename ModesType<V>::S b = (typename ModesType<V>::S)beta;
+  const V be = ModesType<V>::splat(b);
   constexpr int U = LOCAL ? 3 : 5;
 #pragma unroll 1
-  for (int s = 0; s < h; s += U) p_slots<CUBE, LOCAL, U>(s, T.f, rg, be, beta == 0.f);
+  for (int s = 0; s < h; s += U) p_slots<V, CUBE, LOCAL, U>(s, T.f, rg, be, b == 0);
 }
 
 // w += x in FP64 over the thread's column
-template <bool PER>
-__device__ __noinline__ void update_w(const float2 *xg, double *w) {
+template <typename V, bool PER>
+__device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, double *w) {
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
   if (!T.owner) return;
@@ -611,18 +697,22 @@ __device__ __noinline__ void update_w(const float2 *xg, double *w) {
 #pragma unroll 1
   for (int s = 0; s < h; s++) {
     const int i = s * nface + T.f;
-    float2 x[3];
+    V x[3];
     double w0[3], w1[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      x[c] = __ldcg(xg + (c * ntot + i));
+      x[c] = ModesType<V>::ld(xg + (c * ntot + i));
       w0[c] = w[c * wl + i];
       w1[c] = s + h < mz ? w[c * wl + i + h * nface] : 0.0;
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      w[c * wl + i] = w0[c] + (double)x[c].x;
-      if (s + h < mz) w[c * wl + i + h * nface] = w1[c] + (double)x[c].y;
+      if constexpr (ModesType<V>::F64) {
+        w[c * wl + i] = w0[c] + x[c];
+      } else {
+        w[c * wl + i] = w0[c] + (double)x[c].v.x;
+        if (s + h < mz) w[c * wl + i + h * nface] = w1[c] + (double)x[c].v.y;
+      }
     }
   }
 }
@@ -630,8 +720,8 @@ __device__ __noinline__ void update_w(const float2 *xg, double *w) {
 // The residual's face state takes p's place when q is not in shared memory:
 // every column's p waits in q's global work space meanwhile, the padding is
 // zeroed anew.
-template <bool PER>
-__device__ __noinline__ void save_p(float2 *qg) {
+template <typename V, bool PER>
+__device__ __noinline__ void save_p(typename ModesType<V>::Mem *qg) {
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
   if (T.owner)
@@ -639,30 +729,30 @@ __device__ __noinline__ void save_p(float2 *qg) {
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const int i = s * sh.nface + T.f;
-        __stcg(qg + (c * sh.ntot + i), mp()[3 * i + c].v);
+        ModesType<V>::st(qg + (c * sh.ntot + i), mp<V>()[3 * i + c]);
       }
   __syncthreads();
 }
-template <bool PER>
-__device__ __noinline__ void restore_p(const float2 *qg, bool saved) {
+template <typename V, bool PER>
+__device__ __noinline__ void restore_p(const typename ModesType<V>::Mem *qg, bool saved) {
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
-  for (int i = threadIdx.x; i < 3 * sh.ntot; i += blockDim.x) mp()[i] = mk2(0.f, 0.f);
+  for (int i = threadIdx.x; i < 3 * sh.ntot; i += blockDim.x) mp<V>()[i] = zero_of(V());
   __syncthreads();
   if (T.owner && saved)
     for (int s = 0; s < sh.h; s++)
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const int i = s * sh.nface + T.f;
-        mp()[3 * i + c].v = __ldcg(qg + (c * sh.ntot + i));
+        mp<V>()[3 * i + c] = ModesType<V>::ld(qg + (c * sh.ntot + i));
       }
 }
 
 // the tables, materials and start vectors of one load case
-template <bool QS, bool PER>
+template <bool F64, bool PER>
 __device__ __noinline__ void modes_setup(const double *len, const double *mat,
                                          const uint8_t *etype, const double *eps, double *w,
-                                         float2 *rg) {
+                                         void *rv) {
   ModesShared &sh = msh();
   const int t = threadIdx.x;
   const ModesLane<PER> T;
@@ -693,9 +783,9 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
   if (PER) mats = mats << 1 | mats >> (sh.nez - 1) | (mats & 1u) << (sh.nez + 1);
   if (T.column) sh.col[T.f] = mats;
   {
-    float4 *p = reinterpret_cast<float4 *>(mp());  // (3 ntot pairs, rounded down to 16 bytes)
+    float4 *p = mp<float4>();  // (3 ntot pairs, rounded down to 16 bytes)
     for (int i = t; i < 3 * sh.ntot / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t == 0) mp()[3 * sh.ntot - 1] = mk2(0.f, 0.f);
+    if (t == 0) mp<float2>()[3 * sh.ntot - 1] = make_float2(0.f, 0.f);
   }
   // w's padding: the columns without an interior node and the row past the end
   if (T.column && (PER || !T.owner))
@@ -721,7 +811,7 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
              __popc((m3 >> pl) & 3u);
     };
     for (int s = 0; s < sh.h; s++)
-      mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (count(s + sh.h) << 4));
+      mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (F64 ? 0 : count(s + sh.h) << 4));
     const double X = (T.f % nex) * sh.hx[0], Y = (T.f / nex) * sh.hx[1];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
@@ -729,7 +819,7 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
       if (!PER)
         for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
       // a slot without an upper plane keeps a zero there
-      rg[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
+      static_cast<float2 *>(rv)[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
     }
   }
   __syncthreads();
@@ -760,6 +850,8 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
       d[c] = (8 - t) * mode_diag(sh.cd[0], c) + t * mode_diag(sh.cd[1], c);
       s2 += d[c] * d[c];
     }
+#pragma unroll
+    for (int c = 0; c < 3; c++) sh.dl64[t][c] = 1.0 / d[c];
     sh.dl[t] = make_float4((float)(1.0 / d[0]), (float)(1.0 / d[1]), (float)(1.0 / d[2]), 0.f);
     sh.kd2[t] = s2;
   }
@@ -794,15 +886,15 @@ __device__ __noinline__ inline void modes_output(const double *m, double *stress
 // The CTA's work spaces.  Formed anew at every use (hidden from the
 // compiler's view of the loop), so that no pointer holds registers across the
 // marches.
-template <bool QS>
+template <typename V, bool QS>
 struct ModesSpace {
   double *w;
-  float2 *r, *x, *q;
+  typename ModesType<V>::Mem *r, *x, *q;
   __device__ __forceinline__ explicit ModesSpace(const ModesParams &P) {
     unsigned b = blockIdx.x;
     asm volatile("" : "+r"(b));
     w = P.ws_w + (size_t)b * P.w_stride;
-    r = P.ws_v + (size_t)b * (QS ? 2 : 3) * P.v_stride;
+    r = static_cast<typename ModesType<V>::Mem *>(P.ws_v) + (size_t)b * (QS ? 2 : 3) * P.v_stride;
     x = r + P.v_stride;
     q = QS ? nullptr : x + P.v_stride;
   }
@@ -813,7 +905,7 @@ struct ModesSpace {
 // zero fluctuation, w = 0); one at the round-off level of its own
 // cancelling terms is zero, and its load case is solved with that.  Else
 // w = 0: the affine field starts.
-template <bool PER>
+template <bool F64, bool PER>
 __device__ __noinline__ double rhs_norm(double n2, double *w, int ph) {
   const ModesShared &sh = msh();
   const ModesLane<PER> T;
@@ -822,7 +914,7 @@ __device__ __noinline__ double rhs_norm(double n2, double *w, int ph) {
     for (int s = 0; s < sh.h; s++) {
       const unsigned cv = mcnt()[s * sh.nface + T.f];
       v[1] += sh.kd2[cv & 15u];
-      if (s + sh.h < sh.mz) v[1] += sh.kd2[cv >> 4];
+      if (!F64 && s + sh.h < sh.mz) v[1] += sh.kd2[cv >> 4];
     }
   cta_sum<2>(v, ph);
   double um = 0.0;
@@ -861,10 +953,11 @@ __device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_sol
   }
 }
 
-// NT threads at most, MINB CTAs per SM; CUBE: equal element edges; QS: q in
+// V: FP32 pairs or FP64; NT threads at most, MINB CTAs per SM; CUBE: equal element edges; QS: q in
 // shared memory; PER: periodic conditions
-template <int NT, int MINB, bool CUBE, bool QS, bool PER>
+template <typename V, int NT, int MINB, bool CUBE, bool QS, bool PER>
 __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
+  constexpr bool F64 = ModesType<V>::F64;
   ModesShared &sh = msh();
   if (dynamic_smem_bytes() < sizeof(ModesShared)) return;
   int ph = 0;  // the reduction buffer in turn
@@ -876,7 +969,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.rid = P.order[task / P.nrhs];
         sh.k = task % P.nrhs;
         const MeshGeo &mg = P.plans[P.rves[sh.rid].plan].geo;
-        const ModesGeo G(mg.nex, mg.ney, mg.nez, PER);
+        const ModesGeo G(mg.nex, mg.ney, mg.nez, PER, F64);
         if (dynamic_smem_bytes() < (unsigned)G.smem(QS) || G.warps() * 32 > blockDim.x ||
             G.warps() > SP_MODES_MAX_WARPS || G.nez > (PER ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ) ||
             G.nface > SP_MODES_MAX_WARPS * 32)
@@ -902,17 +995,16 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
     if (sh.job == 1) {
       // 1. tables
       {
-        const ModesSpace<QS> ws(P);
+        const ModesSpace<V, QS> ws(P);
         const BatchRve &rv = P.rves[sh.rid];
-        modes_setup<QS, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
+        modes_setup<F64, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
                         P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r);
       }
       // 2. the right-hand side's norm
       double rn0;
       {
-        const ModesSpace<QS> ws(P);
-        rn0 = rhs_norm<PER>(
-            march_residual<CUBE, QS, PER>(ws.w, reinterpret_cast<float *>(ws.r)).x, ws.w, ph);
+        const ModesSpace<V, QS> ws(P);
+        rn0 = rhs_norm<F64, PER>(march_residual<V, CUBE, QS, PER>(ws.w, ws.r).x, ws.w, ph);
         ph ^= 1;
       }
       // 3. refinement
@@ -921,9 +1013,9 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       for (;;) {
         double v[2];
         {
-          const ModesSpace<QS> ws(P);
-          if (!QS && rho != 0.0) save_p<PER>(ws.q);
-          const double2 d = march_residual<CUBE, QS, PER>(ws.w, reinterpret_cast<float *>(ws.r));
+          const ModesSpace<V, QS> ws(P);
+          if (!QS && rho != 0.0) save_p<V, PER>(ws.q);
+          const double2 d = march_residual<V, CUBE, QS, PER>(ws.w, ws.r);
           v[0] = d.x;
           v[1] = d.y;
           cta_sum<2>(v, ph);
@@ -935,24 +1027,24 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         // a reliable update: r is the true residual, the search direction
         // goes on with beta = r.z / rho of the last step
         {
-          const ModesSpace<QS> ws(P);
-          if (!QS) restore_p<PER>(ws.q, rho != 0.0);
-          update_p<CUBE, false, PER>(ws.r, rho != 0.0 ? (float)(v[1] / rho) : 0.f);
+          const ModesSpace<V, QS> ws(P);
+          if (!QS) restore_p<V, PER>(ws.q, rho != 0.0);
+          update_p<V, CUBE, false, PER>(ws.r, rho != 0.0 ? v[1] / rho : 0.0);
         }
         rho = v[1];
         __syncthreads();
         int it = 0;
         while (it < P.max_inner) {
           {
-            const ModesSpace<QS> ws(P);
-            v[0] = march_apply<CUBE, QS, PER>(ws.q);
+            const ModesSpace<V, QS> ws(P);
+            v[0] = march_apply<V, CUBE, QS, PER>(ws.q);
           }
           double d[1] = {v[0]};
           cta_sum<1>(d, ph);
           {
-            const ModesSpace<QS> ws(P);
+            const ModesSpace<V, QS> ws(P);
             const double2 u =
-                update_xr<CUBE, QS, PER>(ws.r, ws.x, ws.q, d[0] != 0.0 ? (float)(rho / d[0]) : 0.f, it == 0);
+                update_xr<V, CUBE, QS, PER>(ws.r, ws.x, ws.q, d[0] != 0.0 ? rho / d[0] : 0.0, it == 0);
             v[0] = u.x;
             v[1] = u.y;
           }
@@ -960,15 +1052,15 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
           it++;
           if (v[1] <= thr) break;
           {
-            const ModesSpace<QS> ws(P);
-            update_p<CUBE, QS, PER>(ws.r, rho != 0.0 ? (float)(v[0] / rho) : 0.f);
+            const ModesSpace<V, QS> ws(P);
+            update_p<V, CUBE, QS, PER>(ws.r, rho != 0.0 ? v[0] / rho : 0.0);
           }
           rho = v[0];
           __syncthreads();
         }
         if (it > 0) {
-          const ModesSpace<QS> ws(P);
-          update_w<PER>(ws.x, ws.w);
+          const ModesSpace<V, QS> ws(P);
+          update_w<V, PER>(ws.x, ws.w);
         }
         outer++;
         if (threadIdx.x == 0) {
@@ -979,7 +1071,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       }
       // 4. averages
       {
-        const ModesSpace<QS> ws(P);
+        const ModesSpace<V, QS> ws(P);
         ph = march_average<PER>(ws.w, ph);
       }
       if (threadIdx.x == 0) {
@@ -1003,13 +1095,15 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
 using ModesFn = void (*)(ModesParams);
 
 // the instantiated classes (threads, CTAs per SM, q in shared memory): the
-// largest blocks of which 6, 3, 2 and 1 fit an SM's register file
-#define SP_MODES_CLASSES(X) \
-  X(64, 8, true) X(160, 3, true) X(256, 2, true) X(512, 1, true) X(640, 1, false)
-#define SP_MODES_EXTERN(NT, MINB, QS) \
-  extern template __global__ void k_modes<NT, MINB, true, QS, false>(ModesParams); \
-  extern template __global__ void k_modes<NT, MINB, false, QS, false>(ModesParams); \
-  extern template __global__ void k_modes<NT, MINB, true, QS, true>(ModesParams); \
-  extern template __global__ void k_modes<NT, MINB, false, QS, true>(ModesParams);
+// largest blocks of which 8, 3, 2 and 1 fit an SM's register file at 128
+// registers a thread, and one of 96 registers for the largest meshes
+#define SP_MODES_CLASSES(X, V) \
+  X(V, 64, 8, true) X(V, 160, 3, true) X(V, 256, 2, true) X(V, 512, 1, true) \
+  X(V, 512, 1, false) X(V, 640, 1, false)
+#define SP_MODES_EXTERN(V, NT, MINB, QS) \
+  extern template __global__ void k_modes<V, NT, MINB, true, QS, false>(ModesParams); \
+  extern template __global__ void k_modes<V, NT, MINB, false, QS, false>(ModesParams); \
+  extern template __global__ void k_modes<V, NT, MINB, true, QS, true>(ModesParams); \
+  extern template __global__ void k_modes<V, NT, MINB, false, QS, true>(ModesParams);
 
 }  // namespace sp

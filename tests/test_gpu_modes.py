@@ -38,9 +38,10 @@ def voxel_batch(cube, seed):
 
 
 @pytest.mark.parametrize("cube", [True, False])
-def test_edges_match_oracle(cube):
+@pytest.mark.parametrize("precision", [mb.SP_PREC_MIXED, mb.SP_PREC_FP64])
+def test_edges_match_oracle(precision, cube):
     descs, ets, meshes, eps = voxel_batch(cube, 5 + cube)
-    b = mb.Batch(descs, nrhs=3, rtol=1e-10, threads=512, ctas_per_sm=1)
+    b = mb.Batch(descs, nrhs=3, rtol=1e-10, threads=512, ctas_per_sm=1, precision=precision)
     for i, et in enumerate(ets):
         b.set_etype(i, et)
     stress, strain, info = b.homogenize(np.ascontiguousarray(eps))
