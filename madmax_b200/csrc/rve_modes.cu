@@ -5,25 +5,37 @@
 
 namespace sp {
 
-SP_MODES_CLASSES(SP_MODES_EXTERN, F2)
-SP_MODES_CLASSES(SP_MODES_EXTERN, double)
+SP_MODES_CLASSES(SP_MODES_EXTERN, F2, false)
+SP_MODES_CLASSES(SP_MODES_EXTERN, F2, true)
+SP_MODES_CLASSES(SP_MODES_EXTERN, double, false)
+SP_MODES_CLASSES(SP_MODES_EXTERN, double, true)
+SP_MODES_PERIODIC(SP_MODES_EXTERN, F2)
+SP_MODES_PERIODIC(SP_MODES_EXTERN, double)
+SP_MODES_AFFINE(SP_MODES_EXTERN, F2)
+SP_MODES_AFFINE(SP_MODES_EXTERN, double)
 
 struct ModesClass {
-  int threads, minb;
-  bool qs;
+  int threads, minb, on;
   ModesFn fn[2][2][2];  // [FP64][periodic][cubes]
 };
 
+#define SP_MODES_FNS(V, NT, MINB, ON, PER) \
+  {k_modes<V, NT, MINB, false, ON, PER>, k_modes<V, NT, MINB, true, ON, PER>}
+#define SP_MODES_ROW(V, NT, MINB, ON, PER) \
+  {NT, MINB, ON, \
+   {{SP_MODES_FNS(F2, NT, MINB, ON, false), SP_MODES_FNS(F2, NT, MINB, ON, true)}, \
+    {SP_MODES_FNS(double, NT, MINB, ON, false), SP_MODES_FNS(double, NT, MINB, ON, true)}}},
 static const ModesClass kClasses[] = {
-#define SP_MODES_FNS(V, NT, MINB, QS) \
-  {{k_modes<V, NT, MINB, false, QS, false>, k_modes<V, NT, MINB, true, QS, false>}, \
-   {k_modes<V, NT, MINB, false, QS, true>, k_modes<V, NT, MINB, true, QS, true>}}
-#define SP_MODES_ROW(V, NT, MINB, QS) \
-  {NT, MINB, QS, {SP_MODES_FNS(V, NT, MINB, QS), SP_MODES_FNS(double, NT, MINB, QS)}},
-    SP_MODES_CLASSES(SP_MODES_ROW, F2)
+    SP_MODES_CLASSES(SP_MODES_ROW, F2, false)
+    {640, 1, 1,
+     {{{nullptr, nullptr}, SP_MODES_FNS(F2, 640, 1, 1, true)},
+      {{nullptr, nullptr}, SP_MODES_FNS(double, 640, 1, 1, true)}}},
+    {512, 1, 0,
+     {{SP_MODES_FNS(F2, 512, 1, 0, false), {nullptr, nullptr}},
+      {SP_MODES_FNS(double, 512, 1, 0, false), {nullptr, nullptr}}}},
+};
 #undef SP_MODES_ROW
 #undef SP_MODES_FNS
-};
 constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
 
 // shared memory of one SM and what a block holds beside its dynamic part
@@ -37,20 +49,21 @@ static int class_room(const ModesClass &k) {
 
 // An RVE runs on the smallest class whose threads hold one element column
 // each and whose shared memory holds its vectors beside the
-// class's other CTAs; it needs an interior node on every axis and at most 31
+// class's other CTAs; it needs an interior node on every axis, at most 32
 // element layers, 30 under periodic conditions (a column's materials are one
-// 32-bit mask, which repeats two layers then).  Larger RVEs
-// keep the solve_rve kernel.
+// 32-bit mask, which repeats two layers then), and at most 1024 columns.
+// Larger RVEs keep the solve_rve kernel.
 int modes_class(const MeshGeo &g, const double *len, bool per, bool f64) {
   if (g.nex < 2 || g.ney < 2 || g.nez < 2) return -1;
-  if (g.nez > (per ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ)) return -1;
-  if ((long long)g.nex * g.ney > 640) return -1;
-  const ModesGeo G(g.nex, g.ney, g.nez, per, f64);
+  if (g.nez > (per ? SP_MODES_MAX_NEZ - 2 : SP_MODES_MAX_NEZ)) return -1;
+  if ((long long)g.nex * g.ney > SP_MODES_MAX_COLS) return -1;
   const double hx = len[0] / g.nex, hy = len[1] / g.ney, hz = len[2] / g.nez;
   const int cube = hx == hy && hx == hz;
   for (int c = 0; c < kNumClasses; c++) {
     const ModesClass &k = kClasses[c];
-    if (G.warps() * 32 <= k.threads && G.smem(k.qs) <= class_room(k)) return 2 * c + cube;
+    if (!k.fn[f64][per][cube]) continue;
+    const ModesGeo G(g.nex, g.ney, g.nez, per, f64, k.on);
+    if (G.rows >= 1 && G.warps() * 32 <= k.threads && G.smem() <= class_room(k)) return 2 * c + cube;
   }
   return -1;
 }
@@ -69,13 +82,14 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     ModesBucket &b = out->buckets.back();
     b.fn = k.fn[f64][per][c & 1];
     b.nrve = (int)ord.size();
-    int ntot = 0, wlen = 0;
+    int ntot = 0, wlen = 0, elen = 0;
     for (int i : ord) {
-      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez, per, f64);
+      const ModesGeo G(geo[i].nex, geo[i].ney, geo[i].nez, per, f64, k.on);
       b.threads = std::max(b.threads, G.warps() * 32);
-      b.smem = std::max(b.smem, G.smem(k.qs));
+      b.smem = std::max(b.smem, G.smem());
       ntot = std::max(ntot, G.ntot);
       wlen = std::max(wlen, G.wlen());
+      elen = std::max(elen, 6 * G.mz * G.nex);
     }
     b.w_stride = ((size_t)3 * wlen + 15) / 16 * 16;
     b.v_stride = ((size_t)3 * ntot + 15) / 16 * 16;
@@ -97,7 +111,11 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     b.grid = (int)std::min<long long>((long long)d->nsm * nb, (long long)b.nrve * nrhs);
     SP_TRY(dmalloc((void **)&b.d_order, ord.size() * sizeof(int), &b.bytes));
     SP_TRY(dmalloc((void **)&b.ws_w, b.grid * b.w_stride * sizeof(double), &b.bytes));
-    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (k.qs ? 2 : 3) * b.v_stride * sizeof(double), &b.bytes));
+    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (4 - k.on) * b.v_stride * sizeof(double), &b.bytes));
+    if (k.on < 2) {
+      b.e_stride = ((size_t)elen + 15) / 16 * 16;
+      SP_TRY(dmalloc((void **)&b.ws_e, b.grid * b.e_stride * sizeof(double), &b.bytes));
+    }
     if (cudaMemcpy(b.d_order, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice))
       return sp_set_error(SP_ERR_CUDA, "sp_batch_create: upload failed");
   }
@@ -119,6 +137,7 @@ void modes_free(ModesPlan *m) {
     cudaFree(k.d_order);
     cudaFree(k.ws_w);
     cudaFree(k.ws_v);
+    cudaFree(k.ws_e);
   }
   for (cudaStream_t s : m->side) cudaStreamDestroy(s);
   for (cudaEvent_t e : m->joined) cudaEventDestroy(e);
@@ -153,6 +172,8 @@ int modes_launch(const ModesPlan &m, const ModesCommon &c, int *counters, cudaSt
     P.ws_v = k.ws_v;
     P.w_stride = k.w_stride;
     P.v_stride = k.v_stride;
+    P.ws_e = k.ws_e;
+    P.e_stride = k.e_stride;
     P.rtol = c.rtol;
     P.inner_rtol = c.inner_rtol;
     P.max_outer = c.max_outer;

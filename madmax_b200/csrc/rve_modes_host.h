@@ -14,8 +14,8 @@ struct ModesBucket {
   int threads = 0, grid = 0, smem = 0, nrve = 0;
   int *d_order = nullptr;
   double *ws_w = nullptr;
-  void *ws_v = nullptr;
-  size_t w_stride = 0, v_stride = 0, bytes = 0;
+  void *ws_v = nullptr, *ws_e = nullptr;
+  size_t w_stride = 0, v_stride = 0, e_stride = 0, bytes = 0;
 };
 
 // The launches of a batch: every bucket but the first on a side stream of its

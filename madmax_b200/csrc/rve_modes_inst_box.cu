@@ -3,7 +3,8 @@
 #include "rve_modes_kernel.cuh"
 
 namespace sp {
-#define SP_MODES_DEFINE(V, NT, MINB, QS) \
-  template __global__ void k_modes<V, NT, MINB, false, QS, false>(ModesParams);
-SP_MODES_CLASSES(SP_MODES_DEFINE, F2)
+#define SP_MODES_DEFINE(V, NT, MINB, ON, PER) \
+  template __global__ void k_modes<V, NT, MINB, false, ON, PER>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE, F2, false)
+SP_MODES_AFFINE(SP_MODES_DEFINE, F2)
 }  // namespace sp

@@ -3,7 +3,8 @@
 #include "rve_modes_kernel.cuh"
 
 namespace sp {
-#define SP_MODES_DEFINE(V, NT, MINB, QS) \
-  template __global__ void k_modes<V, NT, MINB, true, QS, false>(ModesParams);
-SP_MODES_CLASSES(SP_MODES_DEFINE, double)
+#define SP_MODES_DEFINE(V, NT, MINB, ON, PER) \
+  template __global__ void k_modes<V, NT, MINB, true, ON, PER>(ModesParams);
+SP_MODES_CLASSES(SP_MODES_DEFINE, double, false)
+SP_MODES_AFFINE(SP_MODES_DEFINE, double)
 }  // namespace sp

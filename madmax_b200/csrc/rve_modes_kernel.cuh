@@ -32,13 +32,15 @@ struct ModesParams {
   unsigned *done;            // [nrve] finished load cases (0 between launches)
   int *counter;
   double *ws_w;    // per CTA [3][wlen]
-  void *ws_v;      // per CTA r, x and (q not in shared memory) q: [3][ntot] 8-byte values each
-  size_t w_stride, v_stride;  // v_stride: of one of them
+  void *ws_v;      // per CTA [3][ntot] 8-byte values each of r, x, (q in L2) q, (p too) p
+  void *ws_e;      // per CTA (q in L2) shares that cross strips: 2 x [planes][nex][3] values
+  size_t w_stride, v_stride, e_stride;  // v_stride: of one of them
   double rtol, inner_rtol;
   int max_outer, max_inner;
 };
 
-constexpr int SP_MODES_MAX_NEZ = 31;  // a column's materials are one 32-bit mask
+constexpr int SP_MODES_MAX_NEZ = 32;  // a column's materials are one 32-bit mask
+constexpr int SP_MODES_MAX_COLS = 1024;
 constexpr int SP_MODES_MAX_WARPS = 20;
 
 // What the CTA shares while it solves one load case; the first thing in its
@@ -56,8 +58,8 @@ struct ModesShared {
   double red[2 * SP_MODES_MAX_WARPS * 10];
   double cc[2][CC_N];    // cube: lambda, mu, 2 mu, lambda/3, mu/3, (lambda + 4 mu)/9, times c0 a^2
   float2 c6[4][CC_N];    // ... as FP32 pairs: materials of the (lower, upper) layer
-  unsigned col[SP_MODES_MAX_WARPS * 32];  // per column: bit e = material of layer e
-  int nex, ney, nez, nface, mz, h, ntot, wlen, threads;
+  unsigned col[SP_MODES_MAX_COLS];  // per column: bit e = material of layer e
+  int nex, ney, nez, nface, mz, h, ntot, wlen, rows;  // rows: of a strip
   int job, rid, k, outer, inner, wcols, qoff, cntoff, pad[3];  // qoff, cntoff: bytes from p on
 };
 static_assert(sizeof(ModesShared) % 16 == 0, "vectors follow on a 16-byte boundary");
@@ -68,34 +70,42 @@ static_assert(sizeof(ModesShared) % 16 == 0, "vectors follow on a 16-byte bounda
 // columns are preceded by a repetition of its last one, the left neighbour of
 // its first.
 // FP32 vectors have a slot for each pair of planes, FP64 ones for each plane;
-// a value is 8 bytes either way.
+// a value is 8 bytes either way.  `on`: the vectors in shared memory -- 2: p
+// and q, 1: p, 0: neither.  Without q there (affine conditions) the columns
+// are marched in strips of `rows` rows, 512 threads at most, one strip after
+// another.
 struct ModesGeo {
-  int nex, ney, nez, nface, mz, h, ntot, per;
-  __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic, bool f64)
+  int nex, ney, nez, nface, mz, h, ntot, per, on, rows;
+  __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic, bool f64, int onchip)
       : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(periodic ? ez : ez - 1),
-        h(f64 ? mz : (mz + 1) / 2), ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic) {}
+        h(f64 ? mz : (mz + 1) / 2), ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic), on(onchip), rows(ey) {
+    if (on < 2 && !per) {
+      const int fit = 16 * wcols() / rowlanes(), n = fit > 0 ? (ey + fit - 1) / fit : 0;
+      rows = n > 0 ? (ey + n - 1) / n : 0;
+    }
+  }
   __host__ __device__ int wlen() const { return mz * nface + (per ? 0 : nex + 2); }
-  // lanes of a row, of all rows, and of a warp: 32 where rows start at lane 0
-  // (whose left neighbour is the boundary, or its own repetition), else 31
-  // and a repetition of the last lane of the previous warp
+  // lanes of a row, of a strip's rows, and of a warp: 32 where rows start at
+  // lane 0 (whose left neighbour is the boundary, or its own repetition),
+  // else 31 and a repetition of the last lane of the previous warp
   __host__ __device__ int rowlanes() const { return per ? nex + 1 : nex; }
-  __host__ __device__ int lanes() const { return rowlanes() * ney; }
+  __host__ __device__ int lanes() const { return rowlanes() * rows; }
   __host__ __device__ int wcols() const { return 32 % rowlanes() == 0 ? 32 : 31; }
   __host__ __device__ int warps() const { return (lanes() + wcols() - 1) / wcols(); }
-  // Dynamic shared memory: tables, p, then (QS) q, whose place the FP64
-  // residual's face state and exchange planes take too, or (no q) two
-  // exchange planes and the state in p's place; material counts.
+  // Dynamic shared memory: tables, p, then q, whose place the FP64 residual's
+  // face state and exchange planes take too, or (q in L2) two exchange planes,
+  // with the state in p's place or after them; material counts.
   __host__ __device__ int state() const { return 32 * warps() * 8; }
-  __host__ __device__ int pbytes(bool qs) const {
-    const int a = ntot * 24, b = qs ? 0 : 25 * state();
+  __host__ __device__ int pbytes() const {
+    const int a = on >= 1 ? ntot * 24 : 0, b = on == 1 ? 25 * state() : 0;
     return a > b ? a : b;
   }
-  __host__ __device__ int qbytes(bool qs) const {
-    const int a = qs ? ntot * 24 : 0, b = 2 * nface * 24 + (qs ? 13 * state() : 0);
+  __host__ __device__ int qbytes() const {
+    const int a = on == 2 ? ntot * 24 : 0, b = 2 * nex * rows * 24 + (on == 1 ? 0 : 13 * state());
     return a > b ? a : b;
   }
-  __host__ __device__ int smem(bool qs) const {
-    return (int)sizeof(ModesShared) + pbytes(qs) + qbytes(qs) + (h * nface + 15) / 16 * 16;
+  __host__ __device__ int smem() const {
+    return (int)sizeof(ModesShared) + pbytes() + qbytes() + (h * nface + 15) / 16 * 16;
   }
 };
 
@@ -161,21 +171,27 @@ __device__ __forceinline__ void cta_sum(double (&v)[NV], int &ph) {
   ph ^= 1;
 }
 
-// A thread's place in the march.  f: its element column (face); the repeated
-// lanes and the padding threads of the last warp write nothing.
+// A thread's place in the march of a strip.  f: its element column (face);
+// the repeated lanes and the padding threads of the last warp write nothing.
 template <bool PER>
 struct ModesLane {
   int f;
+  int f0, f1;    // columns of the strip: [f0, f1)
   int dx, dy;    // from f to the columns at x + 1 and y + 1
+  int threads;   // of the warps that have a column
   bool warp_on;  // the warp has a column
   bool column;   // the thread has one
   bool owner;    // ... and its node (ex, ey) is an unknown
-  __device__ __forceinline__ ModesLane() {
+  __device__ __forceinline__ explicit ModesLane(int y0 = 0) {
     const ModesShared &sh = msh();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rep = 32 - sh.wcols;
     const int i = warp * sh.wcols + lane - rep, row = PER ? sh.nex + 1 : sh.nex;
-    const int n = row * sh.ney, ic = min(max(i, 0), n - 1);
+    const int rows = min(sh.rows, sh.ney - y0);
+    const int n = row * rows, ic = min(max(i, 0), n - 1);
+    f0 = y0 * sh.nex;
+    f1 = f0 + rows * sh.nex;
     warp_on = warp * sh.wcols < n;
+    threads = (n + sh.wcols - 1) / sh.wcols * 32;
     column = lane >= rep && i < n;
     if (PER) {
       const int y = ic / row, v = ic - y * row, x = v ? v - 1 : sh.nex - 1;
@@ -185,13 +201,15 @@ struct ModesLane {
       column = column && v != 0;
       owner = column;
     } else {
-      f = ic;
+      f = f0 + ic;
       dx = 1;
       dy = sh.nex;
       owner = column && f >= sh.nex && f % sh.nex != 0;
     }
   }
 };
+
+__device__ __forceinline__ unsigned shr32(unsigned m, int n) { return n < 32 ? m >> n : 0u; }
 
 // the columns at x - 1 and y - 1 of an owner's column
 template <bool PER>
@@ -207,21 +225,27 @@ __device__ __forceinline__ void plane_sync(int threads) {
   asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-// q = A p: p, q in shared memory ([slot][3] pairs), q in qg ([3][ntot]) when
-// QS is false; returns the thread's share of p.q.
-template <typename V, bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
+// q = A p on the strip from row y0: p [slot][3] and q in shared memory, or q
+// in qg ([3][ntot]), or p in pg and the shares for the next strip's first row
+// in eg too; returns the thread's share of p.q.
+template <typename V, bool CUBE, int ON, bool PER>
+__device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg, const V *pg, V *eg,
+                                           int y0) {
   using MT = ModesType<V>;
-  constexpr bool F64 = MT::F64;
+  constexpr bool F64 = MT::F64, QS = ON == 2, STRIPS = ON < 2 && !PER;
   // registers to spare for the next slot's values (FP64 has none)
   constexpr bool AHEAD = QS && !F64;
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
+  const ModesLane<PER> T(y0);
   const unsigned mats = sh.col[T.f];
   const int nface = sh.nface, nf3 = 3 * nface, h = sh.h, ntot = sh.ntot;
   const int right = PER ? 3 * T.dx : 3, up = 3 * T.dy;
-  const V *pf = mp<V>() + 3 * T.f;  // corner (0, 0) of slot 0
-  V *const qf = mq<V>() + 3 * T.f;
+  const V *pf = (ON ? mp<V>() : pg) + 3 * T.f;  // corner (0, 0) of slot 0
+  V *const qf = mq<V>() + 3 * (T.f - T.f0);
+  const int ex3 = QS ? nf3 : 3 * sh.rows * sh.nex;
+  // the halves of eg: written by one strip, read by the next
+  const int eread = STRIPS && !((y0 / sh.rows) & 1) ? 3 * sh.mz * sh.nex : 0;
+  const int ewrite = STRIPS ? 3 * sh.mz * sh.nex - eread : 0;
   const bool odd = !F64 && (sh.mz & 1) != 0;
   V raw[3][4], Fa[3][4], Fb[3][4], acc[3][4];
   auto load = [&](const V *a) {
@@ -300,13 +324,19 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
   // one step: F0 the modes of the face below, F1 takes those above (two steps
   // a trip, so that the faces change places without copies)
   auto step = [&](int s, V (&F0)[3][4], V (&F1)[3][4]) {
-    V low[3];
+    V low[3], edge[3];
     if (T.warp_on) {
       V S[3][3], D[3][4], high[3];
+      if (STRIPS) {
+        if (ON == 0 && s + 1 < h) asm volatile("prefetch.global.L1 [%0];" ::"l"(pf + (s + 1) * nf3));
+        if (s > 0 && T.f0 > 0 && T.f < T.f0 + sh.nex)
+#pragma unroll
+          for (int c = 0; c < 3; c++) edge[c] = eg[eread + 3 * ((s - 1) * sh.nex + T.f - T.f0) + c];
+      }
       if (!AHEAD) next(s);
       face_modes(raw, F1);
       layer_modes(F0, F1, S, D);
-      const unsigned ma = (mats >> s) & 1u;
+      const unsigned ma = shr32(mats, s) & 1u;
       if constexpr (F64) {
         if constexpr (CUBE) {
           const double *ct = sh.cc[ma];
@@ -316,7 +346,7 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
           modes_box(S, D, [ct](int i) { return ct[i]; });
         }
       } else {
-        const unsigned mb = (mats >> (s + h)) & 1u;
+        const unsigned mb = shr32(mats, s + h) & 1u;
         if constexpr (CUBE) {
           const float2 *ct = sh.c6[ma + 2 * mb];
           modes_cube(S, D, [ct](int i) { return F2{ct[i]}; });
@@ -328,22 +358,30 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
       layer_back(S, D, acc, low, high);
       // the upper row's share waits where that row's q goes (QS), or in the
       // exchange planes in turn
-      V *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3 + up;
-      if (T.column && s > 0 && (PER || T.f + sh.nex < nface))
+      V *const e = qf + (QS ? (s - 1) : (s & 1)) * ex3 + up;
+      if (T.column && s > 0) {
+        if (PER || T.f + sh.nex < T.f1) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) e[c] = high[c];
+          for (int c = 0; c < 3; c++) e[c] = high[c];
+        } else if (STRIPS && T.f1 < nface) {
+#pragma unroll
+          for (int c = 0; c < 3; c++)
+            eg[ewrite + 3 * ((s - 1) * sh.nex + T.f + sh.nex - T.f1) + c] = high[c];
+        }
+      }
       // the next slot's values before the barrier
       if (AHEAD) next(s + 1);
     }
     if (s > 0) {
-      plane_sync(sh.threads);
+      plane_sync(T.threads);
       if (T.owner) {
-        V *const e = qf + (QS ? (s - 1) : (s & 1)) * nf3;
+        V *const e = qf + (QS ? (s - 1) : (s & 1)) * ex3;
+        const bool seam = STRIPS && T.f0 > 0 && T.f < T.f0 + sh.nex;
         const V *ps = pf + (s - 1) * nf3;
         V t = zero_of(V());
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          low[c] = low[c] + e[c];
+          low[c] = low[c] + (seam ? edge[c] : e[c]);
           if constexpr (F64) {
             if (PER && s == 1 && T.f == 0) low[c] = 0.0;  // the fixed node
           } else {
@@ -377,18 +415,22 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg) {
 // between layers: in registers they spill, and a spill goes to L2, since the
 // vectors leave L1 next to nothing (n = 20: 285k cycles an evaluation with
 // spills, 80k without).
-template <typename V, bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double2 march_residual(const double *w, typename ModesType<V>::Mem *rv) {
+template <typename V, bool CUBE, int ON, bool PER>
+__device__ __noinline__ double2 march_residual(const double *w, typename ModesType<V>::Mem *rv,
+                                               double *eg, int y0) {
+  constexpr bool QS = ON != 1, STRIPS = ON < 2 && !PER;  // QS: 128 registers a thread
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
+  const ModesLane<PER> T(y0);
   const unsigned mats = sh.col[T.f];
   const int nface = sh.nface, right = PER ? T.dx : 1, up = T.dy, wl = sh.wlen, mz = sh.mz, h = sh.h;
   constexpr bool F64 = ModesType<V>::F64;
   double *const ex = mq<double>();  // two exchange planes
   const uint8_t *const cnt = mcnt();
+  const int eread = STRIPS && !((y0 / sh.rows) & 1) ? 3 * mz * sh.nex : 0;  // (see march_apply)
+  const int ewrite = STRIPS ? 3 * mz * sh.nex - eread : 0;
   // [c][m] of the running forces at 4 c + m, of the face's modes 12 further;
   // an odd number of doubles a thread (no bank conflicts)
-  double *const state = (QS ? ex + 6 * nface : mp<double>()) +
+  double *const state = (QS ? ex + 6 * sh.rows * sh.nex : mp<double>()) +
                         (T.warp_on ? threadIdx.x : 0) * (QS ? 13 : 25);
   double n2 = 0.0, rz = 0.0;
   double F0[3][4] = {};  // (QS)
@@ -423,9 +465,12 @@ __device__ __noinline__ double2 march_residual(const double *w, typename ModesTy
   load(0);
 #pragma unroll 1
   for (int s = 0; s <= mz; s++) {
-    double low[3];
-    double *const exs = ex + (s & 1) * 3 * nface;
+    double low[3], edge[3];
+    double *const exs = ex + ((s & 1) * sh.rows * sh.nex + T.f - T.f0) * 3;
     if (T.warp_on) {
+      if (STRIPS && s > 0 && T.f0 > 0 && T.f < T.f0 + sh.nex)
+#pragma unroll
+        for (int c = 0; c < 3; c++) edge[c] = eg[eread + 3 * ((s - 1) * sh.nex + T.f - T.f0) + c];
       double S[3][3], D[3][4];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
@@ -447,14 +492,18 @@ __device__ __noinline__ double2 march_residual(const double *w, typename ModesTy
         D[c][0] += sh.A[3 * c + 2];
       }
       if constexpr (CUBE) {
-        const double *ct = sh.cc[(mats >> s) & 1u];
+        const double *ct = sh.cc[shr32(mats, s) & 1u];
         modes_cube(S, D, [ct](int i) { return ct[i]; });
       } else {
-        const double *ct = sh.cd[(mats >> s) & 1u];
+        const double *ct = sh.cd[shr32(mats, s) & 1u];
         modes_box(S, D, [ct](int i) { return ct[i]; });
       }
-      double *e = exs + 3 * (T.f + up);
-      const bool put = T.column && (PER || T.f + up < nface);
+      double *e = exs + 3 * up;
+      bool put = T.column && (PER || T.f + up < T.f1);
+      if (STRIPS && T.column && s > 0 && T.f + up >= T.f1 && T.f1 < nface) {
+        e = eg + ewrite + 3 * ((s - 1) * sh.nex + T.f + up - T.f1);
+        put = true;
+      }
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         double *const ac = state + 4 * c;
@@ -481,15 +530,15 @@ __device__ __noinline__ double2 march_residual(const double *w, typename ModesTy
         for (int m = 0; m < 4; m++) raw[c][m] = 0.0;
     }
     if (s > 0) {
-      plane_sync(sh.threads);
+      plane_sync(T.threads);
       if (T.owner) {
-        const double *e = exs + 3 * T.f;
+        const bool seam = STRIPS && T.f0 > 0 && T.f < T.f0 + sh.nex;
         const bool hi = !F64 && s - 1 >= h;
         const int i = (hi ? s - 1 - h : s - 1) * nface + T.f;
         const unsigned cv = hi ? cnt[i] >> 4 : cnt[i] & 15u;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          double b = -(low[c] + e[c]);
+          double b = -(low[c] + (seam ? edge[c] : exs[c]));
           if (PER && s == 1 && T.f == 0) b = 0.0;  // the fixed node
           n2 += b * b;
           if constexpr (F64) {
@@ -517,11 +566,13 @@ __device__ __noinline__ double2 march_residual(const double *w, typename ModesTy
 template <bool PER>
 __device__ __noinline__ int march_average(const double *w, int ph) {
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
   double m[10];
 #pragma unroll
   for (int q = 0; q < 10; q++) m[q] = 0.0;
-  if (T.column) m[9] = (double)__popc(sh.col[T.f] & ~(PER ? (1u | 2u << sh.nez) : 0u));
+#pragma unroll 1
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+  const ModesLane<PER> T(y0);
+  if (T.column) m[9] += (double)__popc(sh.col[T.f] & ~(PER ? (1u | 2u << sh.nez) : 0u));
   if (T.owner) {
     const int wl = sh.wlen, mz = sh.mz, nface = sh.nface;
     int left, down;
@@ -543,6 +594,7 @@ __device__ __noinline__ int march_average(const double *w, int ph) {
         for (int d = 0; d < 3; d++) m[3 * c + d] = fma(k[d], v, m[3 * c + d]);
       }
     }
+  }
   }
   cta_sum<10>(m, ph);
   __syncthreads();
@@ -575,15 +627,17 @@ __device__ __forceinline__ void slot_dinv(int i, double (&dz)[3]) {
 
 // One group of up to U slots of update_xr: all loads before the stores, one L2
 // round trip for the group.
-template <typename V, bool CUBE, bool QS, int U>
-__device__ __forceinline__ void xr_slots(int s0, int f, typename ModesType<V>::Mem *rg,
+template <typename V, bool CUBE, int ON, int U>
+__device__ __forceinline__ void xr_slots(int s0, int f, const V *pg, typename ModesType<V>::Mem *rg,
                                          typename ModesType<V>::Mem *xg,
                                          const typename ModesType<V>::Mem *qg, V al, V nal,
                                          bool first, double &vz, double &vr) {
   using MT = ModesType<V>;
   const ModesShared &sh = msh();
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
-  V *const p = mp<V>();
+  constexpr bool QS = ON == 2;
+  V *const q_ = mp<V>() + 3 * ntot;  // (QS)
+  const V *const p = ON ? mp<V>() : pg;
   V r[U][3], q[U][3];
 #pragma unroll
   for (int j = 0; j < U; j++)
@@ -603,14 +657,14 @@ __device__ __forceinline__ void xr_slots(int s0, int f, typename ModesType<V>::M
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const int o = c * ntot + i;
-      const V rn = mad(nal, QS ? p[3 * (ntot + i) + c] : q[j][c], r[j][c]);
+      const V rn = mad(nal, QS ? q_[3 * i + c] : q[j][c], r[j][c]);
       const V dx = al * p[3 * i + c];
       MT::st(rg + o, rn);
       if (first)
         MT::st(xg + o, dx);
       else
         MT::add(xg + o, dx);  // (no value back: nothing waits for it)
-      if constexpr (QS) p[3 * (ntot + i) + c] = rn;
+      if constexpr (QS) q_[3 * i + c] = rn;
       sz = mad(rn, dz[c] * rn, sz);
       sr = mad(rn, rn, sr);
     }
@@ -623,32 +677,34 @@ __device__ __forceinline__ void xr_slots(int s0, int f, typename ModesType<V>::M
 // correction's first step); returns its shares of r.z and r.r.  x is added to
 // in L2: only this thread touches its entries.  q's slots take the new r for
 // the direction update.
-template <typename V, bool CUBE, bool QS, bool PER>
-__device__ __noinline__ double2 update_xr(typename ModesType<V>::Mem *rg,
+template <typename V, bool CUBE, int ON, bool PER>
+__device__ __noinline__ double2 update_xr(const V *pg, typename ModesType<V>::Mem *rg,
                                           typename ModesType<V>::Mem *xg,
                                           const typename ModesType<V>::Mem *qg, double alpha,
                                           bool first) {
-  const ModesLane<PER> T;
-  if (!T.owner) return make_double2(0.0, 0.0);
   const int h = msh().h;
   const typename ModesType<V>::S a = (typename ModesType<V>::S)alpha;
   const V al = ModesType<V>::splat(a), nal = ModesType<V>::splat(-a);
   double vz = 0.0, vr = 0.0;
-  constexpr int U = QS ? 5 : 3;
+  constexpr int U = ON == 2 ? 5 : 3;
 #pragma unroll 1
-  for (int s = 0; s < h; s += U)
-    xr_slots<V, CUBE, QS, U>(s, T.f, rg, xg, qg, al, nal, first, vz, vr);
+  for (int y0 = 0; y0 < (ON == 2 ? 1 : msh().ney); y0 += msh().rows) {
+    const ModesLane<PER> T(y0);
+    if (T.owner)
+#pragma unroll 1
+      for (int s = 0; s < h; s += U)
+        xr_slots<V, CUBE, ON, U>(s, T.f, pg, rg, xg, qg, al, nal, first, vz, vr);
+  }
   return make_double2(vz, vr);
 }
 
 // p = D^-1 r + beta p over the thread's column; r in q's slots (LOCAL) or in
 // rg.  beta = 0 starts afresh without reading p.
 template <typename V, bool CUBE, bool LOCAL, int U>
-__device__ __forceinline__ void p_slots(int s0, int f, const typename ModesType<V>::Mem *rg, V be,
+__device__ __forceinline__ void p_slots(int s0, int f, V *p, const typename ModesType<V>::Mem *rg, V be,
                                         bool fresh) {
   const ModesShared &sh = msh();
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h;
-  V *const p = mp<V>();
   V r[U][3], pv[U][3];
 #pragma unroll
   for (int j = 0; j < U; j++)
@@ -675,25 +731,31 @@ __device__ __forceinline__ void p_slots(int s0, int f, const typename ModesType<
   }
 }
 
-template <typename V, bool CUBE, bool LOCAL, bool PER>
-__device__ __noinline__ void update_p(const typename ModesType<V>::Mem *rg, double beta) {
-  const ModesLane<PER> T;
-  if (!T.owner) return;
+template <typename V, bool CUBE, int ON, bool LOCAL, bool PER>
+__device__ __noinline__ void update_p(V *pg, const typename ModesType<V>::Mem *rg, double beta) {
   const int h = msh().h;
   const typename ModesType<V>::S b = (typename ModesType<V>::S)beta;
   const V be = ModesType<V>::splat(b);
   constexpr int U = LOCAL ? 3 : 5;
 #pragma unroll 1
-  for (int s = 0; s < h; s += U) p_slots<V, CUBE, LOCAL, U>(s, T.f, rg, be, b == 0);
+  for (int y0 = 0; y0 < (ON == 2 ? 1 : msh().ney); y0 += msh().rows) {
+    const ModesLane<PER> T(y0);
+    if (T.owner)
+#pragma unroll 1
+      for (int s = 0; s < h; s += U)
+        p_slots<V, CUBE, LOCAL, U>(s, T.f, ON ? mp<V>() : pg, rg, be, b == 0);
+  }
 }
 
 // w += x in FP64 over the thread's column
 template <typename V, bool PER>
 __device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, double *w) {
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
-  if (!T.owner) return;
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h, mz = sh.mz, wl = sh.wlen;
+#pragma unroll 1
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+  const ModesLane<PER> T(y0);
+  if (!T.owner) continue;
 #pragma unroll 1
   for (int s = 0; s < h; s++) {
     const int i = s * nface + T.f;
@@ -715,6 +777,7 @@ __device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, doub
       }
     }
   }
+  }
 }
 
 // The residual's face state takes p's place when q is not in shared memory:
@@ -723,39 +786,44 @@ __device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, doub
 template <typename V, bool PER>
 __device__ __noinline__ void save_p(typename ModesType<V>::Mem *qg) {
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
-  if (T.owner)
+#pragma unroll 1
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+    const ModesLane<PER> T(y0);
+    if (!T.owner) continue;
     for (int s = 0; s < sh.h; s++)
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const int i = s * sh.nface + T.f;
         ModesType<V>::st(qg + (c * sh.ntot + i), mp<V>()[3 * i + c]);
       }
+  }
   __syncthreads();
 }
 template <typename V, bool PER>
 __device__ __noinline__ void restore_p(const typename ModesType<V>::Mem *qg, bool saved) {
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
   for (int i = threadIdx.x; i < 3 * sh.ntot; i += blockDim.x) mp<V>()[i] = zero_of(V());
   __syncthreads();
-  if (T.owner && saved)
+#pragma unroll 1
+  for (int y0 = 0; saved && y0 < sh.ney; y0 += sh.rows) {
+    const ModesLane<PER> T(y0);
+    if (!T.owner) continue;
     for (int s = 0; s < sh.h; s++)
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const int i = s * sh.nface + T.f;
         mp<V>()[3 * i + c] = ModesType<V>::ld(qg + (c * sh.ntot + i));
       }
+  }
 }
 
 // the tables, materials and start vectors of one load case
-template <bool F64, bool PER>
+template <int ON, bool F64, bool PER>
 __device__ __noinline__ void modes_setup(const double *len, const double *mat,
                                          const uint8_t *etype, const double *eps, double *w,
-                                         void *rv) {
+                                         void *rv, void *pg) {
   ModesShared &sh = msh();
   const int t = threadIdx.x;
-  const ModesLane<PER> T;
   const int nface = sh.nface, nex = sh.nex, wl = sh.wlen;
   if (t < 3) {
     const int n = t == 0 ? sh.nex : (t == 1 ? sh.ney : sh.nez);
@@ -774,23 +842,29 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
     const int v = i == j ? i : (i + j == 1 ? 3 : (i + j == 3 ? 4 : 5));
     sh.E[t - 3] = i == j ? eps[v] : eps[v] / 2;
   }
-  unsigned mats = 0;
-  const uint8_t *et = etype + T.f;
-  if (T.warp_on)
-    for (int e = 0; e < sh.nez; e++) mats |= (unsigned)__ldg(et + e * nface) << e;
-  // bit s: the layer below plane s.  Periodic: layer s - 1, and the first
-  // ones again past the last
-  if (PER) mats = mats << 1 | mats >> (sh.nez - 1) | (mats & 1u) << (sh.nez + 1);
-  if (T.column) sh.col[T.f] = mats;
-  {
-    float4 *p = mp<float4>();  // (3 ntot pairs, rounded down to 16 bytes)
-    for (int i = t; i < 3 * sh.ntot / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t == 0) mp<float2>()[3 * sh.ntot - 1] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+    const ModesLane<PER> T(y0);
+    unsigned mats = 0;
+    const uint8_t *et = etype + T.f;
+    if (T.warp_on)
+      for (int e = 0; e < sh.nez; e++) mats |= (unsigned)__ldg(et + e * nface) << e;
+    // bit s: the layer below plane s.  Periodic: layer s - 1, and the first
+    // ones again past the last
+    if (PER) mats = mats << 1 | mats >> (sh.nez - 1) | (mats & 1u) << (sh.nez + 1);
+    if (T.column) sh.col[T.f] = mats;
+    // w's padding: the columns without an interior node (and below the row
+    // past the end)
+    if (T.column && (PER || !T.owner))
+      for (int c = 0; c < 3; c++)
+        for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = 0.0;
   }
-  // w's padding: the columns without an interior node and the row past the end
-  if (T.column && (PER || !T.owner))
-    for (int c = 0; c < 3; c++)
-      for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = 0.0;
+  {
+    // (3 ntot values, rounded down to 16 bytes)
+    float4 *p = ON ? mp<float4>() : static_cast<float4 *>(pg);
+    for (int i = t; i < 3 * sh.ntot / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t == 0) reinterpret_cast<float2 *>(p)[3 * sh.ntot - 1] = make_float2(0.f, 0.f);
+  }
   if (!PER)
     for (int i = t; i < 3 * (nex + 2); i += blockDim.x)
       w[(i / (nex + 2)) * wl + sh.mz * nface + i % (nex + 2)] = 0.0;
@@ -801,14 +875,17 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
   if (t < 9) sh.A[t] = 4.0 * sh.hx[t % 3] * sh.E[t];
   // fibre elements around the column's nodes; affine conditions: start of the
   // right-hand side's own residual, w = -eps.x inside, i.e. u = 0 inside
+#pragma unroll 1
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+  const ModesLane<PER> T(y0);
   if (T.owner) {
     int left, down;
     modes_below<PER>(T.f, left, down);
-    const unsigned m0 = mats, m1 = sh.col[T.f + left], m2 = sh.col[T.f + down],
+    const unsigned m0 = sh.col[T.f], m1 = sh.col[T.f + left], m2 = sh.col[T.f + down],
                    m3 = sh.col[T.f + left + down];
     auto count = [&](int pl) {
-      return __popc((m0 >> pl) & 3u) + __popc((m1 >> pl) & 3u) + __popc((m2 >> pl) & 3u) +
-             __popc((m3 >> pl) & 3u);
+      return __popc(shr32(m0, pl) & 3u) + __popc(shr32(m1, pl) & 3u) + __popc(shr32(m2, pl) & 3u) +
+             __popc(shr32(m3, pl) & 3u);
     };
     for (int s = 0; s < sh.h; s++)
       mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (F64 ? 0 : count(s + sh.h) << 4));
@@ -821,6 +898,7 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
       // a slot without an upper plane keeps a zero there
       static_cast<float2 *>(rv)[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
     }
+  }
   }
   __syncthreads();
   if (t < 2) {
@@ -886,19 +964,38 @@ __device__ __noinline__ inline void modes_output(const double *m, double *stress
 // The CTA's work spaces.  Formed anew at every use (hidden from the
 // compiler's view of the loop), so that no pointer holds registers across the
 // marches.
-template <typename V, bool QS>
+template <typename V, int ON>
 struct ModesSpace {
   double *w;
-  typename ModesType<V>::Mem *r, *x, *q;
+  typename ModesType<V>::Mem *r, *x, *q;  // q: in L2
+  V *p, *e;                               // p in L2; strips
   __device__ __forceinline__ explicit ModesSpace(const ModesParams &P) {
     unsigned b = blockIdx.x;
     asm volatile("" : "+r"(b));
     w = P.ws_w + (size_t)b * P.w_stride;
-    r = static_cast<typename ModesType<V>::Mem *>(P.ws_v) + (size_t)b * (QS ? 2 : 3) * P.v_stride;
+    r = static_cast<typename ModesType<V>::Mem *>(P.ws_v) + (size_t)b * (4 - ON) * P.v_stride;
     x = r + P.v_stride;
-    q = QS ? nullptr : x + P.v_stride;
+    q = ON == 2 ? nullptr : x + P.v_stride;
+    p = ON ? nullptr : reinterpret_cast<V *>(q + P.v_stride);
+    e = ON == 2 ? nullptr : static_cast<V *>(P.ws_e) + (size_t)b * P.e_stride;
   }
 };
+
+// march_residual over all strips
+template <typename V, bool CUBE, int ON, bool PER>
+__device__ __forceinline__ double2 residual_strips(const ModesSpace<V, ON> &ws) {
+  double *const e = reinterpret_cast<double *>(ws.e);
+  double2 d = march_residual<V, CUBE, ON, PER>(ws.w, ws.r, e, 0);
+  if (ON < 2)
+#pragma unroll 1
+    for (int y0 = msh().rows; y0 < msh().ney; y0 += msh().rows) {
+      __syncthreads();  // the strip below's shares
+      const double2 n = march_residual<V, CUBE, ON, PER>(ws.w, ws.r, e, y0);
+      d.x += n.x;
+      d.y += n.y;
+    }
+  return d;
+}
 
 // Norm of the right-hand side from the thread's share of its square (affine
 // conditions: of u = 0 inside, as modes_setup left w; periodic ones: of the
@@ -908,14 +1005,16 @@ struct ModesSpace {
 template <bool F64, bool PER>
 __device__ __noinline__ double rhs_norm(double n2, double *w, int ph) {
   const ModesShared &sh = msh();
-  const ModesLane<PER> T;
   double v[2] = {n2, 0.0};
-  if (T.owner)
-    for (int s = 0; s < sh.h; s++) {
-      const unsigned cv = mcnt()[s * sh.nface + T.f];
-      v[1] += sh.kd2[cv & 15u];
-      if (!F64 && s + sh.h < sh.mz) v[1] += sh.kd2[cv >> 4];
-    }
+  for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+    const ModesLane<PER> T(y0);
+    if (T.owner)
+      for (int s = 0; s < sh.h; s++) {
+        const unsigned cv = mcnt()[s * sh.nface + T.f];
+        v[1] += sh.kd2[cv & 15u];
+        if (!F64 && s + sh.h < sh.mz) v[1] += sh.kd2[cv >> 4];
+      }
+  }
   cta_sum<2>(v, ph);
   double um = 0.0;
 #pragma unroll
@@ -924,9 +1023,13 @@ __device__ __noinline__ double rhs_norm(double n2, double *w, int ph) {
                       fabs(sh.E[3 * c + 2]) * sh.len[2]);
   double rn0 = sqrt(v[0]);
   if (rn0 <= SP_RHS_FLOOR * sqrt(v[1]) * um) rn0 = 0.0;
-  if (!PER && rn0 > 0.0 && T.owner)
-    for (int c = 0; c < 3; c++)
-      for (int pl = 0; pl < sh.mz; pl++) w[c * sh.wlen + pl * sh.nface + T.f] = 0.0;
+  if (!PER && rn0 > 0.0)
+    for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
+      const ModesLane<PER> T(y0);
+      if (T.owner)
+        for (int c = 0; c < 3; c++)
+          for (int pl = 0; pl < sh.mz; pl++) w[c * sh.wlen + pl * sh.nface + T.f] = 0.0;
+    }
   __syncthreads();
   return rn0;
 }
@@ -953,11 +1056,12 @@ __device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_sol
   }
 }
 
-// V: FP32 pairs or FP64; NT threads at most, MINB CTAs per SM; CUBE: equal element edges; QS: q in
-// shared memory; PER: periodic conditions
-template <typename V, int NT, int MINB, bool CUBE, bool QS, bool PER>
+// V: FP32 pairs or FP64; NT threads at most, MINB CTAs per SM; CUBE: equal
+// element edges; ON: vectors in shared memory (ModesGeo); PER: periodic
+// conditions
+template <typename V, int NT, int MINB, bool CUBE, int ON, bool PER>
 __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
-  constexpr bool F64 = ModesType<V>::F64;
+  constexpr bool F64 = ModesType<V>::F64, QS = ON == 2;
   ModesShared &sh = msh();
   if (dynamic_smem_bytes() < sizeof(ModesShared)) return;
   int ph = 0;  // the reduction buffer in turn
@@ -969,10 +1073,10 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.rid = P.order[task / P.nrhs];
         sh.k = task % P.nrhs;
         const MeshGeo &mg = P.plans[P.rves[sh.rid].plan].geo;
-        const ModesGeo G(mg.nex, mg.ney, mg.nez, PER, F64);
-        if (dynamic_smem_bytes() < (unsigned)G.smem(QS) || G.warps() * 32 > blockDim.x ||
-            G.warps() > SP_MODES_MAX_WARPS || G.nez > (PER ? SP_MODES_MAX_NEZ - 1 : SP_MODES_MAX_NEZ) ||
-            G.nface > SP_MODES_MAX_WARPS * 32)
+        const ModesGeo G(mg.nex, mg.ney, mg.nez, PER, F64, ON);
+        if (dynamic_smem_bytes() < (unsigned)G.smem() || G.warps() * 32 > blockDim.x ||
+            G.warps() > SP_MODES_MAX_WARPS || G.rows < 1 || (PER && ON == 0) ||
+            G.nez > (PER ? SP_MODES_MAX_NEZ - 2 : SP_MODES_MAX_NEZ) || G.nface > SP_MODES_MAX_COLS)
           sh.job = 2;  // launched with less than this RVE needs
         sh.nex = G.nex;
         sh.ney = G.ney;
@@ -983,9 +1087,9 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.ntot = G.ntot;
         sh.wlen = G.wlen();
         sh.wcols = G.wcols();
-        sh.threads = 32 * G.warps();
-        sh.qoff = G.pbytes(QS);
-        sh.cntoff = G.pbytes(QS) + G.qbytes(QS);
+        sh.rows = G.rows;
+        sh.qoff = G.pbytes();
+        sh.cntoff = G.pbytes() + G.qbytes();
         sh.outer = sh.inner = 0;
       }
     }
@@ -995,16 +1099,17 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
     if (sh.job == 1) {
       // 1. tables
       {
-        const ModesSpace<V, QS> ws(P);
+        const ModesSpace<V, ON> ws(P);
         const BatchRve &rv = P.rves[sh.rid];
-        modes_setup<F64, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
-                        P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r);
+        modes_setup<ON, F64, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
+                        P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r,
+                                 ws.p);
       }
       // 2. the right-hand side's norm
       double rn0;
       {
-        const ModesSpace<V, QS> ws(P);
-        rn0 = rhs_norm<F64, PER>(march_residual<V, CUBE, QS, PER>(ws.w, ws.r).x, ws.w, ph);
+        const ModesSpace<V, ON> ws(P);
+        rn0 = rhs_norm<F64, PER>(residual_strips<V, CUBE, ON, PER>(ws).x, ws.w, ph);
         ph ^= 1;
       }
       // 3. refinement
@@ -1013,9 +1118,9 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       for (;;) {
         double v[2];
         {
-          const ModesSpace<V, QS> ws(P);
-          if (!QS && rho != 0.0) save_p<V, PER>(ws.q);
-          const double2 d = march_residual<V, CUBE, QS, PER>(ws.w, ws.r);
+          const ModesSpace<V, ON> ws(P);
+          if (ON == 1 && rho != 0.0) save_p<V, PER>(ws.q);
+          const double2 d = residual_strips<V, CUBE, ON, PER>(ws);
           v[0] = d.x;
           v[1] = d.y;
           cta_sum<2>(v, ph);
@@ -1027,24 +1132,30 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         // a reliable update: r is the true residual, the search direction
         // goes on with beta = r.z / rho of the last step
         {
-          const ModesSpace<V, QS> ws(P);
-          if (!QS) restore_p<V, PER>(ws.q, rho != 0.0);
-          update_p<V, CUBE, false, PER>(ws.r, rho != 0.0 ? v[1] / rho : 0.0);
+          const ModesSpace<V, ON> ws(P);
+          if (ON == 1) restore_p<V, PER>(ws.q, rho != 0.0);
+          update_p<V, CUBE, ON, false, PER>(ws.p, ws.r, rho != 0.0 ? v[1] / rho : 0.0);
         }
         rho = v[1];
         __syncthreads();
         int it = 0;
         while (it < P.max_inner) {
           {
-            const ModesSpace<V, QS> ws(P);
-            v[0] = march_apply<V, CUBE, QS, PER>(ws.q);
+            const ModesSpace<V, ON> ws(P);
+            v[0] = march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, 0);
+            if (ON < 2)
+#pragma unroll 1
+              for (int y0 = sh.rows; y0 < sh.ney; y0 += sh.rows) {
+                __syncthreads();  // the strip below's shares
+                v[0] += march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, y0);
+              }
           }
           double d[1] = {v[0]};
           cta_sum<1>(d, ph);
           {
-            const ModesSpace<V, QS> ws(P);
+            const ModesSpace<V, ON> ws(P);
             const double2 u =
-                update_xr<V, CUBE, QS, PER>(ws.r, ws.x, ws.q, d[0] != 0.0 ? rho / d[0] : 0.0, it == 0);
+                update_xr<V, CUBE, ON, PER>(ws.p, ws.r, ws.x, ws.q, d[0] != 0.0 ? rho / d[0] : 0.0, it == 0);
             v[0] = u.x;
             v[1] = u.y;
           }
@@ -1052,14 +1163,14 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
           it++;
           if (v[1] <= thr) break;
           {
-            const ModesSpace<V, QS> ws(P);
-            update_p<V, CUBE, QS, PER>(ws.r, rho != 0.0 ? v[0] / rho : 0.0);
+            const ModesSpace<V, ON> ws(P);
+            update_p<V, CUBE, ON, QS, PER>(ws.p, ws.r, rho != 0.0 ? v[0] / rho : 0.0);
           }
           rho = v[0];
           __syncthreads();
         }
         if (it > 0) {
-          const ModesSpace<V, QS> ws(P);
+          const ModesSpace<V, ON> ws(P);
           update_w<V, PER>(ws.x, ws.w);
         }
         outer++;
@@ -1071,7 +1182,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
       }
       // 4. averages
       {
-        const ModesSpace<V, QS> ws(P);
+        const ModesSpace<V, ON> ws(P);
         ph = march_average<PER>(ws.w, ph);
       }
       if (threadIdx.x == 0) {
@@ -1094,16 +1205,18 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
 
 using ModesFn = void (*)(ModesParams);
 
-// the instantiated classes (threads, CTAs per SM, q in shared memory): the
-// largest blocks of which 8, 3, 2 and 1 fit an SM's register file at 128
-// registers a thread, and one of 96 registers for the largest meshes
-#define SP_MODES_CLASSES(X, V) \
-  X(V, 64, 8, true) X(V, 160, 3, true) X(V, 256, 2, true) X(V, 512, 1, true) \
-  X(V, 512, 1, false) X(V, 640, 1, false)
-#define SP_MODES_EXTERN(V, NT, MINB, QS) \
-  extern template __global__ void k_modes<V, NT, MINB, true, QS, false>(ModesParams); \
-  extern template __global__ void k_modes<V, NT, MINB, false, QS, false>(ModesParams); \
-  extern template __global__ void k_modes<V, NT, MINB, true, QS, true>(ModesParams); \
-  extern template __global__ void k_modes<V, NT, MINB, false, QS, true>(ModesParams);
+// the instantiated classes (threads, CTAs per SM, vectors in shared memory):
+// the largest blocks of which 8, 3, 2 and 1 fit an SM's register file at 128
+// registers a thread; periodic conditions, which have no strips, also at 96
+// registers for meshes of more columns, affine ones without any vector in
+// shared memory
+#define SP_MODES_CLASSES(X, V, PER) \
+  X(V, 64, 8, 2, PER) X(V, 160, 3, 2, PER) X(V, 256, 2, 2, PER) X(V, 512, 1, 2, PER) \
+  X(V, 512, 1, 1, PER)
+#define SP_MODES_PERIODIC(X, V) X(V, 640, 1, 1, true)
+#define SP_MODES_AFFINE(X, V) X(V, 512, 1, 0, false)
+#define SP_MODES_EXTERN(V, NT, MINB, ON, PER) \
+  extern template __global__ void k_modes<V, NT, MINB, true, ON, PER>(ModesParams); \
+  extern template __global__ void k_modes<V, NT, MINB, false, ON, PER>(ModesParams);
 
 }  // namespace sp

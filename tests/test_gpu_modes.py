@@ -1,8 +1,9 @@
 """The element-mode batch kernel (rve_modes_kernel.cuh) at the edges of its
 range: warps whose rows start at lane 0 or straddle warps, one and two planes
-per half, odd and even plane counts, the largest meshes of each kernel class
-and the first ones past them (which keep the assembled-stencil kernel), cubic
-and box elements, all in one batch.
+per half, odd and even plane counts, the largest meshes of each kernel class,
+two and three strips of rows, 32 element layers, and the first meshes past the
+range (which keep the block-stencil kernel), cubic and box elements, all in
+one batch.
 
 Solves run to a relative residual of 1e-10; a stress error above 1e-8 of
 max|stress| (the suite's tolerance for a 1e-8 residual) is a wrong operator,
@@ -19,7 +20,8 @@ pytestmark = pytest.mark.gpu
 
 MESHES = [(2, 2, 2), (2, 3, 4), (3, 2, 5), (4, 4, 3), (8, 8, 5), (8, 4, 9), (9, 9, 4), (10, 7, 6),
           (12, 12, 3), (16, 16, 4), (16, 10, 7), (32, 3, 4), (31, 4, 3), (20, 20, 3), (13, 31, 2),
-          (25, 25, 3), (26, 25, 3), (5, 4, 31), (5, 4, 32)]
+          (25, 25, 3), (26, 25, 3), (5, 4, 31), (5, 4, 32), (5, 4, 33),
+          (31, 33, 2), (32, 32, 3), (33, 31, 2), (33, 32, 2)]
 
 
 def voxel_batch(cube, seed):
@@ -130,7 +132,7 @@ def test_parallel_launches_captured_in_a_graph():
     import torch
     rng = np.random.default_rng(8)
     descs = [mb.rve_desc(int(n), float(rng.uniform(0.1, 0.35)), (1e9, 2e10), (0.3, 0.2))
-             for n in (6, 12, 20, 24, 26, 16, 9, 6)]
+             for n in (6, 12, 20, 24, 33, 16, 9, 6)]
     b = mb.Batch(descs, threads=512, ctas_per_sm=1)
     s = torch.cuda.Stream()
     sp = C.c_void_p(s.cuda_stream)
