@@ -287,14 +287,15 @@ int sp_batch_last_launches(const sp_batch *b, int *launches);
  * as 7 load cases warm-started from that geometry's previous solution. */
 typedef struct {
   size_t hbm_budget;    /* admission budget in bytes (0: 150 GB) */
-  int max_inflight;     /* request slots solving at once (0: one per CTA) */
+  int max_inflight;     /* requests solving at once (0: as many as fit) */
   int queue_capacity;   /* request ring size (0: 65536) */
   double rtol;          /* default 1e-8 */
   double inner_rtol;    /* CG residual reduction per refinement step (default 1e-4) */
   int idle_spin_limit;  /* empty polls of the dispatcher before the loop returns (0: default
                            2,000,000); the next submit relaunches it */
   int op;               /* SP_OP_STENCIL (default) or SP_OP_ELL */
-  int ctas_per_sm;      /* request slots per SM: 1 or 2 (0: 1 for the stencil, 2 for ELL) */
+  int ctas_per_sm;      /* slots per SM: 1 or 2 (0: by the geometries' sizes for the stencil,
+                           2 for ELL) */
   double refine_rtol;   /* a request whose warm-start prediction misses rtol is solved to
                            this tighter tolerance, so that predictions from its solutions
                            meet rtol without a solve (0: rtol / 100) */

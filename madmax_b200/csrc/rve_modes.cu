@@ -47,6 +47,18 @@ static int class_room(const ModesClass &k) {
   return (std::min(SP_MODES_SM_BYTES / k.minb, SP_MODES_BLOCK_MAX + 1024) - SP_MODES_RESERVED) / 16 * 16;
 }
 
+// The vectors a CTA of `threads` threads and `room` bytes of dynamic shared
+// memory keeps there for an affine FP32 RVE (-1: none of the element-mode kernels)
+int modes_onchip(const MeshGeo &g, int threads, int room) {
+  if (g.nex < 2 || g.ney < 2 || g.nez < 2 || g.nez > SP_MODES_MAX_NEZ) return -1;
+  if ((long long)g.nex * g.ney > SP_MODES_MAX_COLS) return -1;
+  for (int on = 2; on >= 0; on--) {
+    const ModesGeo G(g.nex, g.ney, g.nez, false, false, on);
+    if (G.rows >= 1 && G.warps() * 32 <= threads && G.smem() <= room) return on;
+  }
+  return -1;
+}
+
 // An RVE runs on the smallest class whose threads hold one element column
 // each and whose shared memory holds its vectors beside the
 // class's other CTAs; it needs an interior node on every axis, at most 32
@@ -93,6 +105,7 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     }
     b.w_stride = ((size_t)3 * wlen + 15) / 16 * 16;
     b.v_stride = ((size_t)3 * ntot + 15) / 16 * 16;
+    b.v_cta = (size_t)(4 - k.on) * b.v_stride;
     // the class's largest, the same for every batch: the attribute is the
     // function's, not the launch's
     if (cudaFuncSetAttribute((const void *)b.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -111,7 +124,7 @@ int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
     b.grid = (int)std::min<long long>((long long)d->nsm * nb, (long long)b.nrve * nrhs);
     SP_TRY(dmalloc((void **)&b.d_order, ord.size() * sizeof(int), &b.bytes));
     SP_TRY(dmalloc((void **)&b.ws_w, b.grid * b.w_stride * sizeof(double), &b.bytes));
-    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * (4 - k.on) * b.v_stride * sizeof(double), &b.bytes));
+    SP_TRY(dmalloc((void **)&b.ws_v, b.grid * b.v_cta * sizeof(double), &b.bytes));
     if (k.on < 2) {
       b.e_stride = ((size_t)elen + 15) / 16 * 16;
       SP_TRY(dmalloc((void **)&b.ws_e, b.grid * b.e_stride * sizeof(double), &b.bytes));
@@ -168,16 +181,8 @@ int modes_launch(const ModesPlan &m, const ModesCommon &c, int *counters, cudaSt
     P.task_info = c.task_info;
     P.done = c.done;
     P.counter = counters + i;
-    P.ws_w = k.ws_w;
-    P.ws_v = k.ws_v;
-    P.w_stride = k.w_stride;
-    P.v_stride = k.v_stride;
-    P.ws_e = k.ws_e;
-    P.e_stride = k.e_stride;
-    P.rtol = c.rtol;
-    P.inner_rtol = c.inner_rtol;
-    P.max_outer = c.max_outer;
-    P.max_inner = c.max_inner;
+    P.buf = ModesBufs{k.ws_w, k.ws_v, k.ws_e, k.w_stride, k.v_stride, k.e_stride, k.v_cta};
+    P.lim = ModesLimits{c.rtol, c.inner_rtol, c.rtol, c.max_outer, c.max_inner};
     cudaStream_t st = i ? m.side[i - 1] : s;
     if (i) SP_CUDA_TRY(cudaStreamWaitEvent(st, m.forked, 0));
     k.fn<<<k.grid, k.threads, k.smem, st>>>(P);

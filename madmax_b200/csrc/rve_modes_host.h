@@ -15,7 +15,7 @@ struct ModesBucket {
   int *d_order = nullptr;
   double *ws_w = nullptr;
   void *ws_v = nullptr, *ws_e = nullptr;
-  size_t w_stride = 0, v_stride = 0, e_stride = 0, bytes = 0;
+  size_t w_stride = 0, v_stride = 0, e_stride = 0, v_cta = 0, bytes = 0;
 };
 
 // The launches of a batch: every bucket but the first on a side stream of its
@@ -45,6 +45,7 @@ struct ModesCommon {
 
 // The kernel class of an RVE (-1: none, the solve_rve kernel takes it)
 int modes_class(const MeshGeo &g, const double *len, bool periodic, bool f64);
+int modes_onchip(const MeshGeo &g, int threads, int room);
 // Launches for the RVEs `ids` (largest first), every one of a class >= 0
 int modes_plan(const std::vector<int> &ids, const std::vector<int> &cls,
                const std::vector<MeshGeo> &geo, int nrhs, bool periodic, bool f64, const Device *d,

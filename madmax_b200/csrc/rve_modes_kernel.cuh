@@ -18,6 +18,22 @@
 
 namespace sp {
 
+// Work spaces of a launch's CTAs
+struct ModesBufs {
+  double *ws_w;    // per CTA [3][wlen]
+  void *ws_v;      // per CTA [3][ntot] 8-byte values each of r, x, (q in L2) q, (p too) p
+  void *ws_e;      // per CTA (q in L2) shares that cross strips: 2 x [planes][nex][3] values
+  size_t w_stride, v_stride, e_stride;  // v_stride: of one of them
+  size_t v_cta;                         // ... of a CTA's
+};
+
+// When a load case's solve ends
+struct ModesLimits {
+  double rtol, inner_rtol;
+  double rtol_refine;  // target once a refinement step has run (<= rtol)
+  int max_outer, max_inner;
+};
+
 struct ModesParams {
   const BatchPlan *plans;
   const BatchRve *rves;
@@ -31,12 +47,8 @@ struct ModesParams {
   sp_solve_info *task_info;  // [nrve][nrhs]
   unsigned *done;            // [nrve] finished load cases (0 between launches)
   int *counter;
-  double *ws_w;    // per CTA [3][wlen]
-  void *ws_v;      // per CTA [3][ntot] 8-byte values each of r, x, (q in L2) q, (p too) p
-  void *ws_e;      // per CTA (q in L2) shares that cross strips: 2 x [planes][nex][3] values
-  size_t w_stride, v_stride, e_stride;  // v_stride: of one of them
-  double rtol, inner_rtol;
-  int max_outer, max_inner;
+  ModesBufs buf;
+  ModesLimits lim;
 };
 
 constexpr int SP_MODES_MAX_NEZ = 32;  // a column's materials are one 32-bit mask
@@ -108,6 +120,30 @@ struct ModesGeo {
     return (int)sizeof(ModesShared) + pbytes() + qbytes() + (h * nface + 15) / 16 * 16;
   }
 };
+
+// what the march of G reads from shared memory
+__device__ __forceinline__ void modes_sizes(const ModesGeo &G, ModesShared &sh) {
+  sh.nex = G.nex;
+  sh.ney = G.ney;
+  sh.nez = G.nez;
+  sh.nface = G.nface;
+  sh.mz = G.mz;
+  sh.h = G.h;
+  sh.ntot = G.ntot;
+  sh.wlen = G.wlen();
+  sh.wcols = G.wcols();
+  sh.rows = G.rows;
+  sh.qoff = G.pbytes();
+  sh.cntoff = G.pbytes() + G.qbytes();
+  sh.outer = sh.inner = 0;
+}
+// whether a CTA of the kernel's threads and dynamic shared memory holds it
+__device__ __forceinline__ bool modes_fit(const ModesGeo &G) {
+  return dynamic_smem_bytes() >= (unsigned)G.smem() && G.warps() * 32 <= (int)blockDim.x &&
+         G.warps() <= SP_MODES_MAX_WARPS && G.rows >= 1 && !(G.per && G.on == 0) &&
+         G.nez <= (G.per ? SP_MODES_MAX_NEZ - 2 : SP_MODES_MAX_NEZ) &&
+         G.nface <= SP_MODES_MAX_COLS;
+}
 
 extern __shared__ __align__(16) unsigned char s_modes[];
 __device__ __forceinline__ ModesShared &msh() { return *reinterpret_cast<ModesShared *>(s_modes); }
@@ -817,11 +853,19 @@ __device__ __noinline__ void restore_p(const typename ModesType<V>::Mem *qg, boo
   }
 }
 
+// p = 0 (its padding stays)
+__device__ __noinline__ inline void zero_p(float4 *p) {
+  const int n = 3 * msh().ntot;  // 8-byte values
+  for (int i = threadIdx.x; i < n / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (threadIdx.x == 0) reinterpret_cast<float2 *>(p)[n - 1] = make_float2(0.f, 0.f);
+  __syncthreads();
+}
+
 // the tables, materials and start vectors of one load case
-template <int ON, bool F64, bool PER>
+template <bool F64, bool PER>
 __device__ __noinline__ void modes_setup(const double *len, const double *mat,
                                          const uint8_t *etype, const double *eps, double *w,
-                                         void *rv, void *pg) {
+                                         void *rv) {
   ModesShared &sh = msh();
   const int t = threadIdx.x;
   const int nface = sh.nface, nex = sh.nex, wl = sh.wlen;
@@ -858,12 +902,6 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
     if (T.column && (PER || !T.owner))
       for (int c = 0; c < 3; c++)
         for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = 0.0;
-  }
-  {
-    // (3 ntot values, rounded down to 16 bytes)
-    float4 *p = ON ? mp<float4>() : static_cast<float4 *>(pg);
-    for (int i = t; i < 3 * sh.ntot / 2; i += blockDim.x) p[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (t == 0) reinterpret_cast<float2 *>(p)[3 * sh.ntot - 1] = make_float2(0.f, 0.f);
   }
   if (!PER)
     for (int i = t; i < 3 * (nex + 2); i += blockDim.x)
@@ -936,8 +974,9 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
   __syncthreads();
 }
 
-// Averages from the fibre's integrals m (march_average), by one thread: <strain> = eps, <stress> = D_0 eps + (D_1 -
-// D_0) f, f = the strain's integral over the fibre / volume.
+// Averages from the fibre's integrals m (march_average), by one thread:
+// <strain> = eps, <stress> = D_0 eps + (D_1 - D_0) f, f = the strain's integral
+// over the fibre / volume.
 __device__ __noinline__ inline void modes_output(const double *m, double *stress, double *strain) {
   const ModesShared &sh = msh();
   const double nel = (double)sh.nface * sh.nez;
@@ -969,11 +1008,11 @@ struct ModesSpace {
   double *w;
   typename ModesType<V>::Mem *r, *x, *q;  // q: in L2
   V *p, *e;                               // p in L2; strips
-  __device__ __forceinline__ explicit ModesSpace(const ModesParams &P) {
+  __device__ __forceinline__ explicit ModesSpace(const ModesBufs &P) {
     unsigned b = blockIdx.x;
     asm volatile("" : "+r"(b));
     w = P.ws_w + (size_t)b * P.w_stride;
-    r = static_cast<typename ModesType<V>::Mem *>(P.ws_v) + (size_t)b * (4 - ON) * P.v_stride;
+    r = static_cast<typename ModesType<V>::Mem *>(P.ws_v) + (size_t)b * P.v_cta;
     x = r + P.v_stride;
     q = ON == 2 ? nullptr : x + P.v_stride;
     p = ON ? nullptr : reinterpret_cast<V *>(q + P.v_stride);
@@ -1056,12 +1095,95 @@ __device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_sol
   }
 }
 
+// Refinement from the start iterate in w, as solve_rve's loop: FP64 residual,
+// CG corrections (reliable updates) in V, w += x, until the residual is at
+// most rtol rn0 -- rtol_refine rn0 once a correction has run.  Returns the
+// last relative residual; the counts are in shared memory.
+template <typename V, bool CUBE, int ON, bool PER>
+__device__ __forceinline__ double modes_refine(const ModesBufs &B, const ModesLimits &L, double rn0,
+                                               int &ph) {
+  constexpr bool QS = ON == 2;
+  ModesShared &sh = msh();
+  double rho = 0.0, relres;
+  int outer = 0;
+  for (;;) {
+    double v[2];
+    {
+      const ModesSpace<V, ON> ws(B);
+      if (ON == 1 && rho != 0.0) save_p<V, PER>(ws.q);
+      const double2 d = residual_strips<V, CUBE, ON, PER>(ws);
+      v[0] = d.x;
+      v[1] = d.y;
+      cta_sum<2>(v, ph);
+    }
+    relres = rn0 > 0.0 ? sqrt(v[0]) / rn0 : 0.0;
+    const double target = outer == 0 ? L.rtol : L.rtol_refine;
+    if (!(rn0 > 0.0 && sqrt(v[0]) > target * rn0) || outer >= L.max_outer) break;
+    const double fin = SP_FINAL_MARGIN * L.rtol_refine * rn0;
+    const double thr = fmax(L.inner_rtol * L.inner_rtol * v[0], fin * fin);
+    // a reliable update: r is the true residual, the search direction goes
+    // on with beta = r.z / rho of the last step
+    {
+      const ModesSpace<V, ON> ws(B);
+      if (ON == 1)
+        restore_p<V, PER>(ws.q, rho != 0.0);
+      else if (rho == 0.0)
+        zero_p(ON ? mp<float4>() : reinterpret_cast<float4 *>(ws.p));
+      update_p<V, CUBE, ON, false, PER>(ws.p, ws.r, rho != 0.0 ? v[1] / rho : 0.0);
+    }
+    rho = v[1];
+    __syncthreads();
+    int it = 0;
+    while (it < L.max_inner) {
+      {
+        const ModesSpace<V, ON> ws(B);
+        v[0] = march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, 0);
+        if (ON < 2)
+#pragma unroll 1
+          for (int y0 = sh.rows; y0 < sh.ney; y0 += sh.rows) {
+            __syncthreads();  // the strip below's shares
+            v[0] += march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, y0);
+          }
+      }
+      double d[1] = {v[0]};
+      cta_sum<1>(d, ph);
+      {
+        const ModesSpace<V, ON> ws(B);
+        const double2 u = update_xr<V, CUBE, ON, PER>(ws.p, ws.r, ws.x, ws.q,
+                                                      d[0] != 0.0 ? rho / d[0] : 0.0, it == 0);
+        v[0] = u.x;
+        v[1] = u.y;
+      }
+      cta_sum<2>(v, ph);
+      it++;
+      if (v[1] <= thr) break;
+      {
+        const ModesSpace<V, ON> ws(B);
+        update_p<V, CUBE, ON, QS, PER>(ws.p, ws.r, rho != 0.0 ? v[0] / rho : 0.0);
+      }
+      rho = v[0];
+      __syncthreads();
+    }
+    if (it > 0) {
+      const ModesSpace<V, ON> ws(B);
+      update_w<V, PER>(ws.x, ws.w);
+    }
+    outer++;
+    if (threadIdx.x == 0) {
+      sh.inner += it;
+      sh.outer = outer;
+    }
+    __syncthreads();
+  }
+  return relres;
+}
+
 // V: FP32 pairs or FP64; NT threads at most, MINB CTAs per SM; CUBE: equal
 // element edges; ON: vectors in shared memory (ModesGeo); PER: periodic
 // conditions
 template <typename V, int NT, int MINB, bool CUBE, int ON, bool PER>
 __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
-  constexpr bool F64 = ModesType<V>::F64, QS = ON == 2;
+  constexpr bool F64 = ModesType<V>::F64;
   ModesShared &sh = msh();
   if (dynamic_smem_bytes() < sizeof(ModesShared)) return;
   int ph = 0;  // the reduction buffer in turn
@@ -1074,23 +1196,8 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
         sh.k = task % P.nrhs;
         const MeshGeo &mg = P.plans[P.rves[sh.rid].plan].geo;
         const ModesGeo G(mg.nex, mg.ney, mg.nez, PER, F64, ON);
-        if (dynamic_smem_bytes() < (unsigned)G.smem() || G.warps() * 32 > blockDim.x ||
-            G.warps() > SP_MODES_MAX_WARPS || G.rows < 1 || (PER && ON == 0) ||
-            G.nez > (PER ? SP_MODES_MAX_NEZ - 2 : SP_MODES_MAX_NEZ) || G.nface > SP_MODES_MAX_COLS)
-          sh.job = 2;  // launched with less than this RVE needs
-        sh.nex = G.nex;
-        sh.ney = G.ney;
-        sh.nez = G.nez;
-        sh.nface = G.nface;
-        sh.mz = G.mz;
-        sh.h = G.h;
-        sh.ntot = G.ntot;
-        sh.wlen = G.wlen();
-        sh.wcols = G.wcols();
-        sh.rows = G.rows;
-        sh.qoff = G.pbytes();
-        sh.cntoff = G.pbytes() + G.qbytes();
-        sh.outer = sh.inner = 0;
+        if (!modes_fit(G)) sh.job = 2;  // launched with less than this RVE needs
+        modes_sizes(G, sh);
       }
     }
     __syncthreads();
@@ -1099,90 +1206,23 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
     if (sh.job == 1) {
       // 1. tables
       {
-        const ModesSpace<V, ON> ws(P);
+        const ModesSpace<V, ON> ws(P.buf);
         const BatchRve &rv = P.rves[sh.rid];
-        modes_setup<ON, F64, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
-                        P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r,
-                                 ws.p);
+        modes_setup<F64, PER>(rv.len, P.mats + (size_t)sh.rid * 4, P.etype + rv.etype_off,
+                              P.strains + ((size_t)sh.rid * P.nrhs + sh.k) * 6, ws.w, ws.r);
       }
       // 2. the right-hand side's norm
       double rn0;
       {
-        const ModesSpace<V, ON> ws(P);
+        const ModesSpace<V, ON> ws(P.buf);
         rn0 = rhs_norm<F64, PER>(residual_strips<V, CUBE, ON, PER>(ws).x, ws.w, ph);
         ph ^= 1;
       }
       // 3. refinement
-      double rho = 0.0;
-      int outer = 0;
-      for (;;) {
-        double v[2];
-        {
-          const ModesSpace<V, ON> ws(P);
-          if (ON == 1 && rho != 0.0) save_p<V, PER>(ws.q);
-          const double2 d = residual_strips<V, CUBE, ON, PER>(ws);
-          v[0] = d.x;
-          v[1] = d.y;
-          cta_sum<2>(v, ph);
-        }
-        relres = rn0 > 0.0 ? sqrt(v[0]) / rn0 : 0.0;
-        if (!(rn0 > 0.0 && sqrt(v[0]) > P.rtol * rn0) || outer >= P.max_outer) break;
-        const double fin = SP_FINAL_MARGIN * P.rtol * rn0;
-        const double thr = fmax(P.inner_rtol * P.inner_rtol * v[0], fin * fin);
-        // a reliable update: r is the true residual, the search direction
-        // goes on with beta = r.z / rho of the last step
-        {
-          const ModesSpace<V, ON> ws(P);
-          if (ON == 1) restore_p<V, PER>(ws.q, rho != 0.0);
-          update_p<V, CUBE, ON, false, PER>(ws.p, ws.r, rho != 0.0 ? v[1] / rho : 0.0);
-        }
-        rho = v[1];
-        __syncthreads();
-        int it = 0;
-        while (it < P.max_inner) {
-          {
-            const ModesSpace<V, ON> ws(P);
-            v[0] = march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, 0);
-            if (ON < 2)
-#pragma unroll 1
-              for (int y0 = sh.rows; y0 < sh.ney; y0 += sh.rows) {
-                __syncthreads();  // the strip below's shares
-                v[0] += march_apply<V, CUBE, ON, PER>(ws.q, ws.p, ws.e, y0);
-              }
-          }
-          double d[1] = {v[0]};
-          cta_sum<1>(d, ph);
-          {
-            const ModesSpace<V, ON> ws(P);
-            const double2 u =
-                update_xr<V, CUBE, ON, PER>(ws.p, ws.r, ws.x, ws.q, d[0] != 0.0 ? rho / d[0] : 0.0, it == 0);
-            v[0] = u.x;
-            v[1] = u.y;
-          }
-          cta_sum<2>(v, ph);
-          it++;
-          if (v[1] <= thr) break;
-          {
-            const ModesSpace<V, ON> ws(P);
-            update_p<V, CUBE, ON, QS, PER>(ws.p, ws.r, rho != 0.0 ? v[0] / rho : 0.0);
-          }
-          rho = v[0];
-          __syncthreads();
-        }
-        if (it > 0) {
-          const ModesSpace<V, ON> ws(P);
-          update_w<V, PER>(ws.x, ws.w);
-        }
-        outer++;
-        if (threadIdx.x == 0) {
-          sh.inner += it;
-          sh.outer = outer;
-        }
-        __syncthreads();
-      }
+      relres = modes_refine<V, CUBE, ON, PER>(P.buf, P.lim, rn0, ph);
       // 4. averages
       {
-        const ModesSpace<V, ON> ws(P);
+        const ModesSpace<V, ON> ws(P.buf);
         ph = march_average<PER>(ws.w, ph);
       }
       if (threadIdx.x == 0) {
@@ -1193,7 +1233,7 @@ __global__ void __launch_bounds__(NT, MINB) k_modes(ModesParams P) {
     if (threadIdx.x == 0) {
       sp_solve_info in = {};
       in.relres = relres;
-      in.status = sh.job != 1 ? SP_ERR_STATE : (relres <= P.rtol ? SP_OK : SP_ERR_NOCONV);
+      in.status = sh.job != 1 ? SP_ERR_STATE : (relres <= P.lim.rtol ? SP_OK : SP_ERR_NOCONV);
       in.outer_its = sh.outer;
       in.inner_its = sh.inner;
       modes_report(in, P.task_info + (size_t)sh.rid * P.nrhs, sh.k, P.nrhs, P.done + sh.rid,

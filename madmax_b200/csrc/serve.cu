@@ -35,60 +35,12 @@
 #include <map>
 #include <vector>
 
+#include "rve_modes_host.h"
 #include "rve_solve.cuh"
+#include "serve_internal.h"
 #include "sp_cuda.h"
 
 namespace sp {
-
-constexpr int SERVE_NT = 512;
-constexpr int SERVE_K = 7;  // eps and eps + delta e_i, i = 0..5 (component-major vectors need no padding)
-constexpr int SERVE_NRHS = 7;
-constexpr double FD_DELTA = 0.005;  // micro/inc/micro.h:29
-
-struct ServeGeom {
-  MeshGeo g;
-  const int *cols;
-  const int *nbr;
-  float *vals;  // node-sliced ELL values [nn_pad*243] (assembled operator only)
-  float *dinv;  // component-major [3][nn_pad]
-  const uint8_t *etype;
-  double *Ke;   // [2][576]
-  double *D;    // [72]
-  double *Bbar; // [144]
-  double *warm;     // [SERVE_K][3][nn_pad] solutions of the previous request
-  double *warm_eps; // [SERVE_K][6] its load-case strains
-  double *gram;     // [6][6] b_i . b_j of the unit-strain right-hand sides b_i = -K u_bc(e_i)
-  const int *color_elems;
-  const uint8_t *slot;
-  int color_off[9];
-  int has_warm;
-};
-
-struct ServeReq {
-  int geom, pad;
-  double strain[6];
-};
-
-struct ServeRes {
-  double stress[6];
-  double tangent[36];
-  sp_solve_info info;
-  volatile long long done; // ticket + 1 once the result is valid
-};
-
-struct ServeCtl { // mapped host memory
-  volatile long long tail;
-  volatile int stop;
-  int pad;
-};
-
-struct ServeDev { // device memory
-  unsigned long long claim;
-  volatile long long dtail;
-  volatile int dstop;
-  volatile int dispatcher_gone;
-  int err;
-};
 
 struct ServeParams {
   ServeGeom *geoms;
@@ -455,11 +407,49 @@ static double now_s() {
   return ts.tv_sec + 1e-9 * ts.tv_nsec;
 }
 
+// one store of a geometry's solutions and strains, in doubles
+static size_t store_len(const ModesGeo &G) { return (size_t)SERVE_NRHS * (3 * G.wlen() + 6); }
+
+// The class of the element-mode loop a server runs (-1: the block-stencil or
+// assembled loop of this file): the stencil operator with the slots per SM left
+// open, or one asked for (the last class), and every geometry in the range.
+// Measured: a burst of 96 requests on geometries of n = 8..32, 250 ms in the
+// block-stencil loop, 62 ms in the last class (a CTA per load case instead of
+// one per request, vectors on chip); a step of 512 points with n = 12 RVEs
+// 49.8 ms of micro solves there, 53.0 ms in the last class, whose 16 warps are a
+// third full, and 37.8 ms in the class of 160 threads, three to an SM.
+static int serve_class(int ngeom, const sp_rve_desc *descs, const sp_server_opts &o) {
+  if (o.op != SP_OP_STENCIL || o.ctas_per_sm < 0 || o.ctas_per_sm > 1) return -1;
+  for (int c = o.ctas_per_sm == 1 ? SERVE_CLASSES - 1 : 0; c < SERVE_CLASSES; c++) {
+    const ServeClass &k = kServeClasses[c];
+    bool all = true;
+    for (int i = 0; i < ngeom && all; i++) {
+      const MeshGeo g = make_geo(descs[i].n, descs[i].len);
+      all = modes_onchip(g, k.threads, k.dyn()) >= (c == SERVE_CLASSES - 1 ? 0 : 2);
+    }
+    if (all) return c;
+  }
+  return -1;
+}
+
+// strides of the element-mode loop's work spaces (doubles and 8-byte values)
+static void modes_strides(const sp_rve_desc &d, size_t *w, size_t *v, size_t *e) {
+  const ModesGeo G(d.n[0], d.n[1], d.n[2], false, false, 0);
+  auto up = [](size_t x) { return (x + 15) / 16 * 16; };
+  *w = std::max(*w, up((size_t)3 * G.wlen()));
+  *v = std::max(*v, up((size_t)3 * G.ntot));
+  *e = std::max(*e, up((size_t)6 * G.mz * G.nex));
+}
+
 // device bytes a resident geometry holds (the assembled operator adds its
 // node-sliced FP32 values)
-static size_t geom_bytes(const sp_rve_desc &d, int op) {
+static size_t geom_bytes(const sp_rve_desc &d, int op, bool modes) {
   size_t nn = (size_t)(d.n[0] + 1) * (d.n[1] + 1) * (d.n[2] + 1), np = (nn + 31) / 32 * 32;
   size_t nelm = (size_t)d.n[0] * d.n[1] * d.n[2];
+  if (modes) {
+    const ModesGeo G(d.n[0], d.n[1], d.n[2], false, false, 0);
+    return 3 * np * 4 + nelm + (2 * SP_KE + 72 + 144 + 36) * 8 + store_len(G) * 16 + 1024;
+  }
   return (op == SP_OP_ELL ? np * 243 * 4 : 0) + 3 * np * 4 + nelm +
          (2 * SP_KE + 72 + 144) * 8 + (SERVE_K * (3 * np + 6) + 36) * 8 + 1024;
 }
@@ -487,6 +477,11 @@ struct sp_server_s {
   long long tail = 0, head_done = 0;
   cudaStream_t stream = nullptr;
   ServeParams P;
+  bool modes = false;    // the element-mode loop, of class cls
+  int cls = -1;
+  ServeJob *d_jobs = nullptr;
+  void *ws_m[3] = {nullptr, nullptr, nullptr};  // its work spaces
+  ServeModes M;
 };
 
 static int server_grid(sp_server *s, Device *d);
@@ -517,17 +512,22 @@ extern "C" void sp_server_opts_default(sp_server_opts *o) {
   o->warm_start = SP_WARM_PREDICT;
 }
 
+// `cls`: the element-mode class (in: the one to lay out; out: -1 where its two
+// stores a geometry do not fit a budget that the block-stencil loop fits)
 static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_opts *o, int nsm,
-                         int *slots, size_t *total, size_t *per_slot) {
-  size_t resident = 0;
+                         int *cls, int *slots, size_t *total) {
+  size_t resident = 0, mw = 0, mv = 0, me = 0;
+  for (int i = 0; i < ngeom; i++)
+    for (int k = 0; k < 3; k++)
+      if (descs[i].n[k] < 1 || descs[i].len[k] <= 0)
+        return sp_set_error(SP_ERR_ARG, "geometry %d: bad mesh", i);
+  const bool modes = *cls >= 0;
   std::map<std::vector<int>, int> seen;
   int maxnp = 0;
   for (int i = 0; i < ngeom; i++) {
     const sp_rve_desc &d = descs[i];
-    for (int k = 0; k < 3; k++)
-      if (d.n[k] < 1 || d.len[k] <= 0)
-        return sp_set_error(SP_ERR_ARG, "geometry %d: bad mesh", i);
-    resident += geom_bytes(d, o->op);
+    if (modes) modes_strides(d, &mw, &mv, &me);
+    resident += geom_bytes(d, o->op, modes);
     std::vector<int> key(d.n, d.n + 3);
     if (!seen.count(key)) {
       seen[key] = 1;
@@ -535,11 +535,19 @@ static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_op
     }
     maxnp = std::max(maxnp, ((d.n[0] + 1) * (d.n[1] + 1) * (d.n[2] + 1) + 31) / 32 * 32);
   }
-  size_t slot = (size_t)SERVE_K * 3 * maxnp * (8 + 4 * 4);
-  const int per_sm = o->ctas_per_sm ? o->ctas_per_sm : (o->op == SP_OP_STENCIL ? 1 : 2);
+  const size_t slot = modes ? 8 * (mw + 4 * mv + me) : (size_t)SERVE_K * 3 * maxnp * (8 + 4 * 4);
+  const int per_sm = modes            ? kServeClasses[*cls].ctas
+                     : o->ctas_per_sm ? o->ctas_per_sm
+                                      : (o->op == SP_OP_STENCIL ? 1 : 2);
   int want = nsm * per_sm - 1;
-  if (o->max_inflight > 0 && o->max_inflight < want) want = o->max_inflight;
+  // a slot solves a request, or one of its load cases
+  const long long inflight = (long long)o->max_inflight * (modes ? SERVE_NRHS : 1);
+  if (inflight > 0 && inflight < want) want = (int)inflight;
   size_t budget = o->hbm_budget ? o->hbm_budget : (size_t)150e9;
+  if (modes && resident + 2 * slot > budget) {
+    *cls = -1;
+    return server_layout(ngeom, descs, o, nsm, cls, slots, total);
+  }
   if (resident + slot > budget)
     return sp_set_error(SP_ERR_BUDGET, "geometries need %zu bytes, budget %zu", resident + slot,
                         budget);
@@ -547,7 +555,6 @@ static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_op
   size_t fit = (budget - resident) / slot;
   if ((size_t)want > fit) want = (int)fit;
   *slots = want;
-  *per_slot = slot;
   *total = resident + (size_t)(want + 1) * slot;
   return SP_OK;
 }
@@ -557,9 +564,8 @@ extern "C" int sp_server_plan_bytes(int ngeom, const sp_rve_desc *descs, const s
   if (ngeom < 1 || !descs || !bytes) return sp_set_error(SP_ERR_ARG, "bad argument");
   sp_server_opts o;
   if (opts) o = *opts; else sp_server_opts_default(&o);
-  int slots;
-  size_t per;
-  return server_layout(ngeom, descs, &o, 148, &slots, bytes, &per);
+  int slots, cls = serve_class(ngeom, descs, o);
+  return server_layout(ngeom, descs, &o, 148, &cls, &slots, bytes);
 }
 
 extern "C" int sp_server_destroy(sp_server *s) {
@@ -571,6 +577,8 @@ extern "C" int sp_server_destroy(sp_server *s) {
   cudaFree(s->d_dev);
   cudaFree(s->ws_u);
   cudaFree(s->ws_v);
+  cudaFree(s->d_jobs);
+  for (void *p : s->ws_m) cudaFree(p);
   if (s->h_req) cudaFreeHost(s->h_req);
   if (s->h_res) cudaFreeHost(s->h_res);
   if (s->h_ctl) cudaFreeHost(s->h_ctl);
@@ -595,6 +603,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
     return sp_set_error(SP_ERR_ARG, "sp_server_create: unknown operator");
   if (o.warm_start != SP_WARM_PREDICT && o.warm_start != SP_WARM_LAST)
     return sp_set_error(SP_ERR_ARG, "sp_server_create: unknown warm start");
+  int cls = serve_class(ngeom, descs, o);
   // the stencil solve of 7 load cases wants 128 registers (1 slot per SM)
   if (o.ctas_per_sm == 0) o.ctas_per_sm = (o.op == SP_OP_STENCIL) ? 1 : 2;
   if (o.ctas_per_sm != 1 && o.ctas_per_sm != 2)
@@ -602,8 +611,8 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   Device *d;
   SP_TRY(device(&d));
   int slots;
-  size_t total, per_slot;
-  SP_TRY(server_layout(ngeom, descs, &o, d->nsm, &slots, &total, &per_slot));
+  size_t total;
+  SP_TRY(server_layout(ngeom, descs, &o, d->nsm, &cls, &slots, &total));
   if (slots < 1) return sp_set_error(SP_ERR_BUDGET, "budget leaves no request slot");
   sp_server *s = new sp_server_s();
   s->ngeom = ngeom;
@@ -611,6 +620,9 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   s->dev = d->id;
   s->cap = o.queue_capacity;
   s->grid = slots + 1; // + dispatcher
+  s->cls = cls;
+  s->modes = s->cls >= 0;
+  size_t mw = 0, mv = 0, me = 0;
   int rc = server_grid(s, d);
   std::map<std::vector<int>, DevPlan *> pm;
   std::vector<double> mats((size_t)ngeom * 4);
@@ -642,6 +654,11 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
     void *b[7] = {};
     size_t sz[7] = {o.op == SP_OP_ELL ? np * 243 * 4 : 0, 3 * np * 4, ne + 16, 2 * SP_KE * 8,
                     72 * 8, 144 * 8, (SERVE_K * (3 * np + 6) + 36) * 8};
+    const ModesGeo mg(dd.n[0], dd.n[1], dd.n[2], false, false, 0);
+    if (s->modes) {
+      modes_strides(dd, &mw, &mv, &me);
+      sz[6] = (2 * store_len(mg) + 36) * 8;
+    }
     for (int k = 0; k < 7 && !rc; k++) {
       if (!sz[k]) continue;
       rc = dmalloc(&b[k], sz[k], &s->bytes);
@@ -654,9 +671,22 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
     G.Ke = (double *)b[3];
     G.D = (double *)b[4];
     G.Bbar = (double *)b[5];
-    G.warm = (double *)b[6];
-    G.warm_eps = G.warm + (size_t)SERVE_K * 3 * np;
-    G.gram = G.warm_eps + SERVE_K * 6;
+    if (s->modes) {
+      G.store = (double *)b[6];
+      G.gram = G.store + 2 * store_len(mg);
+      G.wlen = mg.wlen();
+      G.on = modes_onchip(G.g, kServeClasses[s->cls].threads, kServeClasses[s->cls].dyn());
+      G.cube = G.g.hx == G.g.hy && G.g.hx == G.g.hz;
+      for (int k = 0; k < 3; k++) G.len[k] = dd.len[k];
+      for (int k = 0; k < 2; k++) {
+        G.mats[2 * k] = dd.E[k];
+        G.mats[2 * k + 1] = dd.nu[k];
+      }
+    } else {
+      G.warm = (double *)b[6];
+      G.warm_eps = G.warm + (size_t)SERVE_K * 3 * np;
+      G.gram = G.warm_eps + SERVE_K * 6;
+    }
     std::vector<uint8_t> et(ne);
     rc = sp_classify_elements(&dd, et.data(), nullptr);
     if (!rc && cudaMemcpy((void *)G.etype, et.data(), ne, cudaMemcpyHostToDevice))
@@ -677,8 +707,13 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
     rc = dmalloc((void **)&d_scr, (size_t)nasm * (rm_stride + drm_stride) * 4, nullptr);
   if (!rc) rc = dmalloc((void **)&s->d_req, (size_t)s->cap * sizeof(ServeReq), &s->bytes);
   if (!rc) rc = dmalloc((void **)&s->d_dev, sizeof(ServeDev), &s->bytes);
-  if (!rc) rc = dmalloc((void **)&s->ws_u, (size_t)s->grid * s->stride * 8, &s->bytes);
-  if (!rc) rc = dmalloc((void **)&s->ws_v, (size_t)s->grid * 4 * s->stride * 4, &s->bytes);
+  if (!rc && !s->modes) rc = dmalloc((void **)&s->ws_u, (size_t)s->grid * s->stride * 8, &s->bytes);
+  if (!rc && !s->modes) rc = dmalloc((void **)&s->ws_v, (size_t)s->grid * 4 * s->stride * 4, &s->bytes);
+  if (!rc && s->modes) {
+    const size_t sz[3] = {mw, 4 * mv, me};
+    for (int k = 0; k < 3 && !rc; k++) rc = dmalloc(&s->ws_m[k], s->grid * sz[k] * 8, &s->bytes);
+    if (!rc) rc = dmalloc((void **)&s->d_jobs, (size_t)s->cap * sizeof(ServeJob), &s->bytes);
+  }
   if (!rc && (cudaHostAlloc((void **)&s->h_req, (size_t)s->cap * sizeof(ServeReq), cudaHostAllocMapped) ||
               cudaHostAlloc((void **)&s->h_res, (size_t)s->cap * sizeof(ServeRes), cudaHostAllocMapped) ||
               cudaHostAlloc((void **)&s->h_ctl, sizeof(ServeCtl), cudaHostAllocMapped)))
@@ -745,6 +780,28 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   P.max_inner = 4000;
   P.idle_limit = o.idle_spin_limit;
   P.warm_last = o.warm_start == SP_WARM_LAST;
+  if (s->modes) {
+    ServeModes &M = s->M;
+    M.geoms = s->d_geoms;
+    M.ngeom = ngeom;
+    M.cap = s->cap;
+    M.hreq = s->d_req_map;
+    M.dreq = s->d_req;
+    M.jobs = s->d_jobs;
+    M.res = s->d_res_map;
+    M.ctl = s->d_ctl_map;
+    M.dev = s->d_dev;
+    M.buf = ModesBufs{(double *)s->ws_m[0], s->ws_m[1], s->ws_m[2], mw, mv, me,
+                      4 * mv};
+    // a request whose prediction misses rtol is solved tighter, so that the
+    // predictions from its solutions meet rtol without a solve (a start from
+    // the last solutions is solved to rtol)
+    M.lim = ModesLimits{o.rtol, o.inner_rtol, P.warm_last ? o.rtol : o.refine_rtol, P.max_outer,
+                        P.max_inner};
+    M.idle_limit = o.idle_spin_limit;
+    M.warm_last = P.warm_last;
+    M.dyn = kServeClasses[s->cls].dyn();
+  }
   *out = s;
   return SP_OK;
 }
@@ -753,6 +810,15 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
 // dispatcher's counter): the grid never exceeds what the SMs hold.
 static int server_grid(sp_server *s, Device *d) {
   int occ = 0;
+  if (s->modes) {
+    const ServeClass &k = kServeClasses[s->cls];
+    SP_CUDA_TRY(cudaFuncSetAttribute((const void *)k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     k.dyn()));
+    SP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, k.threads, k.dyn()));
+    if (occ < 1) return sp_set_error(SP_ERR_CUDA, "serving kernel does not fit an SM");
+    if (s->grid > d->nsm * occ) s->grid = d->nsm * occ;
+    return SP_OK;
+  }
   const int dyn = serve_dyn_smem(s->o);
   if (dyn)
     SP_CUDA_TRY(cudaFuncSetAttribute((const void *)serve_kernel(s->o),
@@ -772,7 +838,10 @@ static int server_launch(sp_server *s) {
   z.dispatcher_gone = 0;
   SP_CUDA_TRY(cudaMemcpyAsync(s->d_dev, &z, sizeof(z), cudaMemcpyHostToDevice, s->stream));
   SP_CUDA_TRY(cudaStreamSynchronize(s->stream));
-  serve_kernel(s->o)<<<s->grid, SERVE_NT, serve_dyn_smem(s->o), s->stream>>>(s->P);
+  if (s->modes)
+    kServeClasses[s->cls].fn<<<s->grid, kServeClasses[s->cls].threads, s->M.dyn, s->stream>>>(s->M);
+  else
+    serve_kernel(s->o)<<<s->grid, SERVE_NT, serve_dyn_smem(s->o), s->stream>>>(s->P);
   SP_CUDA_TRY(cudaGetLastError());
   s->running = 1;
   s->launches++;
@@ -796,7 +865,7 @@ static int server_keepalive(sp_server *s) {
   if (s->h_ctl->stop) return SP_OK;
   ServeDev z;
   SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
-  if ((long long)z.claim < s->tail) return server_launch(s);
+  if ((long long)z.claim < s->tail * (s->modes ? SERVE_NRHS : 1)) return server_launch(s);
   return SP_OK;
 }
 
@@ -870,7 +939,7 @@ extern "C" int sp_server_stop(sp_server *s) {
   // requests published after the loop saw stop: run them to completion
   ServeDev z;
   SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
-  if ((long long)z.claim < s->tail) {
+  if ((long long)z.claim < s->tail * (s->modes ? SERVE_NRHS : 1)) {
     s->h_ctl->stop = 0;
     SP_TRY(server_launch(s));
     s->h_ctl->stop = 1;

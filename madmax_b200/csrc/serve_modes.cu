@@ -1,0 +1,293 @@
+// serve_modes.cu -- the element-mode request loop: serve.cu's loop with a CTA
+// per load case of a request instead of one per request.
+//
+// A request's 7 load cases (eps and eps + delta e_i, micro/src/
+// homogenize.c:59-94) are tasks of their own, claimed in order by the worker
+// CTAs; the last one to finish forms the tangent, writes the result and
+// raises the done flag.  A task runs the solve of rve_modes_kernel.cuh, whose
+// vectors stay on chip where they fit, started from the geometry's store of
+// the last solved request's fluctuations.
+//
+// Stores.  A geometry has two: the published one and the one being written.
+// A request takes the geometry's lock when its first load case is claimed;
+// without it, it stores nothing.  Its solutions go to the other store and are
+// published (gen + 1) once all 7 are there.  A task that read the published
+// store while a later request's solutions replaced it (gen has moved on)
+// starts cold instead, so no task starts from a mixture of two requests.
+// Nothing waits: a lock that is taken is passed by.
+//
+// What bounds it: a task's set-up and its two residual passes where the
+// prediction holds, the march of the corrections where it does not (the rate
+// of k_modes).  Several CTAs per SM hide the set-up's loads (the classes of
+// serve_internal.h); a task's time is a seventh of a request's, so a burst
+// ends without a long last request.
+#include "serve_internal.h"
+
+namespace sp {
+
+struct ServeShared {
+  long long req;  // ticket, -1: leave
+  int geom, k, gen, stored;
+  double eps[SERVE_NRHS][6];
+  double c[6];  // prediction coefficients
+  double rn0;
+};
+
+// claim the next load case (bounded wait, as in serve.cu); one thread
+__device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
+  ServeDev *D = P.dev;
+  long long task = -1, idle = 0;
+  for (;;) {
+    const unsigned long long h = *(volatile unsigned long long *)&D->claim;
+    const long long end = D->dtail * SERVE_NRHS;
+    if ((long long)h < end) {
+      if (atomicCAS(&D->claim, h, h + 1) == h) {
+        task = (long long)h;
+        break;
+      }
+      continue;
+    }
+    if (D->dstop || D->dispatcher_gone || ++idle > 8LL * P.idle_limit) break;
+    __nanosleep(500);
+  }
+  __threadfence();
+  S.req = task < 0 ? -1 : task / SERVE_NRHS;
+  if (task < 0) return;
+  S.k = (int)(task % SERVE_NRHS);
+  const ServeReq *rq = P.dreq + S.req % P.cap;
+  const int gid = __ldcg(&rq->geom);
+  S.geom = gid;
+  double e0[6];
+  for (int j = 0; j < 6; j++) e0[j] = __ldcg(&rq->strain[j]);
+  for (int c = 0; c < SERVE_NRHS; c++)
+    for (int j = 0; j < 6; j++) S.eps[c][j] = e0[j] + (c == j + 1 ? FD_DELTA : 0.0);
+  if (gid < 0 || gid >= P.ngeom) return;
+  ServeGeom &G = P.geoms[gid];
+  if (S.k == 0)
+    atomicExch(&P.jobs[S.req % P.cap].writer, atomicCAS(&G.lock, 0u, 1u) == 0u ? 1u : 2u);
+  S.gen = (int)atomicAdd(&G.gen, 0u);
+  __threadfence();
+  const double *e = S.eps[S.k];
+  double s = 0.0;
+  for (int a = 0; a < 6; a++)
+    for (int b = 0; b < 6; b++) s += e[a] * __ldg(G.gram + a * 6 + b) * e[b];
+  S.rn0 = sqrt(fmax(s, 0.0));
+  if (S.gen) {
+    const double *se = G.store + (size_t)(S.gen & 1) * SERVE_NRHS * (3 * G.wlen + 6) +
+                       (size_t)SERVE_NRHS * 3 * G.wlen;
+    for (int j = 0; j < 6; j++) {
+      const double b = __ldcg(se + j), d = __ldcg(se + (j + 1) * 6 + j) - b;
+      S.c[j] = d != 0.0 ? (e[j] - b) / d : 0.0;
+    }
+  }
+}
+
+// the start iterate: the fluctuation of the last solution of this load case
+// (last), or predicted to first order from the 7 of the last solved request,
+// or (cold) none.  modes_setup left w = -eps.x inside, which stays for a load
+// case without a right-hand side.
+__device__ __noinline__ void serve_start(const ServeGeom &G, ServeShared &S, bool last, double *w) {
+  if (!(S.rn0 > 0.0)) return;
+  const int n = 3 * G.wlen, t = threadIdx.x;
+  const double *st = G.store + (size_t)(S.gen & 1) * SERVE_NRHS * (n + 6);
+  if (S.gen && last) {
+    for (int i = t; i < n; i += blockDim.x) w[i] = __ldcg(st + (size_t)S.k * n + i);
+  } else if (S.gen) {
+    double c[6];
+#pragma unroll
+    for (int j = 0; j < 6; j++) c[j] = S.c[j];
+    for (int i = t; i < n; i += blockDim.x) {
+      const double w0 = __ldcg(st + i);
+      double v[6];
+#pragma unroll
+      for (int j = 0; j < 6; j++) v[j] = __ldcg(st + (size_t)(j + 1) * n + i);
+      double s = w0;
+#pragma unroll
+      for (int j = 0; j < 6; j++) s = fma(c[j], v[j] - w0, s);
+      w[i] = s;
+    }
+  }
+  __syncthreads();
+  if (S.gen) {
+    if (t == 0) {
+      __threadfence();
+      if ((int)atomicAdd(const_cast<unsigned *>(&G.gen), 0u) != S.gen) S.gen = 0;
+    }
+    __syncthreads();
+  }
+  if (!S.gen)
+    for (int i = t; i < n; i += blockDim.x) w[i] = 0.0;
+  __syncthreads();
+}
+
+// one load case; thread 0 writes its stress average
+template <bool CUBE, int ON>
+__device__ __noinline__ double serve_case(const ServeModes &P, const ServeGeom &G, ServeShared &S,
+                                          double *stress) {
+  ModesShared &sh = msh();
+  if (threadIdx.x == 0) {
+    const ModesGeo M(G.g.nex, G.g.ney, G.g.nez, false, false, ON);
+    modes_sizes(M, sh);
+  }
+  __syncthreads();
+  int ph = 0;
+  {
+    const ModesSpace<F2, ON> ws(P.buf);
+    modes_setup<false, false>(G.len, G.mats, G.etype, S.eps[S.k], ws.w, ws.r);
+    serve_start(G, S, P.warm_last, ws.w);
+  }
+  const double relres = modes_refine<F2, CUBE, ON, false>(P.buf, P.lim, S.rn0, ph);
+  {
+    const ModesSpace<F2, ON> ws(P.buf);
+    march_average<false>(ws.w, ph);
+  }
+  if (threadIdx.x == 0) modes_output(sh.red, stress, nullptr);
+  return relres;
+}
+
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant__ ServeModes P) {
+  __shared__ ServeShared S;
+  const int t = threadIdx.x;
+  ServeDev *D = P.dev;
+  if (blockIdx.x == 0) {
+    // dispatcher: forward host requests into the device ring
+    if (t >= 32) return;
+    long long seen = D->dtail;
+    int idle = 0;
+    for (;;) {
+      long long ht = 0;
+      int hstop = 0;
+      if (t == 0) {
+        ht = P.ctl->tail;
+        hstop = P.ctl->stop;
+      }
+      ht = __shfl_sync(0xffffffffu, ht, 0);
+      hstop = __shfl_sync(0xffffffffu, hstop, 0);
+      __threadfence_system();
+      if (ht > seen) {
+        for (long long i = seen + t; i < ht; i += 32) {
+          const volatile ServeReq *src = P.hreq + (i % P.cap);
+          ServeReq *dst = P.dreq + (i % P.cap);
+          dst->geom = src->geom;
+          for (int k = 0; k < 6; k++) dst->strain[k] = src->strain[k];
+          ServeJob &J = P.jobs[i % P.cap];
+          J.left = SERVE_NRHS;
+          J.stored = J.writer = 0;
+          J.status = J.outer = J.inner = 0;
+          J.relres = 0;
+        }
+        __threadfence();
+        __syncwarp();
+        if (t == 0) D->dtail = ht;
+        seen = ht;
+        idle = 0;
+      } else if (hstop) {
+        if (t == 0) D->dstop = 1;
+        break;
+      } else if (++idle > P.idle_limit) {
+        break;
+      }
+      __nanosleep(1000);
+    }
+    if (t == 0) {
+      __threadfence();
+      D->dispatcher_gone = 1;
+    }
+    return;
+  }
+  if (dynamic_smem_bytes() < (unsigned)P.dyn) return;  // (the host's waits are bounded)
+  for (;;) {
+    if (t == 0) serve_claim(P, S);
+    __syncthreads();
+    if (S.req < 0) break;
+    ServeJob &J = P.jobs[S.req % P.cap];
+    const bool known = S.geom >= 0 && S.geom < P.ngeom;
+    double relres = 0.0;
+    if (known) {
+      ServeGeom &G = P.geoms[S.geom];
+      double *const stress = J.stress[S.k];
+      switch (2 * G.on + (G.cube ? 1 : 0)) {
+        case 5: relres = serve_case<true, 2>(P, G, S, stress); break;
+        case 4: relres = serve_case<false, 2>(P, G, S, stress); break;
+        default:
+          if constexpr (MINB == 1) {  // only the last class serves these
+            switch (2 * G.on + (G.cube ? 1 : 0)) {
+              case 3: relres = serve_case<true, 1>(P, G, S, stress); break;
+              case 2: relres = serve_case<false, 1>(P, G, S, stress); break;
+              case 1: relres = serve_case<true, 0>(P, G, S, stress); break;
+              default: relres = serve_case<false, 0>(P, G, S, stress); break;
+            }
+          }
+      }
+      // keep this load case's solution for the geometry's next requests when
+      // it was solved (it then meets the refined tolerance); one accepted on
+      // its prediction leaves the solved state in place, so predictions do
+      // not drift from it
+      if (t == 0)
+        S.stored = (msh().outer > 0 || !(S.rn0 > 0.0) || S.gen == 0 || P.warm_last) &&
+                   atomicAdd(&J.writer, 0u) == 1u;
+      if (t == 0) __threadfence();
+      __syncthreads();
+      if (S.stored) {
+        const int n = 3 * G.wlen;
+        double *st = G.store + (size_t)((atomicAdd(&G.gen, 0u) + 1) & 1) * SERVE_NRHS * (n + 6);
+        const double *w = P.buf.ws_w + (size_t)blockIdx.x * P.buf.w_stride;
+        for (int i = t; i < n; i += blockDim.x) __stcg(st + (size_t)S.k * n + i, w[i]);
+        if (t < 6) __stcg(st + (size_t)SERVE_NRHS * n + S.k * 6 + t, S.eps[S.k][t]);
+      }
+      __threadfence();
+      __syncthreads();
+    }
+    if (t == 0) {
+      if (known) {
+        const int status = relres <= P.lim.rtol ? SP_OK : SP_ERR_NOCONV;
+        atomicMax(&J.status, status);
+        atomicMax(&J.outer, msh().outer);
+        atomicMax(&J.inner, msh().inner);
+        atomicMax(&J.relres, (unsigned long long)__double_as_longlong(fmax(relres, 0.0)));
+        if (S.stored) atomicAdd(&J.stored, 1u);
+      } else {
+        atomicMax(&J.status, SP_ERR_RANGE);
+      }
+      __threadfence();
+      if (atomicSub(&J.left, 1u) == 1u) {
+        __threadfence();
+        ServeRes *out = P.res + (S.req % P.cap);
+        if (known) {
+          ServeGeom &G = P.geoms[S.geom];
+          const volatile double(*st)[6] = J.stress;
+          for (int v = 0; v < 6; v++) out->stress[v] = st[0][v];
+          // c_tangent[j*6 + i] = (stress(eps + d e_i)_j - stress(eps)_j) / (d e_i)
+          // (micro/src/homogenize.c:79-80)
+          for (int i = 0; i < 6; i++)
+            for (int j = 0; j < 6; j++)
+              out->tangent[j * 6 + i] = (st[i + 1][j] - st[0][j]) / (S.eps[i + 1][i] - S.eps[0][i]);
+          if (atomicAdd(&J.writer, 0u) == 1u) {
+            if (atomicAdd(&J.stored, 0u) == SERVE_NRHS) atomicAdd(&G.gen, 1u);
+            __threadfence();
+            atomicExch(&G.lock, 0u);
+          }
+        }
+        sp_solve_info in = {};
+        in.status = atomicAdd(&J.status, 0);
+        in.outer_its = atomicAdd(&J.outer, 0);
+        in.inner_its = atomicAdd(&J.inner, 0);
+        in.relres = __longlong_as_double((long long)atomicAdd(&J.relres, 0ull));
+        out->info = in;
+        __threadfence_system();
+        out->done = S.req + 1;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// 128 registers a thread at every class; the shared memory of a CTA is the
+// SM's over its CTAs, so a class ends where p and q of a geometry no longer fit
+const ServeClass kServeClasses[SERVE_CLASSES] = {{64, 8, k_serve_modes<64, 8>},
+                                                 {160, 3, k_serve_modes<160, 3>},
+                                                 {256, 2, k_serve_modes<256, 2>},
+                                                 {512, 1, k_serve_modes<512, 1>}};
+
+}  // namespace sp

@@ -257,3 +257,79 @@ def test_micro_message_loop_matches_oracle(mode):
     mb.lib().sp_micro_destroy(h)
     s.stop()
     s.close()
+
+
+# ---------------------------------------------- element-mode request loop ---
+
+MODE_GEOMS = [
+    ((5, 7, 3), (6, 6, 6)),        # 64 threads, eight tasks to an SM
+    ((12, 12, 12), (9, 10, 11)),   # 160 threads, three to an SM
+    ((16, 16, 15),),               # 256 threads, two to an SM
+    ((17, 12, 20), (8, 8, 8)),     # 512 threads, p and q on chip
+    ((24, 20, 20), (32, 10, 31)),  # p on chip; a layer of one strip
+    ((31, 32, 9), (32, 32, 32)),   # strips of rows, no vector on chip
+    ((4, 4, 4), (5, 5, 33)),       # beyond the range: the block-stencil loop
+    ((6, 6, 6), (3, 3, 1)),        # no interior node: the block-stencil loop
+]
+
+
+def mode_desc(n, k):
+    edge = 1.0 / 8 if k % 2 else np.array([0.125, 0.12, 0.13])
+    return mb.rve_desc(n, 0.2, (1e9, 1e9 * (5 + 9 * k)), (0.3, 0.2), list(np.array(n) * edge))
+
+
+def exact_tangents(D):
+    """Effective tangents by the FP64 batch of assembled operators (linear materials:
+    the stress of strain e is C e, and the finite-difference tangent is C)."""
+    b = mb.Batch(D, nrhs=6, precision=mb.SP_PREC_FP64, op=mb.SP_OP_ELL, rtol=1e-11)
+    eye = np.ascontiguousarray(np.broadcast_to(np.eye(6), (len(D), 6, 6)))
+    Cs = np.swapaxes(b.homogenize(eye)[0], 1, 2).copy()
+    b.close()
+    return Cs
+
+
+@pytest.mark.parametrize("k", range(len(MODE_GEOMS)))
+def test_serve_classes_match_batch(k):
+    """Requests one after the other on every class of the loop, against the
+    effective tangent.  Solves to 1e-8 of the right-hand side's norm; the
+    tangent divides a difference of stresses by 0.005, about 2 |eps|."""
+    D = [mode_desc(n, i + k) for i, n in enumerate(MODE_GEOMS[k])]
+    Cs = exact_tangents(D)
+    rng = np.random.default_rng(k)
+    s = mb.Server(D)
+    s.start()
+    for g in [i % len(D) for i in range(4)]:
+        e = rng.normal(0, 1e-3, 6)
+        st, tg, info = s.wait(s.submit(g, e))
+        assert info.status == 0 and info.relres <= 1e-8
+        ref = Cs[g] @ e
+        assert np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+        assert np.abs(np.array(tg).reshape(6, 6) - Cs[g]).max() <= 2e-7 * np.abs(Cs[g]).max()
+    s.stop()
+    s.close()
+
+
+@pytest.mark.parametrize("n,warm", [((6, 6, 6), 0), ((12, 12, 12), 0), ((24, 24, 24), 0),
+                                    ((6, 6, 6), 1)])
+def test_concurrent_cold_requests_on_one_geometry(n, warm):
+    """Requests that arrive together on a geometry without a stored solution,
+    then again: while one stores its solutions the others start from none or
+    from whole ones, never from a mixture."""
+    d = mode_desc(n, 1)
+    Cm = exact_tangents([d])[0]
+    rng = np.random.default_rng(3)
+    nreq = 12 if n[0] > 12 else 40
+    for fresh in range(3):
+        s = mb.Server([d], warm_start=mb.SP_WARM_LAST if warm else mb.SP_WARM_PREDICT)
+        s.start()
+        for again in range(3):
+            E = rng.normal(0, 1e-3, (nreq, 6))
+            tk = [s.submit(0, e) for e in E]
+            for t, e in zip(tk, E):
+                st, tg, info = s.wait(t)
+                assert info.status == 0 and info.relres <= 1e-8
+                ref = Cm @ e
+                assert np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+                assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
+        s.stop()
+        s.close()
