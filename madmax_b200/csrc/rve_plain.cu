@@ -3,7 +3,8 @@
 // (micro/src/homogenize.c:175-225, micro/src/assembly.c:33-137) moved to the
 // GPU without batching or mixed precision: element operators, coloured
 // scatter assembly into ELL, Dirichlet rows/columns, FP64 element residual,
-// Jacobi-PCG (pcg.cuh) and FP64 volume averages.
+// Jacobi-PCG (k_plain_pcg, or pcg.cuh's graph) and FP64 volume averages.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -52,22 +53,56 @@ __global__ void k_affine(MeshGeo g, const double *eps, int nrhs, double *u, bool
                  inside);
 }
 
-// b = -K u (interior), 0 (boundary); norms[k] = ||b_k||^2
+// b = -K u (interior), 0 (boundary); norms[k] = ||b_k||^2.  A thread per
+// (row, load case), load cases fastest: a thread per row, with the K sums in
+// registers, left 27,783 threads for n = 20 and waited on its loads (76 us,
+// 6 load cases).
+constexpr int RES_THREADS = 192;  // a multiple of K = 1, 6 and 8 load cases
 template <int K>
-__global__ void __launch_bounds__(256)
-    k_residual(MeshGeo g, const uint8_t *etype, const double *Ke64, const double *u, double *b,
-               double *norms, double *partial, unsigned *ticket) {
+__global__ void __launch_bounds__(RES_THREADS)
+    k_residual(MeshGeo g, const uint8_t *__restrict__ etype, const double *Ke64,
+               const double *__restrict__ u, double *b, double *norms, double *partial,
+               unsigned *ticket) {
   __shared__ double ke[2 * SP_KE];
   __shared__ double red[33 * K];
   __shared__ double tot[K];
   __shared__ bool flag;
   for (int x = threadIdx.x; x < 2 * SP_KE; x += blockDim.x) ke[x] = Ke64[x];
   __syncthreads();
+  const int q = threadIdx.x % K, nt = gridDim.x * (RES_THREADS / K);
+  double nrm = 0.0;
+  for (int row = (blockIdx.x * RES_THREADS + threadIdx.x) / K; row < g.ndof; row += nt) {
+    const int node = row / 3, d = row % 3;
+    const int i = node % g.nx, j = (node / g.nx) % g.ny, k = node / (g.nx * g.ny);
+    double acc = 0.0;
+    if (!is_bnode(g, node)) {
+#pragma unroll 1
+      for (int c = 0; c < 8; c++) {
+        const int ox = c & 1, oy = (c >> 1) & 1, oz = c >> 2;
+        const int ex = i - 1 + ox, ey = j - 1 + oy, ez = k - 1 + oz;
+        // local index of this node in the element: corner (1-ox, 1-oy, 1-oz)
+        const int cx = 1 - ox, cy = 1 - oy, cz = 1 - oz;
+        const int la = cz * 4 + ((cy == 0) ? (cx ? 1 : 0) : (cx ? 2 : 3));
+        const double *kr = ke + etype[ex + ey * g.nex + ez * g.nex * g.ney] * SP_KE +
+                           (la * 3 + d) * SP_NC;
+        const int n0 = ex + ey * g.nx + ez * g.nx * g.ny;
+        double v[SP_NC];
+#pragma unroll
+        for (int a = 0; a < 8; a++)
+#pragma unroll
+          for (int e = 0; e < 3; e++)
+            v[a * 3 + e] = u[(size_t)(3 * (n0 + corner_x(a) + corner_y(a) * g.nx +
+                                           corner_z(a) * g.nx * g.ny) + e) * K + q];
+#pragma unroll
+        for (int a = 0; a < SP_NC; a++) acc = fma(kr[a], v[a], acc);
+      }
+    }
+    b[(size_t)row * K + q] = -acc;
+    nrm += acc * acc;
+  }
   double mine[K];
-  #pragma unroll
-  for (int k = 0; k < K; k++) mine[k] = 0.0;
-  residual_nodes<K, double>(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g,
-                            etype, ke, u, b, mine);
+#pragma unroll
+  for (int k = 0; k < K; k++) mine[k] = k == q ? nrm : 0.0;
   if (grid_sum<K>(mine, partial, ticket, red, tot, &flag) && threadIdx.x == 0)
     #pragma unroll
     for (int k = 0; k < K; k++) norms[k] = tot[k];
@@ -79,11 +114,12 @@ __global__ void k_add(int n, const double *x, double *u) {
   for (int i = t; i < n * K; i += nt) u[i] += x[i];
 }
 
-// averages of load case q: out[0..5] strain, out[6..11] stress
+// averages of load case q = blockIdx.y: out[0..5] strain, out[6..11] stress
 template <int K>
 __global__ void __launch_bounds__(256)
     k_average(MeshGeo g, const uint8_t *etype, const double *D, const double *Bbar,
-              const double *u, int q, double *out, double *partial, unsigned *ticket) {
+              const double *u, double *out, double *partial, unsigned *ticket) {
+  const int q = blockIdx.y;
   __shared__ double sD[72], sB[144];
   __shared__ double red[33 * 12];
   __shared__ double tot[12];
@@ -96,9 +132,224 @@ __global__ void __launch_bounds__(256)
   for (int v = 0; v < 12; v++) acc[v] = 0.0;
   average_elems<K>(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, g, etype, sD,
                    sB, u, q, acc);
-  if (grid_sum<12>(acc, partial, ticket, red, tot, &flag) && threadIdx.x == 0)
+  if (grid_sum<12>(acc, partial + (size_t)q * gridDim.x * 12, ticket + q, red, tot, &flag) &&
+      threadIdx.x == 0)
     #pragma unroll
     for (int v = 0; v < 12; v++) out[q * 12 + v] = tot[v] / g.vol;
+}
+
+// u [ndof][K] -> out [nrhs][ndof]
+template <int K>
+__global__ void k_split(int n, int nrhs, const double *u, double *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  for (int i = t; i < n * nrhs; i += nt) out[i] = u[(size_t)(i % n) * K + i / n];
+}
+
+// Sums of a[0..N) over the lanes of a warp, spread over the lanes: halves of
+// the array are exchanged and added, 20 exchanges for N = 18 instead of the 90
+// of a butterfly per value.  A lane is left with the total of a[spread_index]
+// (-1: none).
+template <int N, int OFF = 16>
+__device__ __forceinline__ double spread_sum(const double (&a)[N]) {
+  if constexpr (OFF == 0) {
+    return a[0];
+  } else {
+    constexpr int H = (N + 1) / 2;
+    const bool up = threadIdx.x & OFF;
+    double h[H];
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+      const double lo = a[i], hi = H + i < N ? a[H + i] : 0.0;
+      h[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, OFF);
+    }
+    return spread_sum<H, OFF / 2>(h);
+  }
+}
+
+__device__ __forceinline__ int spread_index(int n) {
+  int lo = 0, cnt = n;  // values left here, of n padded ones
+  for (int off = 16; off; off >>= 1) {
+    const int h = (n + 1) / 2;
+    if (threadIdx.x & off) {
+      lo += h;
+      cnt -= h;
+    } else if (cnt > h) {
+      cnt = h;
+    }
+    n = h;
+  }
+  return cnt > 0 ? lo : -1;
+}
+
+struct PlainPcg {
+  MeshGeo g;
+  const double *vals, *dinv, *b;
+  const int *cols;
+  double *z, *x, *r, *q;  // z: D^-1 r, gathered by the other blocks
+  double *u;              // += the solution
+  PcgState *st;
+  double *part_a, *part_b;
+  int onchip;             // r, q, x in shared memory
+};
+
+// Jacobi-PCG of K load cases from x = 0 over the interior nodes in one
+// cooperative launch, a block per SM with a contiguous range of nodes, a warp
+// per node: the node's three rows have one column list, so a gathered value
+// serves three rows, and the 3K sums are spread over the lanes, which own the
+// node's vector entries.  Vectors that no other block reads stay in shared
+// memory.  Only z = D^-1 r is gathered: p = z + beta p and q = A z + beta q
+// (= A p) are local, so an iteration has two grid barriers, one after each
+// reduction.  Every block folds the partial sums in the same order and takes
+// the same exit.
+//
+// What bounds it: the latency of the two barriers and folds and of one gather
+// (the matrix, 18 MB at n = 20, is re-read from L2).  Against three kernels
+// an iteration in a graph, a warp per row: 53 -> 15 us an iteration at n = 20
+// with 6 load cases.
+constexpr int PLAIN_NT = 512;
+template <int K>
+__global__ void __launch_bounds__(PLAIN_NT, 1) k_plain_pcg(const __grid_constant__ PlainPcg P) {
+  namespace cgr = cooperative_groups;
+  cgr::grid_group grid = cgr::this_grid();
+  constexpr int W = 3 * K, NW = PLAIN_NT / 32;
+  extern __shared__ __align__(16) double plain_sm[];
+  __shared__ double red[2][NW][W];
+  __shared__ double tot[2 * K];
+  const MeshGeo &g = P.g;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nb = gridDim.x, blk = blockIdx.x;
+  const int mx = g.nx - 2, my = g.ny - 2, ni = mx * my * (g.nz - 2);
+  const int c0 = (int)((long long)ni * blk / nb), m = (int)((long long)ni * (blk + 1) / nb) - c0;
+  const int mmax = (ni + nb - 1) / nb;
+  double *const p_s = plain_sm;
+  double *const r_s = P.onchip ? p_s + (size_t)mmax * W : P.r;
+  double *const q_s = P.onchip ? r_s + (size_t)mmax * W : P.q;
+  double *const x_s = P.onchip ? q_s + (size_t)mmax * W : P.x;
+  const int own = spread_index(W), k = own < 0 ? 0 : own % K, d = own < 0 ? 0 : own / K;
+  auto node_of = [&](int li) {
+    const int id = c0 + li;
+    return 1 + id % mx + (1 + id / mx % my) * g.nx + (1 + id / (mx * my)) * g.nx * g.ny;
+  };
+  auto at = [&](int li, int node) { return (size_t)(P.onchip ? li : node) * W + own; };
+  // per-block sums of NV values per load case -> part, grid barrier, totals
+  auto sum = [&](double v0, double v1, int nv, double *part) {
+    if (own >= 0) {
+      red[0][warp][own] = v0;
+      red[1][warp][own] = v1;
+    }
+    __syncthreads();
+    for (int v = warp; v < nv * K; v += NW) {
+      const double *e = &red[v / K][lane < NW ? lane : 0][v % K];
+      double s = lane < NW ? e[0] + e[K] + e[2 * K] : 0.0;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) part[(size_t)v * nb + blk] = s;
+    }
+    grid.sync();
+    for (int v = warp; v < nv * K; v += NW) {
+      double s = 0.0;
+      for (int i = lane; i < nb; i += 32) s += __ldcg(part + (size_t)v * nb + i);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+      if (lane == 0) tot[v] = s;
+    }
+    __syncthreads();
+  };
+  const double rtol2 = P.st->rtol2;
+  const int max_its = P.st->max_its, nrhs = P.st->nactive;
+  // start: x = p = q = 0, r = b, z = D^-1 r (0 on the boundary); r.z, b.b
+  const int t = blk * PLAIN_NT + threadIdx.x, nt = nb * PLAIN_NT;
+  for (int node = t; node < g.nn; node += nt)
+    if (is_bnode(g, node))
+      for (int i = 0; i < W; i++) P.z[(size_t)node * W + i] = 0.0;
+  double rz = 0.0, rr = 0.0;
+  if (own >= 0)
+    for (int li = warp; li < m; li += NW) {
+      const int node = node_of(li);
+      const size_t o = at(li, node);
+      const double r = P.b[(size_t)node * W + own], z = P.dinv[node * 3 + d] * r;
+      x_s[o] = q_s[o] = p_s[(size_t)li * W + own] = 0.0;
+      r_s[o] = r;
+      P.z[(size_t)node * W + own] = z;
+      rz += r * z;
+      rr += r * r;
+    }
+  sum(rz, rr, 2, P.part_b);
+  // the scalars of this lane's load case, and how many are active in all
+  double rho = tot[k], beta = 0.0;
+  const double bb = tot[K + k];
+  unsigned act = 0;
+#pragma unroll
+  for (int i = 0; i < K; i++) act |= (tot[K + i] > 0.0 && i < nrhs ? 1u : 0u) << i;
+  __syncthreads();
+  int its = 0;
+  while (act && its < max_its) {
+    double pq = 0.0;
+    for (int li = warp; li < m; li += NW) {
+      const int node = node_of(li);
+      const double *vr = P.vals + (size_t)node * 3 * SP_WP;
+      const int *cr = P.cols + (size_t)node * 3 * SP_WP;
+      double a[W];
+#pragma unroll
+      for (int i = 0; i < W; i++) a[i] = 0.0;
+#pragma unroll
+      for (int s = 0; s < 3; s++) {
+        const int j = lane + 32 * s;
+        if (j < SP_ELL_WIDTH) {
+          const int c = __ldg(cr + j);
+          const double v0 = __ldg(vr + j), v1 = __ldg(vr + SP_WP + j), v2 = __ldg(vr + 2 * SP_WP + j);
+          double zv[K];
+          load_k<double, K, false>(P.z + (size_t)(c < 0 ? 0 : c) * K, zv);
+#pragma unroll
+          for (int i = 0; i < K; i++) {
+            a[i] = fma(v0, zv[i], a[i]);
+            a[K + i] = fma(v1, zv[i], a[K + i]);
+            a[2 * K + i] = fma(v2, zv[i], a[2 * K + i]);
+          }
+        }
+      }
+      const double az = spread_sum<W>(a);
+      if (own >= 0) {
+        const size_t o = at(li, node), op = (size_t)li * W + own;
+        const double p = fma(beta, p_s[op], P.z[(size_t)node * W + own]);
+        const double q = fma(beta, q_s[o], az);
+        p_s[op] = p;
+        q_s[o] = q;
+        pq = fma(p, q, pq);
+      }
+    }
+    sum(pq, 0.0, 1, P.part_a);
+    const double alpha = (act >> k & 1) && tot[k] != 0.0 ? rho / tot[k] : 0.0;
+    rz = rr = 0.0;
+    if (own >= 0)
+      for (int li = warp; li < m; li += NW) {
+        const int node = node_of(li);
+        const size_t o = at(li, node);
+        x_s[o] = fma(alpha, p_s[(size_t)li * W + own], x_s[o]);
+        const double r = fma(-alpha, q_s[o], r_s[o]), z = P.dinv[node * 3 + d] * r;
+        r_s[o] = r;
+        P.z[(size_t)node * W + own] = z;
+        rz = fma(r, z, rz);
+        rr = fma(r, r, rr);
+      }
+    sum(rz, rr, 2, P.part_b);
+    its++;
+    unsigned done = 0;
+    if (tot[K + k] <= rtol2 * bb) done = 1u << k;
+    done = __reduce_or_sync(0xffffffffu, own >= 0 ? done : 0u);
+    act &= ~done;
+    beta = (act >> k & 1) && rho != 0.0 ? tot[k] / rho : 0.0;
+    if (act >> k & 1) rho = tot[k];
+  }
+  if (own >= 0)
+    for (int li = warp; li < m; li += NW) {
+      const int node = node_of(li);
+      P.u[(size_t)node * W + own] += x_s[at(li, node)];
+    }
+  if (t == 0) {
+    P.st->its = its;
+    P.st->nactive = __popc(act);
+  }
 }
 
 // Per-element strain and stress of load case q (micro/src/homogenize.c:
@@ -159,6 +410,32 @@ struct sp_rve_s {
   size_t bytes = 0;
   int last_k = 0, last_nrhs = 0;  // padded and actual load cases of the last solve
 };
+
+// The cooperative solve wants a block on as many SMs at once as it has work
+// for, at most one each; a serving loop on the device may hold some of them
+// for as long as requests come, so beside one the graph of small kernels runs.
+// p has to fit the blocks' shared memory (n <= 54 with 8 load cases); larger
+// RVEs stream the matrix from HBM either way.
+template <int K>
+static int plain_launch(sp_rve *r, Device *d, cudaStream_t s, bool *taken) {
+  *taken = false;
+  const MeshGeo &g = r->g;
+  const long long ni = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
+  if (ni < 1 || d->loops.load() > 0) return SP_OK;
+  const int nb = (int)std::min<long long>(d->nsm, (ni + PLAIN_NT / 32 - 1) / (PLAIN_NT / 32));
+  const size_t vec = (size_t)((ni + nb - 1) / nb) * 3 * K * sizeof(double), room = 200 * 1024;
+  if (vec > room) return SP_OK;
+  PlainPcg P = {g, r->d_vals, r->d_dinv, r->d_b, r->plan->cols, r->d_p, r->d_x, r->d_r, r->d_q,
+                r->d_u, r->d_st, r->d_partial, r->d_partial + (size_t)d->nsm * 2 * K,
+                4 * vec <= room};
+  SP_CUDA_TRY(cudaFuncSetAttribute((const void *)k_plain_pcg<K>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
+  void *args[] = {&P};
+  SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain_pcg<K>, dim3(nb), dim3(PLAIN_NT),
+                                          args, P.onchip ? 4 * vec : vec, s));
+  *taken = true;
+  return SP_OK;
+}
 
 static int rve_assemble(sp_rve *r, Device *d, cudaStream_t s) {
   MeshGeo &g = r->g;
@@ -295,15 +572,10 @@ static int rve_solve_k(sp_rve *r, Device *d, PcgGraph<double, K, 32> *&pcg, int 
                        double *u_out, sp_solve_info *info) {
   cudaStream_t s = d->stream;
   MeshGeo &g = r->g;
-  int nb_node = blocks_for(d, g.ndof / 3, 256);
+  int nb_res = blocks_for(d, (long long)g.ndof * K, RES_THREADS);
   int nb_vec = blocks_for(d, (long long)g.ndof * K, 256);
   int nb_row = blocks_for(d, g.ndof, PCG_THREADS / 32);
   int launches = 0;
-  if (!pcg) {
-    pcg = new PcgGraph<double, K, 32>();
-    SP_TRY(pcg->build(s, nb_row, g.ndof, SP_WP, r->d_vals, r->plan->cols, r->d_dinv, r->d_b,
-                      r->d_x, r->d_r, r->d_p, r->d_q, 1, r->d_st, r->d_partial, r->d_ticket));
-  }
   double eps[KMAX * 6] = {0};
   memcpy(eps, strains, (size_t)nrhs * 6 * sizeof(double));
   SP_CUDA_TRY(cudaMemcpyAsync(r->d_eps, eps, sizeof(eps), cudaMemcpyHostToDevice, s));
@@ -319,7 +591,7 @@ static int rve_solve_k(sp_rve *r, Device *d, PcgGraph<double, K, 32> *&pcg, int 
   // homogeneous RVE), which leaves the error near the material interfaces.
   for (;;) {
     double nrm[KMAX];
-    k_residual<K><<<nb_node, 256, 0, s>>>(g, r->d_etype, r->d_Ke, r->d_u, r->d_b, r->d_out + 8 * 12,
+    k_residual<K><<<nb_res, RES_THREADS, 0, s>>>(g, r->d_etype, r->d_Ke, r->d_u, r->d_b, r->d_out + 8 * 12,
                                          r->d_partial, r->d_ticket);
     launches++;
     SP_CUDA_TRY(cudaMemcpyAsync(nrm, r->d_out + 8 * 12, K * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -343,37 +615,35 @@ static int rve_solve_k(sp_rve *r, Device *d, PcgGraph<double, K, 32> *&pcg, int 
     st0.max_its = 20000;
     SP_CUDA_TRY(cudaMemcpyAsync(r->d_st, &st0, sizeof(st0), cudaMemcpyHostToDevice, s));
     int fixed = 0;
-    SP_TRY(pcg->run(s, &fixed));
-    k_add<K><<<nb_vec, 256, 0, s>>>(g.ndof, r->d_x, r->d_u);
+    bool coop;
+    SP_TRY(plain_launch<K>(r, d, s, &coop));
+    if (!coop) {
+      if (!pcg) {
+        pcg = new PcgGraph<double, K, 32>();
+        SP_TRY(pcg->build(s, nb_row, g.ndof, SP_WP, r->d_vals, r->plan->cols, r->d_dinv, r->d_b,
+                          r->d_x, r->d_r, r->d_p, r->d_q, 1, r->d_st, r->d_partial, r->d_ticket));
+      }
+      SP_TRY(pcg->run(s, &fixed));
+      k_add<K><<<nb_vec, 256, 0, s>>>(g.ndof, r->d_x, r->d_u);
+    }
     PcgState st;
     SP_CUDA_TRY(cudaMemcpyAsync(&st, r->d_st, sizeof(st), cudaMemcpyDeviceToHost, s));
     SP_CUDA_TRY(cudaStreamSynchronize(s));
-    launches += fixed + 3 * st.its + 1;
+    launches += coop ? 1 : fixed + 3 * st.its + 1;
     inner += st.its;
     outer++;
   }
-  for (int q = 0; q < nrhs; q++) {
-    k_average<K><<<blocks_for(d, g.nelm, 256), 256, 0, s>>>(g, r->d_etype, r->d_D, r->d_Bbar,
-                                                            r->d_u, q, r->d_out, r->d_partial,
-                                                            r->d_ticket);
-    launches++;
-  }
+  k_average<K><<<dim3(blocks_for(d, g.nelm, 256), nrhs), 256, 0, s>>>(
+      g, r->d_etype, r->d_D, r->d_Bbar, r->d_u, r->d_out, r->d_partial, r->d_ticket);
+  launches++;
   double out[KMAX * 12];
   SP_CUDA_TRY(cudaMemcpyAsync(out, r->d_out, sizeof(out), cudaMemcpyDeviceToHost, s));
   if (u_out) {
     // u is [ndof][K]; the caller wants [nrhs][ndof]
-    double *h = (double *)malloc((size_t)g.ndof * K * sizeof(double));
-    if (!h) return sp_set_error(SP_ERR_NOMEM, "u staging");
-    cudaError_t e = cudaMemcpyAsync(h, r->d_u, (size_t)g.ndof * K * sizeof(double),
-                                    cudaMemcpyDeviceToHost, s);
-    if (!e) e = cudaStreamSynchronize(s);
-    if (e) {
-      free(h);
-      return sp_set_error(SP_ERR_CUDA, "u download failed");
-    }
-    for (int k = 0; k < nrhs; k++)
-      for (int i = 0; i < g.ndof; i++) u_out[(size_t)k * g.ndof + i] = h[(size_t)i * K + k];
-    free(h);
+    k_split<K><<<nb_vec, 256, 0, s>>>(g.ndof, nrhs, r->d_u, r->d_x);
+    launches++;
+    SP_CUDA_TRY(cudaMemcpyAsync(u_out, r->d_x, (size_t)g.ndof * nrhs * sizeof(double),
+                                cudaMemcpyDeviceToHost, s));
   }
   SP_CUDA_TRY(cudaStreamSynchronize(s));
   double worst = 0.0;

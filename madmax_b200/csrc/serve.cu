@@ -477,6 +477,7 @@ struct sp_server_s {
   long long tail = 0, head_done = 0;
   cudaStream_t stream = nullptr;
   ServeParams P;
+  Device *device = nullptr;
   bool modes = false;    // the element-mode loop, of class cls
   int cls = -1;
   ServeJob *d_jobs = nullptr;
@@ -618,6 +619,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   s->ngeom = ngeom;
   s->o = o;
   s->dev = d->id;
+  s->device = d;
   s->cap = o.queue_capacity;
   s->grid = slots + 1; // + dispatcher
   s->cls = cls;
@@ -843,6 +845,7 @@ static int server_launch(sp_server *s) {
   else
     serve_kernel(s->o)<<<s->grid, SERVE_NT, serve_dyn_smem(s->o), s->stream>>>(s->P);
   SP_CUDA_TRY(cudaGetLastError());
+  if (!s->running) s->device->loops++;
   s->running = 1;
   s->launches++;
   return SP_OK;
@@ -935,6 +938,7 @@ extern "C" int sp_server_stop(sp_server *s) {
   std::atomic_thread_fence(std::memory_order_seq_cst);
   cudaError_t e = cudaStreamSynchronize(s->stream);
   s->running = 0;
+  s->device->loops--;
   if (e) return sp_set_error(SP_ERR_CUDA, "serving loop: %s", cudaGetErrorString(e));
   // requests published after the loop saw stop: run them to completion
   ServeDev z;
@@ -946,6 +950,7 @@ extern "C" int sp_server_stop(sp_server *s) {
     std::atomic_thread_fence(std::memory_order_seq_cst);
     e = cudaStreamSynchronize(s->stream);
     s->running = 0;
+    s->device->loops--;
     if (e) return sp_set_error(SP_ERR_CUDA, "serving loop: %s", cudaGetErrorString(e));
   }
   return SP_OK;

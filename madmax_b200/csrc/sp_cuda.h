@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
@@ -31,6 +32,7 @@ struct Device {
   int id = -1;
   int nsm = 0;
   cudaStream_t stream = nullptr; // library stream (non-blocking)
+  std::atomic<int> loops{0};     // serving loops started and not stopped
 };
 
 // Current device of the calling thread, initialised on first use.
