@@ -115,8 +115,8 @@ PROFILED_TRAFFIC = {
     # -k regex:k_batch -s 13 -c 1 python bench.py --steps 1 --warmup 3 ...
     "k_batch --nrve 4096 --sizes 8 12 16 20 --op stencil --threads 0 --ctas 0 "
     "--inner-rtol 0.003": 663920980224,
-    # k_spmv_rve, the n = 40 structured matrix, cold L2
-    "k_spmv_rve structured ELL n=40": 214213376,
+    # k_spmv_node, the n = 40 structured matrix, cold L2
+    "k_spmv_node structured ELL n=40": 152290000,
 }
 
 
@@ -155,10 +155,10 @@ def structured_ell(n: int, seed: int = 5):
 
 def measure_spmv(mb, stream, sptr, n=40, reps=20):
     """The resident FP64 ELL SpMV (sp_ell_dev_mvp) on one matrix larger than
-    L2, at the lanes-per-row width the library's upload-time autotuner chose
-    (no override), L2 flushed before every timed launch; achieved =
-    algorithmic bytes (stored slots x 12 + x read + y write) / CUDA-event
-    time per launch."""
+    L2, without a lanes-per-row override (rows in node triples: a warp per
+    node), L2 flushed before every timed launch; achieved = algorithmic bytes
+    (stored slots x 8 + a node index per 9 of them x 4 + x read + y write) /
+    CUDA-event time per launch."""
     import torch
     cols, vals = structured_ell(n)
     m = mb.ell_matrix()
@@ -203,20 +203,20 @@ def measure_spmv(mb, stream, sptr, n=40, reps=20):
         torch.cuda.synchronize()
         ms = sum(e0.elapsed_time(e1) for e0, e1 in evs) / reps
         del flush, sink
-        abytes = nnz.value * 12 + 2 * nrow.value * 8
+        abytes = nnz.value * 8 + nnz.value // 9 * 4 + 2 * nrow.value * 8
         peak, peak_kind = measured_peak()
         ach = abytes / (ms / 1e3) / 1e9
-        return {"kernel": "k_spmv_rve (sp_ell_dev_mvp, FP64 ELL, hoisted loads)",
+        return {"kernel": "k_spmv_node (sp_ell_dev_mvp, FP64 ELL, a warp per node)",
                 "matrix": f"hex8 RVE sparsity n={n}: {nrow.value} rows x 84 slots, "
                           f"{nnz.value} stored, {(vals.nbytes + cols.nbytes) / 1e6:.0f} MB > L2",
                 "l2": "flushed before every timed launch (a 256 MB read)",
-                "lanes_per_row": lanes.value,
+                "row_kernel_lanes": lanes.value,
                 "lanes_source": "the library's upload-time autotuner" +
                                 (" (cached choice)" if cached.value else ""),
                 "autotuner_trial_us": {str(w): round(float(t), 2)
                                        for w, t in zip((4, 8, 16, 32), trial)},
                 "ms": ms, "algorithmic_bytes": abytes,
-                "traffic": profiled_traffic("k_spmv_rve", f"structured ELL n={n}")[0],
+                "traffic": profiled_traffic("k_spmv_node", f"structured ELL n={n}")[0],
                 "achieved": ach, "peak": peak, "unit": "GB/s",
                 "frac": ach / peak, "peak_kind": peak_kind, "max_rel_err_vs_numpy": err}
     finally:

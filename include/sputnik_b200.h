@@ -76,7 +76,9 @@ int sp_ell_dev_mvp_host(sp_ell_dev *a, const double *x, double *y);
  * choice).  For 84-slot (RVE-shaped) rows, sp_ell_upload times every width
  * on the uploaded matrix and keeps the fastest (cached per device, row width
  * and row-count octave).  A tuning knob; the result does not depend on it
- * beyond rounding. */
+ * beyond rounding.  A matrix whose rows 3a..3a+2 share one list of whole
+ * nodes' columns (every assembled RVE), of 6,000 rows or more, is multiplied a warp per node instead
+ * while no width is set here. */
 int sp_ell_dev_set_lanes(sp_ell_dev *a, int lanes);
 /* The lanes per row sp_ell_dev_mvp uses, the upload-time trial's time per
  * launch at 4, 8, 16 and 32 lanes (microseconds; trial_us may be NULL) and

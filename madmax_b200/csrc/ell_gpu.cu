@@ -313,6 +313,7 @@ struct sp_ell_dev_s {
   long long true_nnz = 0;  // stored (non-empty) slots
   int *cols = nullptr;    // [nrow][wp]
   double *vals = nullptr; // [nrow][wp]
+  int *nbr = nullptr;     // [nrow/3][28] neighbour nodes, if the rows are node triples
   double *dinv = nullptr;
   double *vec = nullptr;  // 5 vectors of nrow + x of ncol
   PcgState *st = nullptr;
@@ -320,6 +321,74 @@ struct sp_ell_dev_s {
   unsigned *ticket = nullptr;
   PcgGraph<double, 1, 32> *pcg = nullptr;
 };
+
+// y = A x of a matrix in node triples (sp_ell_dev_s::nbr): a node's three rows
+// have one column list, made of whole nodes.  A warp takes NODE_PER nodes; a
+// lane has a column, its three values and one gather for the three rows, and
+// the three sums are spread over the lanes.  One index per 9 values is read
+// instead of 9: 2,128 instead of 3,024 B a node, which bounds it (HBM): 39.2 ->
+// 26.7 us at 206,763 rows against the best row width of k_spmv_rve.
+constexpr int NODE_PER = 2, NODE_WP = 28;
+// Fewer rows fit the caches and are latency: 2,187 rows take 2.3 us here and
+// 2.0 us at the best row width, 6,591 rows 2.4 and 2.6 us, 27,783 rows 3.8 and
+// 5.0 us.
+constexpr int NODE_MIN_ROWS = 6000;
+__global__ void __launch_bounds__(PCG_THREADS)
+    k_spmv_node(int nnode, const double *__restrict__ vals, const int *__restrict__ nbr,
+                const double *__restrict__ x, double *__restrict__ y) {
+  const int lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * (PCG_THREADS / 32) + (threadIdx.x >> 5)) * NODE_PER;
+  if (n0 >= nnode) return;
+  int b[NODE_PER][3];
+  double v[NODE_PER][9];
+#pragma unroll
+  for (int u = 0; u < NODE_PER; u++) {
+    const int node = min(n0 + u, nnode - 1);
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const int j = lane + 32 * s;
+      const bool in = j < SP_ELL_WIDTH;
+      b[u][s] = in ? __ldg(nbr + (size_t)node * NODE_WP + j / 3) : -1;
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+        v[u][3 * s + r] = in ? __ldcs(vals + ((size_t)node * 3 + r) * SP_WP + j) : 0.0;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NODE_PER; u++) {
+    double a[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+      const double xv = b[u][s] < 0 ? 0.0 : __ldg(x + (size_t)b[u][s] * 3 + (lane + 32 * s) % 3);
+#pragma unroll
+      for (int r = 0; r < 3; r++) a[r] = fma(v[u][3 * s + r], xv, a[r]);
+    }
+    const double sum = spread_sum<3>(a);
+    const int r = spread_index(3);
+    if (r >= 0 && n0 + u < nnode) y[(size_t)(n0 + u) * 3 + r] = sum;
+  }
+}
+
+// The neighbour nodes of a matrix whose rows 3a, 3a + 1, 3a + 2 share one
+// list of whole nodes' columns (any order, empty slots last): [nrow/3][28],
+// -1 after the last, for the caller to free.  Null if the matrix is not of
+// this form (or without the memory): the row kernels take any matrix.
+static int *node_lists(const int *cols, int nrow, int wp) {
+  if (wp != SP_WP || nrow % 3 || nrow < NODE_MIN_ROWS) return nullptr;
+  int *nbr = (int *)malloc((size_t)nrow / 3 * NODE_WP * sizeof(int));
+  for (int a = 0; nbr && a < nrow / 3; a++) {
+    const int *c = cols + (size_t)3 * a * wp;
+    for (int j = 0; j < wp; j++) {
+      const int b = j < SP_ELL_WIDTH ? c[j / 3 * 3] : -1, want = b < 0 ? -1 : b + j % 3;
+      if ((b > 0 && b % 3) || c[j] != want || c[wp + j] != want || c[2 * wp + j] != want) {
+        free(nbr);
+        return nullptr;
+      }
+      if (j % 3 == 0) nbr[(size_t)a * NODE_WP + j / 3] = b < 0 ? -1 : b / 3;
+    }
+  }
+  return nbr;
+}
 
 static void launch_spmv_rve(int L, int nb, cudaStream_t s, const sp_ell_dev_s *a, const double *x,
                             double *y) {
@@ -480,6 +549,14 @@ extern "C" int sp_ell_upload(const ell_matrix *m, sp_ell_dev **out) {
                 cudaMemcpy(a->dinv, hd, a->nrow * sizeof(double), cudaMemcpyHostToDevice) ||
                 cudaMemset(a->ticket, 0, 64)))
       rc = sp_set_error(SP_ERR_CUDA, "sp_ell_upload: copy failed");
+    int *nbr = rc ? nullptr : node_lists(hc, a->nrow, a->wp);
+    if (nbr) {
+      const size_t nb = (size_t)a->nrow / 3 * NODE_WP * sizeof(int);
+      rc = dmalloc((void **)&a->nbr, nb, nullptr);
+      if (!rc && cudaMemcpy(a->nbr, nbr, nb, cudaMemcpyHostToDevice))
+        rc = sp_set_error(SP_ERR_CUDA, "sp_ell_upload: copy failed");
+      free(nbr);
+    }
   }
   free(hc);
   free(hv);
@@ -498,6 +575,7 @@ extern "C" int sp_ell_dev_free(sp_ell_dev *a) {
   delete a->pcg;
   cudaFree(a->cols);
   cudaFree(a->vals);
+  cudaFree(a->nbr);
   cudaFree(a->dinv);
   cudaFree(a->vec);
   cudaFree(a->st);
@@ -512,7 +590,12 @@ extern "C" int sp_ell_dev_mvp(sp_ell_dev *a, const double *x_dev, double *y_dev,
   Device *d;
   SP_TRY(device(&d));
   cudaStream_t s = pick_stream(stream, d);
-  if (a->wp == SP_WP) {
+  if (a->nbr && !a->lanes) {
+    // node triples, unless the caller set a row width
+    const int per = PCG_THREADS / 32 * NODE_PER, nnode = a->nrow / 3;
+    k_spmv_node<<<(nnode + per - 1) / per, PCG_THREADS, 0, s>>>(nnode, a->vals, a->nbr, x_dev,
+                                                                y_dev);
+  } else if (a->wp == SP_WP) {
     // RVE-shaped rows: 84 slots, loads hoisted; lanes per row from the
     // caller or the upload-time autotuner
     const int L = a->lanes ? a->lanes : a->lanes_tuned;

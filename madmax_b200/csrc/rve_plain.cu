@@ -145,42 +145,6 @@ __global__ void k_split(int n, int nrhs, const double *u, double *out) {
   for (int i = t; i < n * nrhs; i += nt) out[i] = u[(size_t)(i % n) * K + i / n];
 }
 
-// Sums of a[0..N) over the lanes of a warp, spread over the lanes: halves of
-// the array are exchanged and added, 20 exchanges for N = 18 instead of the 90
-// of a butterfly per value.  A lane is left with the total of a[spread_index]
-// (-1: none).
-template <int N, int OFF = 16>
-__device__ __forceinline__ double spread_sum(const double (&a)[N]) {
-  if constexpr (OFF == 0) {
-    return a[0];
-  } else {
-    constexpr int H = (N + 1) / 2;
-    const bool up = threadIdx.x & OFF;
-    double h[H];
-#pragma unroll
-    for (int i = 0; i < H; i++) {
-      const double lo = a[i], hi = H + i < N ? a[H + i] : 0.0;
-      h[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, OFF);
-    }
-    return spread_sum<H, OFF / 2>(h);
-  }
-}
-
-__device__ __forceinline__ int spread_index(int n) {
-  int lo = 0, cnt = n;  // values left here, of n padded ones
-  for (int off = 16; off; off >>= 1) {
-    const int h = (n + 1) / 2;
-    if (threadIdx.x & off) {
-      lo += h;
-      cnt -= h;
-    } else if (cnt > h) {
-      cnt = h;
-    }
-    n = h;
-  }
-  return cnt > 0 ? lo : -1;
-}
-
 struct PlainPcg {
   MeshGeo g;
   const double *vals, *dinv, *b;

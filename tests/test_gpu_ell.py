@@ -192,3 +192,36 @@ def test_reference_unity_program_linked_to_library(golden_dir, tmp_path):
     assert int([ln for ln in lines if ln.startswith("its")][0].split("=")[1]) == 388
     x = [float(v) for v in open(tmp_path / "sol.dat").read().split()]
     assert x == d["printed_x"]
+
+
+def test_node_kernel_only_takes_node_triples():
+    """The resident SpMV's node kernel (a warp per node) against the host's
+    row sums: an RVE matrix (boundary nodes with short lists, an odd node
+    count), and matrices one change away from its form, which the row kernel
+    has to take: a column out of place in one row, an index list that starts
+    inside a node, and a row count that is no multiple of three."""
+    base = O.assemble(O.cube_mesh(12), np.zeros(12 ** 3, np.uint8), (1e9, 1e9), (0.3, 0.3))
+    rng = np.random.default_rng(3)
+    cases = []
+    for k in range(4):
+        cols, vals = base.cols.copy(), np.where(base.cols >= 0, rng.standard_normal(base.cols.shape), 0.0)
+        if k == 1:
+            cols[7, [0, 1]] = cols[7, [1, 0]]
+        elif k == 2:
+            cols[cols >= 0] = (cols[cols >= 0] + 1) % cols.shape[0]
+        elif k == 3:
+            cols, vals = cols[:-1].copy(), vals[:-1].copy()
+            vals[cols >= cols.shape[0]] = 0.0
+            cols[cols >= cols.shape[0]] = 0
+        cases.append((np.ascontiguousarray(cols), np.ascontiguousarray(vals)))
+    for cols, vals in cases:
+        B = as_lib_matrix(cols, vals)
+        h = mb._vp()
+        mb.check(mb.lib().sp_ell_upload(C.byref(B.m), C.byref(h)), "upload")
+        x = rng.standard_normal(cols.shape[0])
+        y = np.zeros_like(x)
+        mb.check(mb.lib().sp_ell_dev_mvp_host(h, mb.ptr(x), mb.ptr(y)), "mvp")
+        mb.lib().sp_ell_dev_free(h)
+        t = np.where(cols >= 0, vals * x[np.maximum(cols, 0)], 0.0)
+        # 81 terms in any order: at most 81 roundings of the magnitudes' sum
+        assert (np.abs(y - t.sum(1)) <= 81 * 2.0 ** -53 * np.abs(t).sum(1) * 2).all()
