@@ -415,9 +415,10 @@ static size_t store_len(const ModesGeo &G) { return (size_t)SERVE_NRHS * (3 * G.
 // open, or one asked for (the last class), and every geometry in the range.
 // Measured: a burst of 96 requests on geometries of n = 8..32, 250 ms in the
 // block-stencil loop, 62 ms in the last class (a CTA per load case instead of
-// one per request, vectors on chip); a step of 512 points with n = 12 RVEs
-// 49.8 ms of micro solves there, 53.0 ms in the last class, whose 16 warps are a
-// third full, and 37.8 ms in the class of 160 threads, three to an SM.
+// one per request, vectors on chip); three passes over 6,912 points with n = 12
+// RVEs 49.8 ms there, 53.0 ms in the last class, whose 16 warps are a third
+// full, and 37.8 ms in the class of 160 threads, three to an SM (17.6 ms since
+// every CTA gets its share of the tasks, see serve_claim).
 static int serve_class(int ngeom, const sp_rve_desc *descs, const sp_server_opts &o) {
   if (o.op != SP_OP_STENCIL || o.ctas_per_sm < 0 || o.ctas_per_sm > 1) return -1;
   for (int c = o.ctas_per_sm == 1 ? SERVE_CLASSES - 1 : 0; c < SERVE_CLASSES; c++) {
@@ -832,10 +833,23 @@ static int server_grid(sp_server *s, Device *d) {
   return SP_OK;
 }
 
+// The element-mode loop's tickets may run past the published load cases; those
+// are free again once the loop has ended.
+static long long tickets(const sp_server *s, const ServeDev &z) {
+  return s->modes ? std::min((long long)z.claim, (long long)z.dtail * SERVE_NRHS)
+                  : (long long)z.claim;
+}
+
+// whether an ended loop left submitted requests unclaimed
+static bool unclaimed(const sp_server *s, const ServeDev &z) {
+  return tickets(s, z) < s->tail * (s->modes ? SERVE_NRHS : 1);
+}
+
 static int server_launch(sp_server *s) {
   // reset the liveness flags, keep the claim and device counters
   ServeDev z;
   SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
+  z.claim = (unsigned long long)tickets(s, z);
   z.dstop = 0;
   z.dispatcher_gone = 0;
   SP_CUDA_TRY(cudaMemcpyAsync(s->d_dev, &z, sizeof(z), cudaMemcpyHostToDevice, s->stream));
@@ -868,7 +882,7 @@ static int server_keepalive(sp_server *s) {
   if (s->h_ctl->stop) return SP_OK;
   ServeDev z;
   SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
-  if ((long long)z.claim < s->tail * (s->modes ? SERVE_NRHS : 1)) return server_launch(s);
+  if (unclaimed(s, z)) return server_launch(s);
   return SP_OK;
 }
 
@@ -943,7 +957,7 @@ extern "C" int sp_server_stop(sp_server *s) {
   // requests published after the loop saw stop: run them to completion
   ServeDev z;
   SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
-  if ((long long)z.claim < s->tail * (s->modes ? SERVE_NRHS : 1)) {
+  if (unclaimed(s, z)) {
     s->h_ctl->stop = 0;
     SP_TRY(server_launch(s));
     s->h_ctl->stop = 1;

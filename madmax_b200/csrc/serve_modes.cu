@@ -33,21 +33,28 @@ struct ServeShared {
   double rn0;
 };
 
-// claim the next load case (bounded wait, as in serve.cu); one thread
+// Claim the next load case; one thread.  When work is published a CTA takes
+// the next ticket and keeps it: another may have taken the last published one
+// in between, so it waits for its own to be published.  (With a compare-and-
+// swap on the counter the CTAs of the die far from it lost every race: half of
+// them served nothing, and three passes over 6,912 points with n = 12 RVEs took
+// 38.4 ms instead of 17.6 ms.)  The wait ends with the
+// dispatcher, after its last publication; its own bound, 8 times the
+// dispatcher's, is a safeguard.
 __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
   ServeDev *D = P.dev;
-  long long task = -1, idle = 0;
+  long long task = -1, ticket = -1, idle = 0;
   for (;;) {
-    const unsigned long long h = *(volatile unsigned long long *)&D->claim;
+    const bool last = D->dstop || D->dispatcher_gone || ++idle > 8LL * P.idle_limit;
+    __threadfence();
     const long long end = D->dtail * SERVE_NRHS;
-    if ((long long)h < end) {
-      if (atomicCAS(&D->claim, h, h + 1) == h) {
-        task = (long long)h;
-        break;
-      }
-      continue;
+    if (ticket < 0 && (long long)*(volatile unsigned long long *)&D->claim < end)
+      ticket = (long long)atomicAdd(&D->claim, 1ull);
+    if (ticket >= 0 && ticket < end) {
+      task = ticket;
+      break;
     }
-    if (D->dstop || D->dispatcher_gone || ++idle > 8LL * P.idle_limit) break;
+    if (last) break;
     __nanosleep(500);
   }
   __threadfence();
@@ -183,6 +190,7 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
         seen = ht;
         idle = 0;
       } else if (hstop) {
+        __threadfence();  // the last publication first
         if (t == 0) D->dstop = 1;
         break;
       } else if (++idle > P.idle_limit) {
