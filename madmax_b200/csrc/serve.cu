@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
   __shared__ double srn0[SERVE_K];       // right-hand-side norms from the Gram matrix
   __shared__ CgShared sh;
   __shared__ long long s_job;
-  __shared__ int s_geom;
+  __shared__ int s_geom, s_store;
+  __shared__ unsigned s_gen;
   const int t = threadIdx.x;
   ServeDev *D = P.dev;
 
@@ -257,6 +258,10 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
           for (int c = 0; c < SERVE_NRHS; c++) seps[c * 6 + k] = e;
         }
         for (int i = 0; i < 6; i++) seps[(i + 1) * 6 + i] = seps[(i + 1) * 6 + i] + FD_DELTA;
+        if (gid >= 0 && gid < P.ngeom) {
+          s_gen = atomicAdd(&P.geoms[gid].gen, 0u);
+          __threadfence();
+        }
       }
     }
     __syncthreads();
@@ -286,7 +291,10 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
     // (exact for linear materials up to the previous solves' tolerance) for
     // every load case inside; eps . x on the boundary (below)
     const size_t nu = (size_t)SERVE_K * 3 * g.nn_pad;
-    const bool warm = *(volatile int *)&G.has_warm;
+    // The stored solutions' generation is odd while a request writes them; a
+    // start taken from them while it changed may mix two requests and is
+    // dropped for the cold one.
+    bool warm = s_gen > 0 && !(s_gen & 1u);
     if (t < SERVE_K) {
       // ||b(eps_k)||^2 = eps_k^T G eps_k
       double s = 0.0;
@@ -339,6 +347,12 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
       }
     }
     __syncthreads();
+    if (warm && t == 0) {
+      __threadfence();
+      if (atomicAdd(&G.gen, 0u) != s_gen) s_gen = 0;
+    }
+    __syncthreads();
+    warm = warm && s_gen > 0;
     if constexpr (PT)
       stencil_ptable(t, SERVE_NT, sKe, s_ptab);
     else if constexpr (STENCIL)
@@ -377,15 +391,25 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
     // start when it ran a refinement step (they then meet refine_rtol); a
     // request accepted on its prediction leaves the solved state in place,
     // so predictions do not drift from it
-    const bool store = in.outer_its > 0 || !warm || P.warm_last;
-    if (store) {
+    // (one writer at a time: a request that finds another writing stores none)
+    if (t == 0) {
+      s_store = (in.outer_its > 0 || !warm || P.warm_last) && atomicCAS(&G.lock, 0u, 1u) == 0u;
+      if (s_store) atomicAdd(&G.gen, 1u);
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_store) {
       for (size_t i = t; i < nu; i += SERVE_NT) __stcg(G.warm + i, u[i]);
       if (t < SERVE_K * 6) __stcg(G.warm_eps + t, seps[t]);
     }
     __threadfence();
     __syncthreads();
     if (t == 0) {
-      if (store) G.has_warm = 1;
+      if (s_store) {
+        atomicAdd(&G.gen, 1u);
+        __threadfence();
+        atomicExch(&G.lock, 0u);
+      }
       for (int v = 0; v < 6; v++) out->stress[v] = savg[6 + v];
       // c_tangent[j*6 + i] = (stress(eps + d e_i)_j - stress(eps)_j) / (d e_i)
       // (micro/src/homogenize.c:79-80)

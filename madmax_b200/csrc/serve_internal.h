@@ -27,14 +27,14 @@ struct ServeGeom {
   const int *color_elems;
   const uint8_t *slot;
   int color_off[9];
-  int has_warm;
   // element-mode loop (serve_modes.cu)
   double mats[4], len[3];
   int on, cube;      // vectors on chip; equal element edges
   int wlen, pad;
   double *store;     // two stores of ([SERVE_NRHS][3][wlen] fluctuations, [SERVE_NRHS][6] strains)
-  unsigned gen;      // published stores so far; the last one is store gen & 1
-  unsigned lock;     // 1: a request in flight writes the other store
+  unsigned gen;      // published stores so far, the last one in store gen & 1
+                     // (serve.cu's loop: twice the stores, odd while one is written)
+  unsigned lock;     // 1: a request in flight writes a store
 };
 
 struct ServeReq {

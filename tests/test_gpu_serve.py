@@ -309,9 +309,11 @@ def test_serve_classes_match_batch(k):
     s.close()
 
 
-@pytest.mark.parametrize("n,warm", [((6, 6, 6), 0), ((12, 12, 12), 0), ((24, 24, 24), 0),
-                                    ((6, 6, 6), 1)])
-def test_concurrent_cold_requests_on_one_geometry(n, warm):
+@pytest.mark.parametrize("n,warm,opts", [
+    ((6, 6, 6), 0, {}), ((12, 12, 12), 0, {}), ((24, 24, 24), 0, {}), ((6, 6, 6), 1, {}),
+    ((6, 6, 6), 0, {"ctas_per_sm": 2}), ((6, 6, 6), 1, {"op": mb.SP_OP_ELL}),
+    ((5, 5, 33), 0, {})])
+def test_concurrent_cold_requests_on_one_geometry(n, warm, opts):
     """Requests that arrive together on a geometry without a stored solution,
     then again: while one stores its solutions the others start from none or
     from whole ones, never from a mixture."""
@@ -320,7 +322,7 @@ def test_concurrent_cold_requests_on_one_geometry(n, warm):
     rng = np.random.default_rng(3)
     nreq = 12 if n[0] > 12 else 40
     for fresh in range(3):
-        s = mb.Server([d], warm_start=mb.SP_WARM_LAST if warm else mb.SP_WARM_PREDICT)
+        s = mb.Server([d], warm_start=mb.SP_WARM_LAST if warm else mb.SP_WARM_PREDICT, **opts)
         s.start()
         for again in range(3):
             E = rng.normal(0, 1e-3, (nreq, 6))
