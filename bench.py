@@ -59,32 +59,38 @@ def nnz_true(n: int) -> int:
     return 9 * (3 * (n + 1) - 2) ** 3
 
 
-def algorithmic_bytes(sizes, inner_its, outer_its, k=6, stencil=True):
-    """Bytes the batched solve must move per launch.  Per CG iteration: the
-    SpMM input and output vectors, plus, for the assembled operator, the
-    FP32 matrix values (4 B per structural nonzero) and one int32 column node
-    per 3x3 block (the node-sliced ELL stores one per block), or, for the
-    stencil operator, one material byte per element; and 8 FP32 vector
-    passes.  Per refinement step 3 FP64 vector passes, plus one for the
-    residual of the boundary values alone (the right-hand side the stopping
-    rule is relative to; the solve starts from the affine field).  Once per
-    RVE the node-sliced values written (assembled operator) or the stencil's
-    Jacobi diagonal."""
+def algorithmic_bytes(sizes, inner_its, outer_its, k=6):
+    """Bytes the batched solve on assembled values must move per launch.  Per
+    CG iteration: the SpMM input and output vectors, the FP32 matrix values
+    (4 B per structural nonzero) and one int32 column node per 3x3 block (the
+    node-sliced ELL stores one per block); and 8 FP32 vector passes.  Per
+    refinement step 3 FP64 vector passes, plus one for the residual of the
+    boundary values alone (the right-hand side the stopping rule is relative
+    to; the solve starts from the affine field).  Once per RVE the node-sliced
+    values written."""
     total = 0.0
     for n, it, ot in zip(sizes, inner_its, outer_its):
         n, it, ot = int(n), float(it), float(ot)
         ndof = 3 * (n + 1) ** 3
-        nelm = n ** 3
-        if stencil:
-            spmm = nelm + 2 * k * ndof * 4
-            setup = ndof * 4
-        else:
-            spmm = nnz_true(n) * 4 + nnz_true(n) // 9 * 4 + 2 * k * ndof * 4
-            setup = ((n + 1) ** 3 + 31) // 32 * 32 * 243 * 4  # node-sliced values written
+        spmm = nnz_true(n) * 4 + nnz_true(n) // 9 * 4 + 2 * k * ndof * 4
+        setup = ((n + 1) ** 3 + 31) // 32 * 32 * 243 * 4  # node-sliced values written
         vec = 8 * k * ndof * 4
         refine = 3 * k * ndof * 8
         total += it * (spmm + vec) + (ot + 2) * refine + setup
     return total
+
+
+def operator_flops(sizes, inner_its, k=6):
+    """FP32 operations of the operator's products as a 27-point stencil of 3x3
+    blocks (162 a row), the interior rows of every CG iteration of the RVE's
+    longest load case: what the element-mode solve, whose vectors stay on chip
+    and in L2, is measured against."""
+    return sum(k * 3.0 * max(int(n) - 1, 0) ** 3 * 162 * float(it)
+               for n, it in zip(sizes, inner_its))
+
+
+# nominal FP32 rate of one B200: 148 SMs x 128 lanes x 2 x 1.965 GHz
+FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e-3
 
 
 def l2_note(args, sizes, batch):
@@ -110,11 +116,6 @@ def argv_tail(args):
 # bench cannot count DRAM bytes itself, so a run whose workload differs
 # reports null.
 PROFILED_TRAFFIC = {
-    # k_batch, stencil operator, autotuned shape: ncu --metrics dram__bytes_read.sum,
-    # dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
-    # -k regex:k_batch -s 13 -c 1 python bench.py --steps 1 --warmup 3 ...
-    "k_batch --nrve 4096 --sizes 8 12 16 20 --op stencil --threads 0 --ctas 0 "
-    "--inner-rtol 0.003": 663920980224,
     # k_spmv_node, the n = 40 structured matrix, cold L2
     "k_spmv_node structured ELL n=40": 152290000,
 }
@@ -483,6 +484,7 @@ def run_ours(args):
     if dist:
         dist.barrier()
     clocks = sampler.stop()
+    launches = batch.last_launches()  # kernels of one launch
     per_launch_ms = [evs[k].elapsed_time(evs[k + 1]) for k in range(args.steps)]
     total_ms = max_over_ranks(dist, sum(per_launch_ms), "cuda")
     value = whole_job_rate(world, args.nrve, args.steps, total_ms)
@@ -521,11 +523,19 @@ def run_ours(args):
 
     line = None
     if rank == 0:
-        abytes = algorithmic_bytes(sizes, inf["inner"], inf["outer"], stencil=args.op == "stencil")
-        traffic, traffic_src = profiled_traffic("k_batch", " ".join(argv_tail(args)))
+        kernel = "k_batch" if args.op == "ell" else "k_modes"
+        traffic, traffic_src = profiled_traffic(kernel, " ".join(argv_tail(args)))
         avg_ms = total_ms / args.steps
-        achieved = abytes / (avg_ms / 1000.0) / 1e9
-        peak, peak_kind = measured_peak()
+        if args.op == "ell":
+            work = algorithmic_bytes(sizes, inf["inner"], inf["outer"])
+            peak, peak_kind = measured_peak()
+            roof = {"bound": "hbm", "unit": "GB/s", "algorithmic_bytes": work}
+            achieved = work / (avg_ms / 1000.0) / 1e9
+        else:
+            work = operator_flops(sizes, inf["inner"])
+            peak, peak_kind = FP32_PEAK_TFLOPS, "nominal FP32"
+            roof = {"bound": "fp32", "unit": "TFLOP/s", "operator_flops": work}
+            achieved = work / (avg_ms / 1000.0) / 1e12
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": avg_ms,
@@ -541,12 +551,10 @@ def run_ours(args):
                        "parallelism": f"replicas x{world} (independent RVEs per rank)"},
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "gpu_launches": args.steps,
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak,
+            "gpu_launches": args.steps * launches,
+            "roofline": {**roof, "achieved": achieved, "peak": peak, "frac": achieved / peak,
                          "traffic": traffic, "traffic_source": traffic_src,
-                         "algorithmic_bytes": abytes,
-                         "peak_kind": peak_kind, "kernel": "k_batch (persistent)"},
+                         "peak_kind": peak_kind, "kernel": f"{kernel} (persistent)"},
             "clocks": clocks,
             "converged": converged, "max_relres": float(inf["relres"].max()),
             "autotuner": tuned,

@@ -224,7 +224,10 @@ typedef struct {
                         registers per thread) on a sample of the batch at create time and
                         keeps the fastest, cached per device, kernel, precision, load cases
                         and dominant mesh size; SP_TUNE_OFF takes the fixed defaults (512 x 1
-                        for the stencil, 512 x 2 for the assembled operator).  A tuned
+                        for the stencil, 512 x 2 for the assembled operator).  Stencil
+                        solves at 512 x 1 run in element modes, in CTAs chosen by each
+                        RVE's size, where its mesh is in their range (2 to 32 layers, at
+                        most 1024 columns of elements).  A tuned
                         batch's results do not depend on the launch, but the shape -- and so
                         the last bits of the sums -- may depend on the batch's composition;
                         fix threads and ctas_per_sm for bit-identical results across batches */

@@ -409,7 +409,7 @@ def batch_opts(**kw) -> sp_batch_opts:
 
 
 class Batch:
-    """Many RVEs solved by one persistent launch (mixed precision by default)."""
+    """Many RVEs solved per launch (mixed precision by default)."""
 
     def __init__(self, descs, **opts):
         self.n = len(descs)

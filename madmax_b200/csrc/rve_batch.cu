@@ -1,6 +1,11 @@
 // rve_batch.cu -- batched, mixed-precision homogenization of many RVEs in
 // one persistent launch.
 //
+// Stencil batches left to the autotuner or asked for as 512 threads x 1 run in
+// element modes, a load case per CTA (rve_modes_kernel.cuh); what follows
+// holds for the other shapes, the assembled operator, clusters and RVEs beyond
+// the element modes' range.
+//
 // Each CTA takes the next RVE from a work counter (largest meshes first) and
 // runs the whole micro solve of micro/src/homogenize.c:175-225 for all load
 // cases of that RVE on its own:
@@ -215,8 +220,8 @@ struct sp_batch_s {
   size_t bytes = 0;
   TuneRecord tune;  // the autotuner's trial (tune.n == 0: shape fixed by the caller)
   int tune_slots = 0;  // work spaces allocated while the autotuner runs
-  // 512 x 1 stencil: RVEs the element-mode
-  // kernel takes, in one launch per class; `rest` keep k_batch
+  // 512 x 1 stencil: the RVEs that the element-mode kernel takes, in one launch
+  // per class; the others keep k_batch
   std::vector<MeshGeo> geo;      // per RVE
   std::vector<int> cls;          // per RVE: element-mode class or -1
   ModesPlan modes;
@@ -227,7 +232,9 @@ struct sp_batch_s {
   ModesCommon mc;
 };
 
-// the shape whose stencil solves run the element-mode kernel
+// The shape whose stencil solves run the element-mode kernel: the default and
+// the shape the autotuner compares the others with (4096 RVEs of n = 8..20
+// 332 ms in k_batch, 118 ms in element modes).
 static bool uses_modes(const Shape &s) {
   return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op != SP_OP_ELL;
 }

@@ -11,6 +11,17 @@
 // What a CTA runs is the solve of rve_solve.cuh for K = 1: FP64 residual of
 // u = eps.x + w (here marched in element modes too), FP32 Jacobi-PCG
 // corrections as reliable updates, w += x in FP64, volume averages in FP64.
+//
+// What bounds it: the march's serial chain over the planes (a barrier and the
+// shared-memory exchange per plane) with its shuffles and packed FP32 work,
+// ~27,000 cycles an application at n = 20 against ~12,000 of issue slots (n = 16:
+// issue slots 48%, L1 data pipe 64% busy, DRAM idle).  Small
+// RVEs hide it with several CTAs per SM (classes at the end of this file), so
+// a class is as small as threads and shared memory allow.  Measured against
+// the block stencil with all load cases in one CTA: 4096 RVEs of n = 8..20
+// 332 -> 118 ms, 1 RVE of n = 24 with 6 load cases 42 -> 5.5 ms (6 SMs instead
+// of 1), periodic 256 RVEs of n = 9..17 34 -> 4.9 ms, FP64 192 RVEs of n = 8..16
+// 21 -> 4.7 ms, 74 RVEs of n = 32 (no vector on chip) 206 -> 63 ms.
 #pragma once
 
 #include "rve_batch_kernel.cuh"
@@ -90,7 +101,8 @@ struct ModesGeo {
   int nex, ney, nez, nface, mz, h, ntot, per, on, rows;
   __host__ __device__ ModesGeo(int ex, int ey, int ez, bool periodic, bool f64, int onchip)
       : nex(ex), ney(ey), nez(ez), nface(ex * ey), mz(periodic ? ez : ez - 1),
-        h(f64 ? mz : (mz + 1) / 2), ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic), on(onchip), rows(ey) {
+        h(f64 ? mz : (mz + 1) / 2), ntot(h * ex * ey + (periodic ? 0 : ex + 2)), per(periodic),
+        on(onchip), rows(ey) {
     if (on < 2 && !per) {
       const int fit = 16 * wcols() / rowlanes(), n = fit > 0 ? (ey + fit - 1) / fit : 0;
       rows = n > 0 ? (ey + n - 1) / n : 0;
@@ -607,30 +619,30 @@ __device__ __noinline__ int march_average(const double *w, int ph) {
   for (int q = 0; q < 10; q++) m[q] = 0.0;
 #pragma unroll 1
   for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
-  const ModesLane<PER> T(y0);
-  if (T.column) m[9] += (double)__popc(sh.col[T.f] & ~(PER ? (1u | 2u << sh.nez) : 0u));
-  if (T.owner) {
-    const int wl = sh.wlen, mz = sh.mz, nface = sh.nface;
-    int left, down;
-    modes_below<PER>(T.f, left, down);
-    const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f + left], c1 = sh.col[T.f + down],
-                   c0 = sh.col[T.f + left + down];
-#pragma unroll 4
-    for (int pl = 0; pl < mz; pl++) {
-      const unsigned b0 = (c0 >> pl) & 3u, b1 = (c1 >> pl) & 3u, b2 = (c2 >> pl) & 3u,
-                     b3 = (c3 >> pl) & 3u;
-      const int n0 = __popc(b0), n1 = __popc(b1), n2 = __popc(b2), n3 = __popc(b3);
-      const int lower = (b0 & 1) + (b1 & 1) + (b2 & 1) + (b3 & 1);
-      const double k[3] = {(double)(n0 + n2 - n1 - n3), (double)(n0 + n1 - n2 - n3),
-                           (double)(2 * lower - (n0 + n1 + n2 + n3))};
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const double v = w[c * wl + pl * nface + T.f];
-#pragma unroll
-        for (int d = 0; d < 3; d++) m[3 * c + d] = fma(k[d], v, m[3 * c + d]);
+    const ModesLane<PER> T(y0);
+    if (T.column) m[9] += (double)__popc(sh.col[T.f] & ~(PER ? (1u | 2u << sh.nez) : 0u));
+    if (T.owner) {
+      const int wl = sh.wlen, mz = sh.mz, nface = sh.nface;
+      int left, down;
+      modes_below<PER>(T.f, left, down);
+      const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f + left], c1 = sh.col[T.f + down],
+                     c0 = sh.col[T.f + left + down];
+  #pragma unroll 4
+      for (int pl = 0; pl < mz; pl++) {
+        const unsigned b0 = (c0 >> pl) & 3u, b1 = (c1 >> pl) & 3u, b2 = (c2 >> pl) & 3u,
+                       b3 = (c3 >> pl) & 3u;
+        const int n0 = __popc(b0), n1 = __popc(b1), n2 = __popc(b2), n3 = __popc(b3);
+        const int lower = (b0 & 1) + (b1 & 1) + (b2 & 1) + (b3 & 1);
+        const double k[3] = {(double)(n0 + n2 - n1 - n3), (double)(n0 + n1 - n2 - n3),
+                             (double)(2 * lower - (n0 + n1 + n2 + n3))};
+  #pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double v = w[c * wl + pl * nface + T.f];
+  #pragma unroll
+          for (int d = 0; d < 3; d++) m[3 * c + d] = fma(k[d], v, m[3 * c + d]);
+        }
       }
     }
-  }
   }
   cta_sum<10>(m, ph);
   __syncthreads();
@@ -790,29 +802,29 @@ __device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, doub
   const int nface = sh.nface, ntot = sh.ntot, h = sh.h, mz = sh.mz, wl = sh.wlen;
 #pragma unroll 1
   for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
-  const ModesLane<PER> T(y0);
-  if (!T.owner) continue;
-#pragma unroll 1
-  for (int s = 0; s < h; s++) {
-    const int i = s * nface + T.f;
-    V x[3];
-    double w0[3], w1[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      x[c] = ModesType<V>::ld(xg + (c * ntot + i));
-      w0[c] = w[c * wl + i];
-      w1[c] = s + h < mz ? w[c * wl + i + h * nface] : 0.0;
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      if constexpr (ModesType<V>::F64) {
-        w[c * wl + i] = w0[c] + x[c];
-      } else {
-        w[c * wl + i] = w0[c] + (double)x[c].v.x;
-        if (s + h < mz) w[c * wl + i + h * nface] = w1[c] + (double)x[c].v.y;
+    const ModesLane<PER> T(y0);
+    if (!T.owner) continue;
+  #pragma unroll 1
+    for (int s = 0; s < h; s++) {
+      const int i = s * nface + T.f;
+      V x[3];
+      double w0[3], w1[3];
+  #pragma unroll
+      for (int c = 0; c < 3; c++) {
+        x[c] = ModesType<V>::ld(xg + (c * ntot + i));
+        w0[c] = w[c * wl + i];
+        w1[c] = s + h < mz ? w[c * wl + i + h * nface] : 0.0;
+      }
+  #pragma unroll
+      for (int c = 0; c < 3; c++) {
+        if constexpr (ModesType<V>::F64) {
+          w[c * wl + i] = w0[c] + x[c];
+        } else {
+          w[c * wl + i] = w0[c] + (double)x[c].v.x;
+          if (s + h < mz) w[c * wl + i + h * nface] = w1[c] + (double)x[c].v.y;
+        }
       }
     }
-  }
   }
 }
 
@@ -915,28 +927,28 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
   // right-hand side's own residual, w = -eps.x inside, i.e. u = 0 inside
 #pragma unroll 1
   for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
-  const ModesLane<PER> T(y0);
-  if (T.owner) {
-    int left, down;
-    modes_below<PER>(T.f, left, down);
-    const unsigned m0 = sh.col[T.f], m1 = sh.col[T.f + left], m2 = sh.col[T.f + down],
-                   m3 = sh.col[T.f + left + down];
-    auto count = [&](int pl) {
-      return __popc(shr32(m0, pl) & 3u) + __popc(shr32(m1, pl) & 3u) + __popc(shr32(m2, pl) & 3u) +
-             __popc(shr32(m3, pl) & 3u);
-    };
-    for (int s = 0; s < sh.h; s++)
-      mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (F64 ? 0 : count(s + sh.h) << 4));
-    const double X = (T.f % nex) * sh.hx[0], Y = (T.f / nex) * sh.hx[1];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const double xy = sh.E[3 * c] * X + sh.E[3 * c + 1] * Y, ez = sh.E[3 * c + 2] * sh.hx[2];
-      if (!PER)
-        for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
-      // a slot without an upper plane keeps a zero there
-      static_cast<float2 *>(rv)[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
+    const ModesLane<PER> T(y0);
+    if (T.owner) {
+      int left, down;
+      modes_below<PER>(T.f, left, down);
+      const unsigned m0 = sh.col[T.f], m1 = sh.col[T.f + left], m2 = sh.col[T.f + down],
+                     m3 = sh.col[T.f + left + down];
+      auto count = [&](int pl) {
+        return __popc(shr32(m0, pl) & 3u) + __popc(shr32(m1, pl) & 3u) + __popc(shr32(m2, pl) & 3u) +
+               __popc(shr32(m3, pl) & 3u);
+      };
+      for (int s = 0; s < sh.h; s++)
+        mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (F64 ? 0 : count(s + sh.h) << 4));
+      const double X = (T.f % nex) * sh.hx[0], Y = (T.f / nex) * sh.hx[1];
+  #pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const double xy = sh.E[3 * c] * X + sh.E[3 * c + 1] * Y, ez = sh.E[3 * c + 2] * sh.hx[2];
+        if (!PER)
+          for (int pl = 0; pl < sh.mz; pl++) w[c * wl + pl * nface + T.f] = -(xy + ez * (pl + 1));
+        // a slot without an upper plane keeps a zero there
+        static_cast<float2 *>(rv)[c * sh.ntot + (sh.h - 1) * nface + T.f] = make_float2(0.f, 0.f);
+      }
     }
-  }
   }
   __syncthreads();
   if (t < 2) {
