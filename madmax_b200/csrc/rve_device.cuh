@@ -270,60 +270,6 @@ __device__ inline void affine_boundary(int t, int nt, const MeshGeo &g, const do
   }
 }
 
-// ------------------------------------------------- FP64 element residual ---
-
-// Newton right-hand side b = -K u on interior dofs, 0 on boundary dofs
-// (micro/src/assembly.c:33-82 then negative_res, micro/src/homogenize.c:
-// 289-303): one thread per dof row sums, over the (up to 8) elements of the
-// row's node, Ke_t[row][:] u_e.  For linear elastic elements Ke_t u_e =
-// sum_gp B^T sigma(B u_e) w exactly.  Writes b into rb (type R) and adds
-// |b|^2 per load case into nrm2[K].
-template <int K, typename R>
-__device__ inline void residual_nodes(int t, int nt, const MeshGeo &g,
-                                      const uint8_t *__restrict__ etype,
-                                      const double *Ke /*[2][576], shared*/,
-                                      const double *__restrict__ u, R *rb, double *nrm2) {
-  for (int row = t; row < g.ndof; row += nt) {
-    int node = row / 3, d = row % 3;
-    int i = node % g.nx, j = (node / g.nx) % g.ny, k = node / (g.nx * g.ny);
-    double acc[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) acc[q] = 0.0;
-    bool bnd = (i == 0 || j == 0 || k == 0 || i == g.nx - 1 || j == g.ny - 1 || k == g.nz - 1);
-    if (!bnd) {
-      // interior node: all 8 surrounding elements exist
-#pragma unroll 1
-      for (int c = 0; c < 8; c++) {
-        int ox = (c & 1), oy = (c >> 1) & 1, oz = c >> 2;
-        int ex = i - 1 + ox, ey = j - 1 + oy, ez = k - 1 + oz;
-        int e = ex + ey * g.nex + ez * g.nex * g.ney;
-        // local index of this node in element e: corner (1-ox, 1-oy, 1-oz)
-        int cx = 1 - ox, cy = 1 - oy, cz = 1 - oz;
-        int la = cz * 4 + ((cy == 0) ? (cx ? 1 : 0) : (cx ? 2 : 3));
-        const double *ke = Ke + etype[e] * SP_KE + (la * 3 + d) * SP_NC;
-        int n0 = ex + ey * g.nx + ez * g.nx * g.ny;
-#pragma unroll 2
-        for (int b = 0; b < 8; b++) {
-          int nb = n0 + corner_x(b) + corner_y(b) * g.nx + corner_z(b) * g.nx * g.ny;
-          const double *ub = u + (size_t)nb * 3 * K;
-#pragma unroll
-          for (int db = 0; db < 3; db++) {
-            double kv = ke[b * 3 + db];
-#pragma unroll
-            for (int q = 0; q < K; q++) acc[q] = fma(kv, ub[db * K + q], acc[q]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < K; q++) {
-      double b = -acc[q];
-      rb[(size_t)row * K + q] = (R)b;
-      nrm2[q] += b * b;
-    }
-  }
-}
-
 // --------------------------------------------------------------- SpMM ---
 
 // Load the K values of one dof.  NC: the data is read-only for the whole
@@ -1710,7 +1656,7 @@ __device__ inline void average_per(int t, int nt, const MeshGeo &g,
 }
 
 // b = -K u on interior dofs, 0 on the boundary and on padding (component-
-// major vectors; see residual_nodes for the arithmetic).  BCONLY: u's
+// major vectors; k_residual in rve_plain.cu has the same arithmetic).  BCONLY: u's
 // interior values are read as 0, giving the right-hand side -K u_bc of the
 // load cases.  SCALE: also adds, per load case, the squared norm of the rows'
 // sums of term magnitudes into scale2[K] (the size below which b is

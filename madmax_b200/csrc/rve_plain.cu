@@ -53,7 +53,11 @@ __global__ void k_affine(MeshGeo g, const double *eps, int nrhs, double *u, bool
                  inside);
 }
 
-// b = -K u (interior), 0 (boundary); norms[k] = ||b_k||^2.  A thread per
+// Newton right-hand side b = -K u on interior dofs, 0 on boundary dofs
+// (micro/src/assembly.c:33-82 then negative_res, micro/src/homogenize.c:
+// 289-303), as the sum over the elements of the row's node of Ke_t[row][:] u_e
+// (for linear elastic elements sum_gp B^T sigma(B u_e) w exactly);
+// norms[k] = ||b_k||^2.  A thread per
 // (row, load case), load cases fastest: a thread per row, with the K sums in
 // registers, left 27,783 threads for n = 20 and waited on its loads (76 us,
 // 6 load cases).
