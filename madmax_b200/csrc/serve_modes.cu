@@ -40,14 +40,17 @@ struct ServeShared {
 // them served nothing, and three passes over 6,912 points with n = 12 RVEs took
 // 38.4 ms instead of 17.6 ms.)  The wait ends with the
 // dispatcher, after its last publication; its own bound, 8 times the
-// dispatcher's, is a safeguard.
+// dispatcher's since the last publication, is a safeguard (a ticket given up
+// while the dispatcher runs would leave its load case unsolved).
 __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
   ServeDev *D = P.dev;
-  long long task = -1, ticket = -1, idle = 0;
+  long long task = -1, ticket = -1, idle = 0, seen = -1;
   for (;;) {
     const bool last = D->dstop || D->dispatcher_gone || ++idle > 8LL * P.idle_limit;
     __threadfence();
     const long long end = D->dtail * SERVE_NRHS;
+    if (end != seen) idle = 0;
+    seen = end;
     if (ticket < 0 && (long long)*(volatile unsigned long long *)&D->claim < end)
       ticket = (long long)atomicAdd(&D->claim, 1ull);
     if (ticket >= 0 && ticket < end) {

@@ -335,3 +335,29 @@ def test_concurrent_cold_requests_on_one_geometry(n, warm, opts):
                 assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
         s.stop()
         s.close()
+
+
+def test_slow_requests_after_a_burst():
+    """CTAs that took tickets past the end of a burst keep them while requests
+    come one by one, for many times the idle limit in all, and across a loop
+    that left and was relaunched: every request is answered."""
+    d = mode_desc((6, 6, 6), 1)
+    Cm = exact_tangents([d])[0]
+    rng = np.random.default_rng(9)
+    s = mb.Server([d], idle_spin_limit=2000)
+    s.start()
+
+    def ask(n):
+        E = rng.normal(0, 1e-3, (n, 6))
+        for t, e in [(s.submit(0, e), e) for e in E]:
+            st, _, info = s.wait(t)
+            ref = Cm @ e
+            assert info.status == 0 and np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+
+    for gap in (0.0, 5e-4, 2e-3, 3e-2):
+        ask(300)
+        for _ in range(60 if gap < 1e-2 else 5):
+            time.sleep(gap)
+            ask(1)
+    s.stop()
+    s.close()
