@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
       double s = 0.0;
       for (int a = 0; a < 6; a++)
         for (int c = 0; c < 6; c++) s += seps[t * 6 + a] * __ldg(G.gram + a * 6 + c) * seps[t * 6 + c];
-      srn0[t] = sqrt(fmax(s, 0.0));
+      srn0[t] = s <= 0.0 ? 0.0 : sqrt(s);  // (a NaN stays one)
     }
     if (warm && P.warm_last) {
       // the last request's solution of each load case, shifted by the affine
@@ -390,10 +390,21 @@ __global__ void __launch_bounds__(SERVE_NT, MINB) k_serve(ServeParams P) {
     // keep this request's solutions and strains as the geometry's next warm
     // start when it ran a refinement step (they then meet refine_rtol); a
     // request accepted on its prediction leaves the solved state in place,
-    // so predictions do not drift from it
+    // so predictions do not drift from it; one with a load case no nearer than
+    // a cold start (a residual of 1) or not a number is no start for the next
     // (one writer at a time: a request that finds another writing stores none)
     if (t == 0) {
-      s_store = (in.outer_its > 0 || !warm || P.warm_last) && atomicCAS(&G.lock, 0u, 1u) == 0u;
+      bool near = true, number = true;
+      for (int k = 0; k < SERVE_NRHS; k++) {
+        number = number && isfinite(srn0[k]) && isfinite(sh.rn[k]);
+        near = near && (sh.rn[k] < srn0[k] || !(srn0[k] > 0.0));
+      }
+      if (!number) {
+        in.status = SP_ERR_NOCONV;
+        in.relres = nan("");
+      }
+      s_store = (in.outer_its > 0 || !warm || P.warm_last) && near && number &&
+                atomicCAS(&G.lock, 0u, 1u) == 0u;
       if (s_store) atomicAdd(&G.gen, 1u);
       __threadfence();
     }

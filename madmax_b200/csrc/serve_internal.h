@@ -69,7 +69,7 @@ struct ServeJob {
   unsigned stored;  // load cases written to the geometry's other store
   unsigned writer;  // 1: this request holds the geometry's lock; 0: undecided
   int status, outer, inner;
-  unsigned long long relres;  // bits of the largest (non-negative) one
+  unsigned long long relres;  // bits of the largest one (non-negative or NaN)
   double stress[SERVE_NRHS][6];
 };
 

@@ -81,7 +81,7 @@ __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
   double s = 0.0;
   for (int a = 0; a < 6; a++)
     for (int b = 0; b < 6; b++) s += e[a] * __ldg(G.gram + a * 6 + b) * e[b];
-  S.rn0 = sqrt(fmax(s, 0.0));
+  S.rn0 = s <= 0.0 ? 0.0 : sqrt(s);  // (a NaN stays one)
   if (S.gen) {
     const double *se = G.store + (size_t)(S.gen & 1) * SERVE_NRHS * (3 * G.wlen + 6) +
                        (size_t)SERVE_NRHS * 3 * G.wlen;
@@ -130,7 +130,9 @@ __device__ __noinline__ void serve_start(const ServeGeom &G, ServeShared &S, boo
   __syncthreads();
 }
 
-// one load case; thread 0 writes its stress average
+// one load case; thread 0 writes its stress average.  Returns its relative
+// residual, NaN for a strain without a finite right-hand side (which is left
+// without a step).
 template <bool CUBE, int ON>
 __device__ __noinline__ double serve_case(const ServeModes &P, const ServeGeom &G, ServeShared &S,
                                           double *stress) {
@@ -152,7 +154,7 @@ __device__ __noinline__ double serve_case(const ServeModes &P, const ServeGeom &
     march_average<false>(ws.w, ph);
   }
   if (threadIdx.x == 0) modes_output(sh.red, stress, nullptr);
-  return relres;
+  return isfinite(S.rn0) ? relres : nan("");
 }
 
 template <int NT, int MINB>
@@ -234,10 +236,11 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
       // keep this load case's solution for the geometry's next requests when
       // it was solved (it then meets the refined tolerance); one accepted on
       // its prediction leaves the solved state in place, so predictions do
-      // not drift from it
+      // not drift from it.  One that is no nearer than a cold start (a residual
+      // of 1) or not a number is no start for the next.
       if (t == 0)
         S.stored = (msh().outer > 0 || !(S.rn0 > 0.0) || S.gen == 0 || P.warm_last) &&
-                   atomicAdd(&J.writer, 0u) == 1u;
+                   relres < 1.0 && atomicAdd(&J.writer, 0u) == 1u;
       if (t == 0) __threadfence();
       __syncthreads();
       if (S.stored) {
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
         atomicMax(&J.status, status);
         atomicMax(&J.outer, msh().outer);
         atomicMax(&J.inner, msh().inner);
-        atomicMax(&J.relres, (unsigned long long)__double_as_longlong(fmax(relres, 0.0)));
+        // (bits of a non-negative number grow with it, and NaN's are above all)
+        atomicMax(&J.relres, (unsigned long long)__double_as_longlong(relres >= 0.0 ? relres : nan("")));
         if (S.stored) atomicAdd(&J.stored, 1u);
       } else {
         atomicMax(&J.status, SP_ERR_RANGE);

@@ -361,3 +361,31 @@ def test_slow_requests_after_a_burst():
             ask(1)
     s.stop()
     s.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("warm", [mb.SP_WARM_PREDICT, mb.SP_WARM_LAST])
+@pytest.mark.parametrize("opts", [{}, {"ctas_per_sm": 2}, {"op": mb.SP_OP_ELL}])
+def test_non_finite_request_does_not_outlast_its_answer(opts, warm, bad):
+    """A request with a non-finite strain, on a geometry without and with a
+    stored solution, is answered as not converged; the requests after it on the
+    same geometry are solved as if it had not been there."""
+    d = mode_desc((6, 6, 6), 1)
+    Cm = exact_tangents([d])[0]
+    rng = np.random.default_rng(4)
+    s = mb.Server([d], warm_start=warm, **opts)
+    s.start()
+    for k in range(3):
+        e = rng.normal(0, 1e-3, 6)
+        e[(1, 3, 0)[k]] = bad
+        info = s.wait(s.submit(0, e))[2]
+        assert info.status == mb.SP_ERR_NOCONV and np.isnan(info.relres)
+        for _ in range(2):
+            e = rng.normal(0, 1e-3, 6)
+            st, tg, info = s.wait(s.submit(0, e))
+            assert info.status == 0 and info.relres <= 1e-8
+            ref = Cm @ e
+            assert np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+            assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
+    s.stop()
+    s.close()
