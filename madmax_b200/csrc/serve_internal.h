@@ -66,7 +66,10 @@ struct ServeDev { // device memory
 // A request in the element-mode loop: its load cases are tasks of their own
 struct ServeJob {
   unsigned left;    // load cases still to finish
-  unsigned stored;  // load cases written to the geometry's other store
+  unsigned stored;  // bit k: load case k is in the geometry's other store
+  unsigned met;     // bit k: ... met the tolerance as predicted from store gen[k]
+  unsigned solved;  // load cases kept for more than their prediction
+  unsigned gen[SERVE_NRHS];
   unsigned writer;  // 1: this request holds the geometry's lock; 0: undecided
   int status, outer, inner;
   unsigned long long relres;  // bits of the largest one (non-negative or NaN)

@@ -11,7 +11,11 @@
 // Stores.  A geometry has two: the published one and the one being written.
 // A request takes the geometry's lock when its first load case is claimed;
 // without it, it stores nothing.  Its solutions go to the other store and are
-// published (gen + 1) once all 7 are there.  A task that read the published
+// published (gen + 1) once all 7 are there.  Where some load cases were solved
+// and others met the tolerance on their prediction, the request's last task
+// adds the predictions, formed again from the published store, which stands
+// as long as the lock is held; a request that met all of its predictions
+// publishes nothing.  A task that read the published
 // store while a later request's solutions replaced it (gen has moved on)
 // starts cold instead, so no task starts from a mixture of two requests.
 // Nothing waits: a lock that is taken is passed by.
@@ -28,10 +32,35 @@ namespace sp {
 struct ServeShared {
   long long req;  // ticket, -1: leave
   int geom, k, gen, stored;
+  int last;       // the request's last task: 1, and 2 to publish its solutions
+  unsigned fill;  // ... after adding the predictions of these load cases
   double eps[SERVE_NRHS][6];
   double c[6];  // prediction coefficients
   double rn0;
 };
+
+// first-order prediction of a load case of strain e from the solutions w_k of
+// a store's strains: w = w_0 + sum_j c_j (w_j+1 - w_0)
+__device__ __forceinline__ const double *serve_store(const ServeGeom &G, unsigned gen) {
+  return G.store + (size_t)(gen & 1u) * SERVE_NRHS * (3 * G.wlen + 6);
+}
+__device__ __noinline__ void serve_coefs(const ServeGeom &G, unsigned gen, const double *e, double *c) {
+  const double *se = serve_store(G, gen) + (size_t)SERVE_NRHS * 3 * G.wlen;
+  for (int j = 0; j < 6; j++) {
+    const double b = __ldcg(se + j), d = __ldcg(se + (j + 1) * 6 + j) - b;
+    c[j] = d != 0.0 ? (e[j] - b) / d : 0.0;
+  }
+}
+__device__ __forceinline__ double serve_predict(const double *st, int n, const double (&c)[6], int i) {
+  const double w0 = __ldcg(st + i);
+  double v[6];
+#pragma unroll
+  for (int j = 0; j < 6; j++) v[j] = __ldcg(st + (size_t)(j + 1) * n + i);
+  double s = w0;
+#pragma unroll
+  for (int j = 0; j < 6; j++) s = fma(c[j], v[j] - w0, s);
+  return s;
+}
 
 // Claim the next load case; one thread.  When work is published a CTA takes
 // the next ticket and keeps it: another may have taken the last published one
@@ -82,14 +111,21 @@ __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
   for (int a = 0; a < 6; a++)
     for (int b = 0; b < 6; b++) s += e[a] * __ldg(G.gram + a * 6 + b) * e[b];
   S.rn0 = s <= 0.0 ? 0.0 : sqrt(s);  // (a NaN stays one)
-  if (S.gen) {
-    const double *se = G.store + (size_t)(S.gen & 1) * SERVE_NRHS * (3 * G.wlen + 6) +
-                       (size_t)SERVE_NRHS * 3 * G.wlen;
-    for (int j = 0; j < 6; j++) {
-      const double b = __ldcg(se + j), d = __ldcg(se + (j + 1) * 6 + j) - b;
-      S.c[j] = d != 0.0 ? (e[j] - b) / d : 0.0;
-    }
-  }
+  if (S.gen) serve_coefs(G, S.gen, e, S.c);
+}
+
+// whether the request's last task publishes its solutions, and the load cases
+// whose predictions belong to them; one thread
+__device__ __noinline__ void serve_finish(ServeJob &J, ServeGeom &G, ServeShared &S) {
+  if (atomicAdd(&J.writer, 0u) != 1u || atomicAdd(&J.solved, 0u) == 0u) return;
+  const unsigned gen = atomicAdd(&G.gen, 0u), stored = atomicAdd(&J.stored, 0u),
+                 met = atomicAdd(&J.met, 0u) & ~stored;
+  for (int k = 0; k < SERVE_NRHS; k++)
+    if ((met >> k & 1u) && *(volatile unsigned *)(J.gen + k) == gen) S.fill |= 1u << k;
+  if ((stored | S.fill) == (1u << SERVE_NRHS) - 1)
+    S.last = 2;
+  else
+    S.fill = 0;
 }
 
 // the start iterate: the fluctuation of the last solution of this load case
@@ -99,23 +135,14 @@ __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
 __device__ __noinline__ void serve_start(const ServeGeom &G, ServeShared &S, bool last, double *w) {
   if (!(S.rn0 > 0.0)) return;
   const int n = 3 * G.wlen, t = threadIdx.x;
-  const double *st = G.store + (size_t)(S.gen & 1) * SERVE_NRHS * (n + 6);
+  const double *st = serve_store(G, S.gen);
   if (S.gen && last) {
     for (int i = t; i < n; i += blockDim.x) w[i] = __ldcg(st + (size_t)S.k * n + i);
   } else if (S.gen) {
     double c[6];
 #pragma unroll
     for (int j = 0; j < 6; j++) c[j] = S.c[j];
-    for (int i = t; i < n; i += blockDim.x) {
-      const double w0 = __ldcg(st + i);
-      double v[6];
-#pragma unroll
-      for (int j = 0; j < 6; j++) v[j] = __ldcg(st + (size_t)(j + 1) * n + i);
-      double s = w0;
-#pragma unroll
-      for (int j = 0; j < 6; j++) s = fma(c[j], v[j] - w0, s);
-      w[i] = s;
-    }
+    for (int i = t; i < n; i += blockDim.x) w[i] = serve_predict(st, n, c, i);
   }
   __syncthreads();
   if (S.gen) {
@@ -127,6 +154,25 @@ __device__ __noinline__ void serve_start(const ServeGeom &G, ServeShared &S, boo
   }
   if (!S.gen)
     for (int i = t; i < n; i += blockDim.x) w[i] = 0.0;
+  __syncthreads();
+}
+
+// the predictions of the load cases S.fill into the store being written
+__device__ __noinline__ void serve_fill(ServeGeom &G, const ServeShared &S) {
+  const int n = 3 * G.wlen, t = threadIdx.x;
+  const unsigned gen = atomicAdd(&G.gen, 0u);
+  const double *from = serve_store(G, gen);
+  double *to = const_cast<double *>(serve_store(G, gen + 1));
+#pragma unroll 1
+  for (int k = 0; k < SERVE_NRHS; k++) {
+    if (!(S.fill >> k & 1u)) continue;
+    double c[6];
+    serve_coefs(G, gen, S.eps[k], c);
+    for (int i = t; i < n; i += blockDim.x)
+      __stcg(to + (size_t)k * n + i, serve_predict(from, n, c, i));
+    if (t < 6) __stcg(to + (size_t)SERVE_NRHS * n + k * 6 + t, S.eps[k][t]);
+  }
+  __threadfence();
   __syncthreads();
 }
 
@@ -185,7 +231,7 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
           for (int k = 0; k < 6; k++) dst->strain[k] = src->strain[k];
           ServeJob &J = P.jobs[i % P.cap];
           J.left = SERVE_NRHS;
-          J.stored = J.writer = 0;
+          J.stored = J.met = J.solved = J.writer = 0;
           J.status = J.outer = J.inner = 0;
           J.relres = 0;
         }
@@ -238,14 +284,20 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
       // its prediction leaves the solved state in place, so predictions do
       // not drift from it.  One that is no nearer than a cold start (a residual
       // of 1) or not a number is no start for the next.
-      if (t == 0)
-        S.stored = (msh().outer > 0 || !(S.rn0 > 0.0) || S.gen == 0 || P.warm_last) &&
-                   relres < 1.0 && atomicAdd(&J.writer, 0u) == 1u;
+      if (t == 0) {
+        const bool solved = msh().outer > 0 || S.gen == 0 || P.warm_last;
+        S.stored = (solved || !(S.rn0 > 0.0)) && relres < 1.0 && atomicAdd(&J.writer, 0u) == 1u;
+        if (S.stored && solved) atomicAdd(&J.solved, 1u);
+        if (!solved && S.rn0 > 0.0 && relres <= P.lim.rtol) {
+          J.gen[S.k] = (unsigned)S.gen;  // (fenced before left counts down)
+          atomicOr(&J.met, 1u << S.k);
+        }
+      }
       if (t == 0) __threadfence();
       __syncthreads();
       if (S.stored) {
         const int n = 3 * G.wlen;
-        double *st = G.store + (size_t)((atomicAdd(&G.gen, 0u) + 1) & 1) * SERVE_NRHS * (n + 6);
+        double *st = const_cast<double *>(serve_store(G, atomicAdd(&G.gen, 0u) + 1));
         const double *w = P.buf.ws_w + (size_t)blockIdx.x * P.buf.w_stride;
         for (int i = t; i < n; i += blockDim.x) __stcg(st + (size_t)S.k * n + i, w[i]);
         if (t < 6) __stcg(st + (size_t)SERVE_NRHS * n + S.k * 6 + t, S.eps[S.k][t]);
@@ -261,12 +313,22 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
         atomicMax(&J.inner, msh().inner);
         // (bits of a non-negative number grow with it, and NaN's are above all)
         atomicMax(&J.relres, (unsigned long long)__double_as_longlong(relres >= 0.0 ? relres : nan("")));
-        if (S.stored) atomicAdd(&J.stored, 1u);
+        if (S.stored) atomicOr(&J.stored, 1u << S.k);
       } else {
         atomicMax(&J.status, SP_ERR_RANGE);
       }
       __threadfence();
-      if (atomicSub(&J.left, 1u) == 1u) {
+      S.last = atomicSub(&J.left, 1u) == 1u;
+      S.fill = 0;
+      if (S.last && known) {
+        __threadfence();
+        serve_finish(J, P.geoms[S.geom], S);
+      }
+    }
+    __syncthreads();
+    if (S.last) {
+      if (S.fill) serve_fill(P.geoms[S.geom], S);
+      if (t == 0) {
         __threadfence();
         ServeRes *out = P.res + (S.req % P.cap);
         if (known) {
@@ -279,7 +341,7 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
             for (int j = 0; j < 6; j++)
               out->tangent[j * 6 + i] = (st[i + 1][j] - st[0][j]) / (S.eps[i + 1][i] - S.eps[0][i]);
           if (atomicAdd(&J.writer, 0u) == 1u) {
-            if (atomicAdd(&J.stored, 0u) == SERVE_NRHS) atomicAdd(&G.gen, 1u);
+            if (S.last == 2) atomicAdd(&G.gen, 1u);
             __threadfence();
             atomicExch(&G.lock, 0u);
           }

@@ -389,3 +389,29 @@ def test_non_finite_request_does_not_outlast_its_answer(opts, warm, bad):
             assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
     s.stop()
     s.close()
+
+
+@pytest.mark.parametrize("n", [(6, 6, 6), (12, 12, 12), (24, 24, 24)])
+def test_request_that_misses_in_some_load_cases_is_kept(n):
+    """A base strain far below the stored one: its load case misses the
+    prediction, the six of eps + 0.005 e_i meet it.  The request's solutions
+    become the geometry's store all the same, so that later requests of that
+    size are predicted."""
+    d = mode_desc(n, 1)
+    Cm = exact_tangents([d])[0]
+    rng = np.random.default_rng(6)
+    s = mb.Server([d])
+    s.start()
+    big, small = rng.normal(0, 1e-3, 6), rng.normal(0, 1e-9, 6)
+    first = s.wait(s.submit(0, big))[2]
+    second = s.wait(s.submit(0, small))[2]
+    assert first.inner_its > second.inner_its > 0
+    for _ in range(3):
+        e = small * rng.uniform(0.9, 1.1)
+        st, tg, info = s.wait(s.submit(0, e))
+        assert info.status == 0 and info.inner_its == 0
+        ref = Cm @ e
+        assert np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+        assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
+    s.stop()
+    s.close()
