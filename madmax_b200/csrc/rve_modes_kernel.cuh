@@ -170,7 +170,9 @@ __device__ __forceinline__ V *mq() {
 }
 __device__ __forceinline__ uint8_t *mcnt() { return mp<uint8_t>() + msh().cntoff; }
 
-// FP32 pairs or FP64 values: their memory type and the type of their scalars
+// FP32 pairs or FP64 values: their memory type and the type of their scalars.
+// dot: the product(s) of a and b, formed and added in FP64 -- squares of FP32
+// residuals leave FP32's range where the residuals do not.
 template <typename V>
 struct ModesType;
 template <>
@@ -182,7 +184,16 @@ struct ModesType<F2> {
   __device__ static void st(float2 *a, F2 v) { __stcg(a, v.v); }
   __device__ static void add(float2 *a, F2 v) { atomicAdd(a, v.v); }
   __device__ static F2 splat(float s) { return mk2(s, s); }
-  __device__ static double sum(F2 v) { return (double)(v.v.x + v.v.y); }
+  __device__ static double dot(F2 a, F2 b) {
+    return fma((double)a.v.y, (double)b.v.y, (double)a.v.x * (double)b.v.x);
+  }
+  // sums of the squares of a[0..2], of the lower and of the upper planes
+  __device__ static void squares(const F2 (&a)[3], double (&s)[2]) {
+    const double x0 = a[0].v.x, x1 = a[1].v.x, x2 = a[2].v.x;
+    const double y0 = a[0].v.y, y1 = a[1].v.y, y2 = a[2].v.y;
+    s[0] = x0 * x0 + x1 * x1 + x2 * x2;
+    s[1] = y0 * y0 + y1 * y1 + y2 * y2;
+  }
 };
 template <>
 struct ModesType<double> {
@@ -193,7 +204,11 @@ struct ModesType<double> {
   __device__ static void st(double *a, double v) { __stcg(a, v); }
   __device__ static void add(double *a, double v) { atomicAdd(a, v); }
   __device__ static double splat(double s) { return s; }
-  __device__ static double sum(double v) { return v; }
+  __device__ static double dot(double a, double b) { return a * b; }
+  __device__ static void squares(const double (&a)[3], double (&s)[2]) {
+    s[0] = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+    s[1] = 0.0;
+  }
 };
 
 // Sum NV doubles over the CTA in a fixed order; every thread gets the
@@ -426,7 +441,7 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg, const
         V *const e = qf + (QS ? (s - 1) : (s & 1)) * ex3;
         const bool seam = STRIPS && T.f0 > 0 && T.f < T.f0 + sh.nex;
         const V *ps = pf + (s - 1) * nf3;
-        V t = zero_of(V());
+        double t[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           low[c] = low[c] + (seam ? edge[c] : e[c]);
@@ -440,9 +455,9 @@ __device__ __noinline__ double march_apply(typename ModesType<V>::Mem *qg, const
             e[c] = low[c];
           else
             MT::st(qg + (size_t)c * ntot + (s - 1) * nface + T.f, low[c]);
-          t = mad(low[c], ps[c], t);
+          t[c] = MT::dot(low[c], ps[c]);
         }
-        pq += MT::sum(t);
+        pq += t[0] + t[1] + t[2];
       }
     }
   };
@@ -699,25 +714,32 @@ __device__ __forceinline__ void xr_slots(int s0, int f, const V *pg, typename Mo
   for (int j = 0; j < U; j++) {
     if (s0 + j >= h) break;
     const int i = (s0 + j) * nface + f;
-    V dz[3];
-    slot_dinv<CUBE>(i, dz);
-    V sz = zero_of(V()), sr = zero_of(V());
+    V rn[3], dz[3];
+    if (!CUBE) slot_dinv<CUBE>(i, dz);
+    double zr[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const int o = c * ntot + i;
-      const V rn = mad(nal, QS ? q_[3 * i + c] : q[j][c], r[j][c]);
+      rn[c] = mad(nal, QS ? q_[3 * i + c] : q[j][c], r[j][c]);
       const V dx = al * p[3 * i + c];
-      MT::st(rg + o, rn);
+      MT::st(rg + o, rn[c]);
       if (first)
         MT::st(xg + o, dx);
       else
         MT::add(xg + o, dx);  // (no value back: nothing waits for it)
-      if constexpr (QS) q_[3 * i + c] = rn;
-      sz = mad(rn, dz[c] * rn, sz);
-      sr = mad(rn, rn, sr);
+      if constexpr (QS) q_[3 * i + c] = rn[c];
+      if (!CUBE) zr[c] = MT::dot(dz[c] * rn[c], rn[c]);
     }
-    vz += MT::sum(sz);
-    vr += MT::sum(sr);
+    double s2[2];  // r.r of the slot's one or two planes
+    MT::squares(rn, s2);
+    vr += s2[0] + s2[1];
+    if (CUBE) {  // the components' diagonal is the same: r.z from the squares
+      const unsigned cv = mcnt()[i];
+      vz += sh.dl64[cv & 15u][0] * s2[0];
+      if (!MT::F64) vz += sh.dl64[cv >> 4][0] * s2[1];
+    } else {
+      vz += zr[0] + zr[1] + zr[2];
+    }
   }
 }
 

@@ -155,3 +155,39 @@ def test_parallel_launches_captured_in_a_graph():
         assert np.array_equal(out, direct)
     del g
     b.close()
+
+
+@pytest.mark.parametrize("length,E,strain", [(1.0, 1e9, 1e-14), (1.0, 1e9, 1e-18),
+                                             (1e-6, 1e9, 1e-6), (1e-6, 1e9, 1e-10),
+                                             (1e-9, 1.0, 1e-3)])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_units_do_not_matter(periodic, length, E, strain):
+    """Small strains, lengths and moduli: the squared residuals that steer the
+    FP32 corrections are far below the smallest FP32 number.  The stress of a
+    linear RVE scales with E and the strain and not with its size, so the
+    oracle solves the RVE of unit length."""
+    from oracle import periodic as PER
+    rng = np.random.default_rng(31)
+    meshes = [(4, 4, 4), (7, 5, 6), (8, 8, 5)] if periodic else [(4, 4, 4), (7, 5, 6), (17, 24, 7)]
+    descs, ets, refs = [], [], []
+    eps = rng.normal(0, 1.0, (len(meshes), 2, 6))
+    for i, n in enumerate(meshes):
+        ln = [v / 8.0 for v in n]
+        nu = (0.3, 0.22)
+        descs.append(mb.rve_desc(n, 0.2, (E, 30 * E), nu, [v * length for v in ln]))
+        ets.append((rng.random(n[0] * n[1] * n[2]) < 0.4).astype(np.uint8))
+        m = O.mesh(3, [v + 1 for v in n], ln)
+        if periodic:
+            st = PER.homogenize_periodic(m, ets[i], (1.0, 30.0), nu, eps[i])[1]
+        else:
+            st = O.homogenize(m, ets[i], (1.0, 30.0), nu, eps[i], rtol=1e-12, lin_rtol=1e-13)[1]
+        refs.append(np.asarray(st) * E * strain)
+    b = mb.Batch(descs, nrhs=2, rtol=1e-10, threads=512, ctas_per_sm=1,
+                 bc=mb.SP_BC_PERIODIC if periodic else mb.SP_BC_AFFINE)
+    for i, et in enumerate(ets):
+        b.set_etype(i, et)
+    stress, _, info = b.homogenize(np.ascontiguousarray(eps * strain))
+    inf = mb.info_array(info)
+    assert (inf["status"] == 0).all() and (inf["relres"] <= 1e-10).all(), inf
+    for i, ref in enumerate(refs):
+        assert np.abs(stress[i] - ref).max() <= 1e-8 * np.abs(ref).max(), meshes[i]

@@ -415,3 +415,32 @@ def test_request_that_misses_in_some_load_cases_is_kept(n):
         assert np.abs(np.array(tg).reshape(6, 6) - Cm).max() <= 2e-7 * np.abs(Cm).max()
     s.stop()
     s.close()
+
+
+@pytest.mark.parametrize("scale,strain", [(1.0, 1e-14), (1.0, 1e-18), (1e-6, 1e-10)])
+@pytest.mark.parametrize("warm", [mb.SP_WARM_PREDICT, mb.SP_WARM_LAST])
+def test_small_strains_and_lengths(warm, scale, strain):
+    """Strains at the round-off level of an unloaded point, and edges of
+    micrometres in SI units: the residual norms that steer CG are squares far
+    below the smallest FP32 number.  One geometry of each place the vectors
+    may lie in."""
+    D = []
+    for n in ((6, 6, 6), (24, 20, 20), (31, 32, 9)):
+        D.append(mb.rve_desc(n, 0.2, (1e9, 2e10), (0.3, 0.2), list(np.array(n) / 8.0)))
+    Cs = exact_tangents(D)
+    for d in D:
+        for k in range(3):
+            d.len[k] *= scale
+        d.radius *= scale
+    rng = np.random.default_rng(12)
+    s = mb.Server(D, warm_start=warm)
+    s.start()
+    for g in (0, 1, 2, 0, 1, 2):
+        e = rng.normal(0, strain, 6)
+        st, tg, info = s.wait(s.submit(g, e))
+        assert info.status == 0 and info.relres <= 1e-8
+        ref = Cs[g] @ e
+        assert np.abs(st - ref).max() <= 2e-8 * np.abs(ref).max()
+        assert np.abs(np.array(tg).reshape(6, 6) - Cs[g]).max() <= 2e-7 * np.abs(Cs[g]).max()
+    s.stop()
+    s.close()
