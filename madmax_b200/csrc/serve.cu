@@ -880,6 +880,13 @@ static bool unclaimed(const sp_server *s, const ServeDev &z) {
   return tickets(s, z) < s->tail * (s->modes ? SERVE_NRHS : 1);
 }
 
+// the state an ended loop left
+static int loop_state(sp_server *s, ServeDev *z) {
+  SP_CUDA_TRY(cudaMemcpy(z, s->d_dev, sizeof(*z), cudaMemcpyDeviceToHost));
+  if (z->lost) return sp_set_error(SP_ERR_TIMEOUT, "serving loop: a load case was given up");
+  return SP_OK;
+}
+
 static int server_launch(sp_server *s) {
   // reset the liveness flags, keep the claim and device counters
   ServeDev z;
@@ -916,7 +923,7 @@ static int server_keepalive(sp_server *s) {
   if (q != cudaSuccess) return sp_set_error(SP_ERR_CUDA, "serving loop failed: %s", cudaGetErrorString(q));
   if (s->h_ctl->stop) return SP_OK;
   ServeDev z;
-  SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
+  SP_TRY(loop_state(s, &z));
   if (unclaimed(s, z)) return server_launch(s);
   return SP_OK;
 }
@@ -991,7 +998,7 @@ extern "C" int sp_server_stop(sp_server *s) {
   if (e) return sp_set_error(SP_ERR_CUDA, "serving loop: %s", cudaGetErrorString(e));
   // requests published after the loop saw stop: run them to completion
   ServeDev z;
-  SP_CUDA_TRY(cudaMemcpy(&z, s->d_dev, sizeof(z), cudaMemcpyDeviceToHost));
+  SP_TRY(loop_state(s, &z));
   if (unclaimed(s, z)) {
     s->h_ctl->stop = 0;
     SP_TRY(server_launch(s));

@@ -60,7 +60,7 @@ struct ServeDev { // device memory
   volatile long long dtail;
   volatile int dstop;
   volatile int dispatcher_gone;
-  int err;
+  int lost;  // 1: a worker gave up a ticket, whose load case stays unsolved
 };
 
 // A request in the element-mode loop: its load cases are tasks of their own

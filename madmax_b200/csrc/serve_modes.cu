@@ -26,6 +26,7 @@
 // serve_internal.h); a task's time is a seventh of a request's, so a burst
 // ends without a long last request.
 #include "serve_internal.h"
+#include "serve_ticket.h"
 
 namespace sp {
 
@@ -63,32 +64,26 @@ __device__ __forceinline__ double serve_predict(const double *st, int n, const d
 }
 
 // Claim the next load case; one thread.  When work is published a CTA takes
-// the next ticket and keeps it: another may have taken the last published one
-// in between, so it waits for its own to be published.  (With a compare-and-
-// swap on the counter the CTAs of the die far from it lost every race: half of
-// them served nothing, and three passes over 6,912 points with n = 12 RVEs took
-// 38.4 ms instead of 17.6 ms.)  The wait ends with the
-// dispatcher, after its last publication; its own bound, 8 times the
-// dispatcher's since the last publication, is a safeguard (a ticket given up
-// while the dispatcher runs would leave its load case unsolved).
+// the next ticket and keeps it (serve_ticket.h): another may have taken the
+// last published one in between, so it waits for its own to be published.
+// (With a compare-and-swap on the counter the CTAs of the die far from it lost
+// every race: half of them served nothing, and three passes over 6,912 points
+// with n = 12 RVEs took 38.4 ms instead of 17.6 ms.)
 __device__ __noinline__ void serve_claim(const ServeModes &P, ServeShared &S) {
   ServeDev *D = P.dev;
-  long long task = -1, ticket = -1, idle = 0, seen = -1;
+  ServeWait wait;
+  long long task;
   for (;;) {
-    const bool last = D->dstop || D->dispatcher_gone || ++idle > 8LL * P.idle_limit;
+    const bool gone = D->dstop || D->dispatcher_gone;
     __threadfence();
-    const long long end = D->dtail * SERVE_NRHS;
-    if (end != seen) idle = 0;
-    seen = end;
-    if (ticket < 0 && (long long)*(volatile unsigned long long *)&D->claim < end)
-      ticket = (long long)atomicAdd(&D->claim, 1ull);
-    if (ticket >= 0 && ticket < end) {
-      task = ticket;
-      break;
-    }
-    if (last) break;
+    task = serve_poll(
+        wait, gone, D->dtail * SERVE_NRHS, P.idle_limit,
+        [&] { return (long long)*(volatile unsigned long long *)&D->claim; },
+        [&] { return (long long)atomicAdd(&D->claim, 1ull); });
+    if (task != SERVE_WAIT) break;
     __nanosleep(500);
   }
+  if (task == SERVE_LOST) atomicExch(&D->lost, 1);
   __threadfence();
   S.req = task < 0 ? -1 : task / SERVE_NRHS;
   if (task < 0) return;
