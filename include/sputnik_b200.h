@@ -222,8 +222,9 @@ typedef struct {
   int tune;          /* with threads, ctas_per_sm 0 and cluster 1: SP_TUNE_AUTO (default)
                         times every instantiated CTA shape (threads x CTAs per SM, i.e.
                         registers per thread) on a sample of the batch at create time and
-                        keeps the fastest, cached per device, kernel, precision, load cases
-                        and dominant mesh size; SP_TUNE_OFF takes the fixed defaults (512 x 1
+                        keeps the fastest, cached per device, kernel, precision, load cases,
+                        dominant mesh size and share of the work in the element modes' range
+                        (below); SP_TUNE_OFF takes the fixed defaults (512 x 1
                         for the stencil, 512 x 2 for the assembled operator).  Stencil
                         solves at 512 x 1 run in element modes, in CTAs chosen by each
                         RVE's size, where its mesh is in their range (2 to 32 layers, at

@@ -185,7 +185,10 @@ static std::vector<Shape> tune_candidates(const sp_batch_opts &o) {
   return {{512, 1, 1, kop}, {512, 2, 1, kop}, {256, 2, 1, kop}, {256, 4, 1, kop}};
 }
 
-using TuneKey = std::array<int, 5>;  // device, kernel operator, precision, load cases, size class
+// device, kernel operator, precision, load cases, size class, quarters of the
+// work in the element modes' range.  With the stencil the load cases are the
+// batch's own (tasks of the element modes), else those of the kernel.
+using TuneKey = std::array<int, 6>;
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneRecord> g_tune_cache;
 
@@ -523,9 +526,12 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
   bool trial = false;
   if (tune && !rc) {
     std::map<int, double> by_edge;
+    double all = 0.0, modal = 0.0;
     for (int i = 0; i < nrve; i++) {
       const MeshGeo &g = hplans[hrves[i].plan].geo;
       work[i] = rve_work(g);
+      all += work[i];
+      if (b->cls[i] >= 0) modal += work[i];
       by_edge[std::max(g.nex, std::max(g.ney, g.nez))] += work[i];
     }
     int dom = 0;
@@ -535,7 +541,9 @@ extern "C" int sp_batch_create(int nrve, const sp_rve_desc *descs, const sp_batc
         wmax = kv.second;
         dom = kv.first;
       }
-    tkey = {d->id, kernel_op(o), o.precision, kp, dom};
+    const bool st = o.op == SP_OP_STENCIL;
+    tkey = {d->id, kernel_op(o), o.precision, st ? nrhs : kp, dom,
+            st ? (int)std::lround(4.0 * modal / all) : 0};
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
       auto it = g_tune_cache.find(tkey);

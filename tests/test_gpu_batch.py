@@ -367,3 +367,17 @@ def test_batch_launch_captured_in_a_cuda_graph():
     for i in (0, 3):
         st = oracle_stress(descs[i], np.eye(6))
         assert np.abs(direct[i] - st).max() <= 1e-8 * np.abs(st).max()
+
+
+def test_tuned_shape_is_kept_for_one_kind_of_batch():
+    """The element modes take an RVE by its layers and columns, and a load case
+    at a time: a shape timed on RVEs beyond their range, or with another number
+    of load cases, is not taken over by a batch of the same largest edge."""
+    out = mb.rve_desc((33, 33, 33), 0.2, (1e9, 2e10), (0.3, 0.2), [33 / 8.0] * 3)
+    ins = mb.rve_desc((33, 8, 8), 0.2, (1e9, 2e10), (0.3, 0.2), [33 / 8.0, 1.0, 1.0])
+    seen = []
+    for d, k in ((out, 2), (ins, 2), (ins, 2), (ins, 5), (out, 2)):
+        b = mb.Batch([d] * 3, nrhs=k, rtol=1e-6)
+        seen.append(b.tune_report()["from_cache"])
+        b.close()
+    assert seen == [False, False, True, False, True]
