@@ -31,6 +31,7 @@ int device(Device **out) {
       return sp_set_error(SP_ERR_CUDA, "device %d is sm_%d%d; this build targets sm_100a", t_dev,
                           prop.major, prop.minor);
     d.nsm = prop.multiProcessorCount;
+    SP_CUDA_TRY(cudaEventCreateWithFlags(&d.alone, cudaEventDisableTiming));
     SP_CUDA_TRY(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
     d.id = t_dev;
   }

@@ -389,7 +389,7 @@ static int plain_launch(sp_rve *r, Device *d, cudaStream_t s, bool *taken) {
   *taken = false;
   const MeshGeo &g = r->g;
   const long long ni = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  if (ni < 1 || d->loops.load() > 0) return SP_OK;
+  if (ni < 1) return SP_OK;
   const int nb = (int)std::min<long long>(d->nsm, (ni + PLAIN_NT / 32 - 1) / (PLAIN_NT / 32));
   const size_t vec = (size_t)((ni + nb - 1) / nb) * 3 * K * sizeof(double), room = 200 * 1024;
   if (vec > room) return SP_OK;
@@ -399,10 +399,14 @@ static int plain_launch(sp_rve *r, Device *d, cudaStream_t s, bool *taken) {
   SP_CUDA_TRY(cudaFuncSetAttribute((const void *)k_plain_pcg<K>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
   void *args[] = {&P};
-  SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain_pcg<K>, dim3(nb), dim3(PLAIN_NT),
-                                          args, P.onchip ? 4 * vec : vec, s));
-  *taken = true;
-  return SP_OK;
+  return d->gate.launch_alone(
+      [&]() -> int {
+        SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain_pcg<K>, dim3(nb),
+                                                dim3(PLAIN_NT), args, P.onchip ? 4 * vec : vec, s));
+        SP_CUDA_TRY(cudaEventRecord(d->alone, s));
+        return SP_OK;
+      },
+      taken);
 }
 
 static int rve_assemble(sp_rve *r, Device *d, cudaStream_t s) {

@@ -896,12 +896,16 @@ static int server_launch(sp_server *s) {
   z.dispatcher_gone = 0;
   SP_CUDA_TRY(cudaMemcpyAsync(s->d_dev, &z, sizeof(z), cudaMemcpyHostToDevice, s->stream));
   SP_CUDA_TRY(cudaStreamSynchronize(s->stream));
-  if (s->modes)
-    kServeClasses[s->cls].fn<<<s->grid, kServeClasses[s->cls].threads, s->M.dyn, s->stream>>>(s->M);
-  else
-    serve_kernel(s->o)<<<s->grid, SERVE_NT, serve_dyn_smem(s->o), s->stream>>>(s->P);
-  SP_CUDA_TRY(cudaGetLastError());
-  if (!s->running) s->device->loops++;
+  auto launch = [&]() -> int {
+    SP_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->device->alone, 0));
+    if (s->modes)
+      kServeClasses[s->cls].fn<<<s->grid, kServeClasses[s->cls].threads, s->M.dyn, s->stream>>>(s->M);
+    else
+      serve_kernel(s->o)<<<s->grid, SERVE_NT, serve_dyn_smem(s->o), s->stream>>>(s->P);
+    SP_CUDA_TRY(cudaGetLastError());
+    return SP_OK;
+  };
+  SP_TRY(s->running ? launch() : s->device->gate.start_loop(launch));
   s->running = 1;
   s->launches++;
   return SP_OK;
@@ -994,7 +998,7 @@ extern "C" int sp_server_stop(sp_server *s) {
   std::atomic_thread_fence(std::memory_order_seq_cst);
   cudaError_t e = cudaStreamSynchronize(s->stream);
   s->running = 0;
-  s->device->loops--;
+  s->device->gate.stop_loop();
   if (e) return sp_set_error(SP_ERR_CUDA, "serving loop: %s", cudaGetErrorString(e));
   // requests published after the loop saw stop: run them to completion
   ServeDev z;
@@ -1006,7 +1010,7 @@ extern "C" int sp_server_stop(sp_server *s) {
     std::atomic_thread_fence(std::memory_order_seq_cst);
     e = cudaStreamSynchronize(s->stream);
     s->running = 0;
-    s->device->loops--;
+    s->device->gate.stop_loop();
     if (e) return sp_set_error(SP_ERR_CUDA, "serving loop: %s", cudaGetErrorString(e));
   }
   return SP_OK;

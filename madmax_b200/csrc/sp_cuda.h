@@ -5,10 +5,10 @@
 
 #include <cuda_runtime.h>
 
-#include <atomic>
 #include <cstddef>
 #include <cstdint>
 
+#include "loop_gate.h"
 #include "rve_device.cuh"
 #include "sp_internal.h"
 
@@ -32,7 +32,8 @@ struct Device {
   int id = -1;
   int nsm = 0;
   cudaStream_t stream = nullptr; // library stream (non-blocking)
-  std::atomic<int> loops{0};     // serving loops started and not stopped
+  LoopGate gate;                 // serving loops started and not stopped
+  cudaEvent_t alone = nullptr;   // the last launch through gate.launch_alone
 };
 
 // Current device of the calling thread, initialised on first use.
