@@ -383,7 +383,8 @@ struct sp_rve_s {
 // for, at most one each; a serving loop on the device may hold some of them
 // for as long as requests come, so beside one the graph of small kernels runs.
 // p has to fit the blocks' shared memory (n <= 54 with 8 load cases); larger
-// RVEs stream the matrix from HBM either way.
+// RVEs stream the matrix from HBM either way.  Where the launch is refused (SMs
+// held by another process's partition, say) the graph runs too.
 template <int K>
 static int plain_launch(sp_rve *r, Device *d, cudaStream_t s, bool *taken) {
   *taken = false;
@@ -399,14 +400,20 @@ static int plain_launch(sp_rve *r, Device *d, cudaStream_t s, bool *taken) {
   SP_CUDA_TRY(cudaFuncSetAttribute((const void *)k_plain_pcg<K>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
   void *args[] = {&P};
-  return d->gate.launch_alone(
+  bool refused = false;
+  SP_TRY(d->gate.launch_alone(
       [&]() -> int {
-        SP_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_plain_pcg<K>, dim3(nb),
-                                                dim3(PLAIN_NT), args, P.onchip ? 4 * vec : vec, s));
-        SP_CUDA_TRY(cudaEventRecord(d->alone, s));
+        refused = cudaLaunchCooperativeKernel((const void *)k_plain_pcg<K>, dim3(nb), dim3(PLAIN_NT),
+                                              args, P.onchip ? 4 * vec : vec, s) != cudaSuccess;
+        if (!refused) SP_CUDA_TRY(cudaEventRecord(d->alone, s));
         return SP_OK;
       },
-      taken);
+      taken));
+  if (refused) {
+    cudaGetLastError();  // (an error that outlasts the launch comes back from the graph)
+    *taken = false;
+  }
+  return SP_OK;
 }
 
 static int rve_assemble(sp_rve *r, Device *d, cudaStream_t s) {
