@@ -372,7 +372,8 @@ __global__ void __launch_bounds__(PCG_THREADS)
 // The neighbour nodes of a matrix whose rows 3a, 3a + 1, 3a + 2 share one
 // list of whole nodes' columns (any order, empty slots last): [nrow/3][28],
 // -1 after the last, for the caller to free.  Null if the matrix is not of
-// this form (or without the memory): the row kernels take any matrix.
+// this form (or without the memory, as on the device): the row kernels take
+// any matrix.
 static int *node_lists(const int *cols, int nrow, int wp) {
   if (wp != SP_WP || nrow % 3 || nrow < NODE_MIN_ROWS) return nullptr;
   int *nbr = (int *)malloc((size_t)nrow / 3 * NODE_WP * sizeof(int));
@@ -552,8 +553,8 @@ extern "C" int sp_ell_upload(const ell_matrix *m, sp_ell_dev **out) {
     int *nbr = rc ? nullptr : node_lists(hc, a->nrow, a->wp);
     if (nbr) {
       const size_t nb = (size_t)a->nrow / 3 * NODE_WP * sizeof(int);
-      rc = dmalloc((void **)&a->nbr, nb, nullptr);
-      if (!rc && cudaMemcpy(a->nbr, nbr, nb, cudaMemcpyHostToDevice))
+      if (dmalloc((void **)&a->nbr, nb, nullptr) == SP_OK &&
+          cudaMemcpy(a->nbr, nbr, nb, cudaMemcpyHostToDevice))
         rc = sp_set_error(SP_ERR_CUDA, "sp_ell_upload: copy failed");
       free(nbr);
     }

@@ -1,6 +1,6 @@
-"""Calls that have another way when the driver refuses a launch: the refusal
-is an error code from a stand-in for the driver's entry point (preloaded in a
-child process), which launches nothing."""
+"""Calls that have another way when the driver refuses a launch or an
+allocation: the refusal is an error code from a stand-in for the driver's entry
+point (preloaded in a child process), which launches and allocates nothing."""
 import os
 import shutil
 import subprocess
@@ -38,6 +38,16 @@ static int my_coop(void *f, unsigned gx, unsigned gy, unsigned gz, unsigned bx, 
   return refuse_coop() ? 720 : coop(f, gx, gy, gz, bx, by, bz, sm, s, args);
 }
 
+static int (*alloc)(unsigned long long *, size_t);
+static int my_alloc(unsigned long long *p, size_t n) {
+  const char *bytes = getenv("REFUSE_BYTES");
+  if (bytes && n == strtoull(bytes, NULL, 10)) {
+    fprintf(stderr, "refused %zu bytes\n", n);
+    return 2;
+  }
+  return alloc(p, n);
+}
+
 static int my_proc(const char *, void **, int, unsigned long long, void *);
 static int (*proc)(const char *, void **, int, unsigned long long, void *);
 
@@ -50,6 +60,10 @@ static void *stand_in(const char *name, void *real) {
   if (!strcmp(name, "cuLaunchCooperativeKernel")) {
     *(void **)&coop = real;
     return (void *)my_coop;
+  }
+  if (!strcmp(name, "cuMemAlloc") || !strcmp(name, "cuMemAlloc_v2")) {
+    *(void **)&alloc = real;
+    return (void *)my_alloc;
   }
   return real;
 }
@@ -95,3 +109,30 @@ def test_plain_solve_without_cooperative_launches(tmp_path):
     """The graph of small kernels (three launches an iteration) solves it."""
     r = child(tmp_path, PLAIN, REFUSE_COOPERATIVE="1")
     assert "refused a cooperative launch" in r.stderr
+
+
+SPMV = """
+import ctypes as C
+import numpy as np
+import madmax_b200 as mb
+from oracle import oracle as O
+A = O.assemble(O.cube_mesh(13), np.zeros(13 ** 3, np.uint8), (1e9, 1e9), (0.3, 0.3))
+n, w = A.cols.shape
+B = mb.EllMatrix(n, n, w)
+B.cols[:], B.vals[:] = A.cols, A.vals
+h = mb._vp()
+mb.check(mb.lib().sp_ell_upload(C.byref(B.m), C.byref(h)), "sp_ell_upload")
+x = np.random.default_rng(2).standard_normal(n)
+y = np.zeros(n)
+mb.check(mb.lib().sp_ell_dev_mvp_host(h, mb.ptr(x), mb.ptr(y)), "sp_ell_dev_mvp_host")
+ref = A.mvp(x)
+assert np.abs(y - ref).max() <= 1e-13 * np.abs(ref).max()
+"""
+
+
+def test_upload_without_room_for_the_neighbour_lists(tmp_path):
+    """n = 13: 14^3 nodes with 28 neighbours of 4 bytes.  The row kernel takes
+    the matrix."""
+    n = 14 ** 3 * 28 * 4
+    r = child(tmp_path, SPMV, REFUSE_BYTES=str(n))
+    assert "refused %d bytes" % n in r.stderr
