@@ -468,14 +468,22 @@ static int serve_class(int ngeom, const sp_rve_desc *descs, const sp_server_opts
   return -1;
 }
 
-// strides of the element-mode loop's work spaces (doubles and 8-byte values)
-static void modes_strides(const sp_rve_desc &d, size_t *w, size_t *v, size_t *e) {
-  const ModesGeo G(d.n[0], d.n[1], d.n[2], false, false, 0);
-  auto up = [](size_t x) { return (x + 15) / 16 * 16; };
-  *w = std::max(*w, up((size_t)3 * G.wlen()));
-  *v = std::max(*v, up((size_t)3 * G.ntot));
-  *e = std::max(*e, up((size_t)6 * G.mz * G.nex));
-}
+// The work space of a CTA of the element-mode loop, in doubles: w, nv vectors
+// of v (r and x, and what is not on chip of q and p), shares across strips
+struct ModesSlot {
+  size_t w = 0, v = 0, e = 0;
+  int nv = 2;
+  void add(const sp_rve_desc &d, const ServeClass &k) {
+    const ModesGeo G(d.n[0], d.n[1], d.n[2], false, false, 0);
+    const int on = modes_onchip(make_geo(d.n, d.len), k.threads, k.dyn());
+    auto up = [](size_t x) { return (x + 15) / 16 * 16; };
+    w = std::max(w, up((size_t)3 * G.wlen()));
+    v = std::max(v, up((size_t)3 * G.ntot));
+    if (on < 2) e = std::max(e, up((size_t)6 * G.mz * G.nex));
+    nv = std::max(nv, 4 - on);
+  }
+  size_t bytes() const { return 8 * (w + nv * v + e); }
+};
 
 // device bytes a resident geometry holds (the assembled operator adds its
 // node-sliced FP32 values)
@@ -549,50 +557,63 @@ extern "C" void sp_server_opts_default(sp_server_opts *o) {
   o->warm_start = SP_WARM_PREDICT;
 }
 
-// `cls`: the element-mode class (in: the one to lay out; out: -1 where its two
-// stores a geometry do not fit a budget that the block-stencil loop fits)
+// `cls`: the element-mode class (in: the one the geometries allow; out: -1
+// where the budget leaves that loop fewer CTAs than the former one, whose
+// geometries hold one store instead of two: with the same CTAs the element
+// modes are the faster, with a few of them they are not).  What the former
+// loop does not fit is refused.
 static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_opts *o, int nsm,
                          int *cls, int *slots, size_t *total) {
-  size_t resident = 0, mw = 0, mv = 0, me = 0;
+  size_t resident[2] = {0, 0}, plans = 0;  // of the former loop, of the element modes
   for (int i = 0; i < ngeom; i++)
     for (int k = 0; k < 3; k++)
       if (descs[i].n[k] < 1 || descs[i].len[k] <= 0)
         return sp_set_error(SP_ERR_ARG, "geometry %d: bad mesh", i);
-  const bool modes = *cls >= 0;
   std::map<std::vector<int>, int> seen;
   int maxnp = 0;
+  ModesSlot mslot;
   for (int i = 0; i < ngeom; i++) {
     const sp_rve_desc &d = descs[i];
-    if (modes) modes_strides(d, &mw, &mv, &me);
-    resident += geom_bytes(d, o->op, modes);
+    resident[0] += geom_bytes(d, o->op, false);
+    if (*cls >= 0) {
+      resident[1] += geom_bytes(d, o->op, true);
+      mslot.add(d, kServeClasses[*cls]);
+    }
     std::vector<int> key(d.n, d.n + 3);
     if (!seen.count(key)) {
       seen[key] = 1;
-      resident += plan_bytes(d.n);
+      plans += plan_bytes(d.n);
     }
     maxnp = std::max(maxnp, ((d.n[0] + 1) * (d.n[1] + 1) * (d.n[2] + 1) + 31) / 32 * 32);
   }
-  const size_t slot = modes ? 8 * (mw + 4 * mv + me) : (size_t)SERVE_K * 3 * maxnp * (8 + 4 * 4);
-  const int per_sm = modes            ? kServeClasses[*cls].ctas
-                     : o->ctas_per_sm ? o->ctas_per_sm
-                                      : (o->op == SP_OP_STENCIL ? 1 : 2);
-  int want = nsm * per_sm - 1;
-  // a slot solves a request, or one of its load cases
-  const long long inflight = (long long)o->max_inflight * (modes ? SERVE_NRHS : 1);
-  if (inflight > 0 && inflight < want) want = (int)inflight;
-  size_t budget = o->hbm_budget ? o->hbm_budget : (size_t)150e9;
-  if (modes && resident + 2 * slot > budget) {
-    *cls = -1;
-    return server_layout(ngeom, descs, o, nsm, cls, slots, total);
-  }
-  if (resident + slot > budget)
-    return sp_set_error(SP_ERR_BUDGET, "geometries need %zu bytes, budget %zu", resident + slot,
+  resident[0] += plans;
+  resident[1] += plans;  // (the request rings are beside the budget)
+  const size_t budget = o->hbm_budget ? o->hbm_budget : (size_t)150e9;
+  // HBM admission: as many concurrent slots (CTAs) as the budget allows.  A slot
+  // solves a request, or one of its load cases.
+  auto fit = [&](size_t res, size_t slot, int per_sm, long long inflight) {
+    long long want = (long long)nsm * per_sm - 1;
+    if (inflight > 0 && inflight < want) want = inflight;
+    return std::min(want, (long long)((budget - res) / slot));
+  };
+  const size_t slot = (size_t)SERVE_K * 3 * maxnp * (8 + 4 * 4);
+  if (resident[0] + slot > budget)
+    return sp_set_error(SP_ERR_BUDGET, "geometries need %zu bytes, budget %zu", resident[0] + slot,
                         budget);
-  // HBM admission: as many concurrent request slots as the budget allows
-  size_t fit = (budget - resident) / slot;
-  if ((size_t)want > fit) want = (int)fit;
-  *slots = want;
-  *total = resident + (size_t)(want + 1) * slot;
+  const int per_sm = o->ctas_per_sm ? o->ctas_per_sm : (o->op == SP_OP_STENCIL ? 1 : 2);
+  *slots = (int)fit(resident[0], slot, per_sm, o->max_inflight);
+  *total = resident[0] + (size_t)(*slots + 1) * slot;
+  if (*cls < 0) return SP_OK;
+  long long m = 0;
+  const size_t own = resident[1] + mslot.bytes();  // with the dispatcher's
+  if (own < budget)
+    m = fit(own, mslot.bytes(), kServeClasses[*cls].ctas, (long long)o->max_inflight * SERVE_NRHS);
+  if (m < 1 || m < *slots) {
+    *cls = -1;
+    return SP_OK;
+  }
+  *slots = (int)m;
+  *total = resident[1] + (size_t)(m + 1) * mslot.bytes();
   return SP_OK;
 }
 
@@ -660,7 +681,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   s->grid = slots + 1; // + dispatcher
   s->cls = cls;
   s->modes = s->cls >= 0;
-  size_t mw = 0, mv = 0, me = 0;
+  ModesSlot ms;
   int rc = server_grid(s, d);
   std::map<std::vector<int>, DevPlan *> pm;
   std::vector<double> mats((size_t)ngeom * 4);
@@ -694,7 +715,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
                     72 * 8, 144 * 8, (SERVE_K * (3 * np + 6) + 36) * 8};
     const ModesGeo mg(dd.n[0], dd.n[1], dd.n[2], false, false, 0);
     if (s->modes) {
-      modes_strides(dd, &mw, &mv, &me);
+      ms.add(dd, kServeClasses[s->cls]);
       sz[6] = (2 * store_len(mg) + 36) * 8;
     }
     for (int k = 0; k < 7 && !rc; k++) {
@@ -748,7 +769,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
   if (!rc && !s->modes) rc = dmalloc((void **)&s->ws_u, (size_t)s->grid * s->stride * 8, &s->bytes);
   if (!rc && !s->modes) rc = dmalloc((void **)&s->ws_v, (size_t)s->grid * 4 * s->stride * 4, &s->bytes);
   if (!rc && s->modes) {
-    const size_t sz[3] = {mw, 4 * mv, me};
+    const size_t sz[3] = {ms.w, ms.nv * ms.v, ms.e};
     for (int k = 0; k < 3 && !rc; k++) rc = dmalloc(&s->ws_m[k], s->grid * sz[k] * 8, &s->bytes);
     if (!rc) rc = dmalloc((void **)&s->d_jobs, (size_t)s->cap * sizeof(ServeJob), &s->bytes);
   }
@@ -829,8 +850,7 @@ extern "C" int sp_server_create(int ngeom, const sp_rve_desc *descs, const sp_se
     M.res = s->d_res_map;
     M.ctl = s->d_ctl_map;
     M.dev = s->d_dev;
-    M.buf = ModesBufs{(double *)s->ws_m[0], s->ws_m[1], s->ws_m[2], mw, mv, me,
-                      4 * mv};
+    M.buf = ModesBufs{(double *)s->ws_m[0], s->ws_m[1], s->ws_m[2], ms.w, ms.v, ms.e, ms.nv * ms.v};
     // a request whose prediction misses rtol is solved tighter, so that the
     // predictions from its solutions meet rtol without a solve (a start from
     // the last solutions is solved to rtol)

@@ -260,3 +260,33 @@ def test_solvers_header_includes_slepc_under_dslepc(tmp_path):
     no = subprocess.run(["gcc", "-std=gnu11", "-fsyntax-only"] + inc + [str(src)],
                         capture_output=True, text=True)
     assert no.returncode != 0 and "EPS" in no.stderr
+
+
+@pytest.mark.parametrize("sizes", [(8, 12, 16, 20), (6,) * 50, (12,) * 400, (24, 32)])
+def test_tight_budgets_keep_the_slots_of_the_former_loop(sizes):
+    """The element-mode loop holds two stores a geometry, the former loop one.
+    Where the budget leaves it fewer CTAs than the former loop's request slots,
+    the former loop is laid out, with as many slots as ever; what that does not
+    fit is refused.  (Two slots per SM ask for the former loop.)"""
+    descs = (mb.sp_rve_desc * len(sizes))(*[mb.rve_desc(n) for n in sizes])
+
+    def plan(**kw):
+        b = C.c_size_t()
+        o = mb.server_opts(**kw)
+        return mb.lib().sp_server_plan_bytes(len(sizes), descs, C.byref(o), C.byref(b)), b.value
+
+    def sizes_of(per_request, **kw):  # resident bytes and bytes a slot
+        one, two = (plan(max_inflight=k, **kw)[1] for k in (1, 2))
+        slot = (two - one) // per_request
+        return one - (per_request + 1) * slot, slot
+
+    old, oslot = sizes_of(1, ctas_per_sm=2)
+    new, nslot = sizes_of(7)
+    for slots in range(1, 148):
+        budget = old + slots * oslot + oslot // 2
+        rc, total = plan(hbm_budget=budget)
+        assert rc == 0
+        if total != old + (slots + 1) * oslot:
+            assert total <= budget and (total - new) // nslot - 1 >= slots, slots
+    assert plan(hbm_budget=old + oslot - 1)[0] == mb.SP_ERR_BUDGET
+    assert plan()[1] >= new + 148 * nslot
