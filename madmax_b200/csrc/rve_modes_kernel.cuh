@@ -1122,7 +1122,8 @@ __device__ __noinline__ inline void modes_report(const sp_solve_info &in, sp_sol
       if (c->status > all.status) all.status = c->status;
       if (c->outer_its > all.outer_its) all.outer_its = c->outer_its;
       if (c->inner_its > all.inner_its) all.inner_its = c->inner_its;
-      all.relres = fmax(all.relres, c->relres);
+      const double r = c->relres;
+      if (!isnan(all.relres) && !(r <= all.relres)) all.relres = r;  // (NaN is the worst)
     }
     *out = all;
     *done = 0;

@@ -191,3 +191,23 @@ def test_units_do_not_matter(periodic, length, E, strain):
     assert (inf["status"] == 0).all() and (inf["relres"] <= 1e-10).all(), inf
     for i, ref in enumerate(refs):
         assert np.abs(stress[i] - ref).max() <= 1e-8 * np.abs(ref).max(), meshes[i]
+
+
+@pytest.mark.parametrize("k", [0, 2])
+def test_breakdown_is_reported(k):
+    """A strain whose forces leave FP32's range breaks its load case down: the
+    RVE reports the residual that is not a number, whichever load case has it;
+    the other RVE is solved."""
+    descs = [mb.rve_desc(5, 0.3, (1e9, 2e10)), mb.rve_desc(4, 0.3, (1e9, 2e10))]
+    eps = np.random.default_rng(2).normal(0, 1e-3, (2, 3, 6))
+    eps[0, k] *= 1e38
+    b = mb.Batch(descs, nrhs=3, threads=512, ctas_per_sm=1)
+    b.upload(np.ascontiguousarray(eps))
+    b.launch()
+    info = (mb.sp_solve_info * 2)()
+    b.download(np.zeros((2, 3, 6)), None, info)
+    import torch
+    torch.cuda.synchronize()
+    assert info[0].status == mb.SP_ERR_NOCONV and np.isnan(info[0].relres)
+    assert info[1].status == 0 and info[1].relres <= 1e-8
+    b.close()
