@@ -211,3 +211,41 @@ def test_breakdown_is_reported(k):
     assert info[0].status == mb.SP_ERR_NOCONV and np.isnan(info[0].relres)
     assert info[1].status == 0 and info[1].relres <= 1e-8
     b.close()
+
+
+@pytest.mark.parametrize("cube", [True, False])
+def test_periodic_fp64_edges(cube):
+    """FP64 under periodic conditions: odd and even planes, rows across warps,
+    the wide class, p and q or p alone on chip, and the first meshes past the
+    range, on random voxel materials.  The periodic oracle's direct solve, and for
+    the largest meshes the block stencil's FP64 batch; solves to 1e-10."""
+    from oracle import periodic as PER
+    rng = np.random.default_rng(53 + cube)
+    meshes = PER_MESHES + [(18, 17, 13), (20, 20, 16), (18, 18, 30), (20, 20, 20), (24, 20, 22)]
+    descs, ets, lens = [], [], []
+    for n in meshes:
+        edge = rng.uniform(0.05, 0.2, 3)
+        lens.append([n[k] / 8.0 if cube else n[k] * edge[k] for k in range(3)])
+        descs.append(mb.rve_desc(n, 0.2, (1e9, 1e9 * float(rng.uniform(2, 100))), (0.3, 0.25),
+                                 lens[-1]))
+        ets.append((rng.random(n[0] * n[1] * n[2]) < 0.4).astype(np.uint8))
+    eps = rng.normal(0, 1e-3, (len(descs), 2, 6))
+    out = []
+    for ctas in (1, 2):
+        b = mb.Batch(descs, nrhs=2, rtol=1e-10, bc=mb.SP_BC_PERIODIC, precision=mb.SP_PREC_FP64,
+                     threads=512, ctas_per_sm=ctas)
+        for i, et in enumerate(ets):
+            b.set_etype(i, et)
+        s, strain, info = b.homogenize(np.ascontiguousarray(eps))
+        inf = mb.info_array(info)
+        assert (inf["status"] == 0).all() and (inf["relres"] <= 1e-10).all()
+        assert np.allclose(strain, eps, rtol=0, atol=1e-14)
+        assert (b.last_launches() > 2) == (ctas == 1)
+        out.append(s)
+        b.close()
+    for i, n in enumerate(meshes):
+        ref = out[1][i]
+        if np.prod(n) <= 1500:
+            m = O.mesh(3, [v + 1 for v in n], lens[i])
+            ref = PER.homogenize_periodic(m, ets[i], tuple(descs[i].E), tuple(descs[i].nu), eps[i])[1]
+        assert np.abs(out[0][i] - ref).max() <= 1e-8 * np.abs(ref).max(), (n, cube)
