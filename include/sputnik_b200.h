@@ -67,7 +67,8 @@ typedef struct sp_ell_dev_s sp_ell_dev;
 int sp_ell_upload(const ell_matrix *m, sp_ell_dev **out);
 int sp_ell_dev_free(sp_ell_dev *a);
 /* y = A x with device pointers on `stream` (cudaStream_t, NULL = library
- * stream): one warp per row, 128-bit loads.  Result within rounding of the
+ * stream): a warp per node for a matrix in node triples, else a part of a warp
+ * per row (see sp_ell_dev_set_lanes).  Result within rounding of the
  * reference's ell_mvp (src/ell.c:127-141). */
 int sp_ell_dev_mvp(sp_ell_dev *a, const double *x_dev, double *y_dev, void *stream);
 /* Same with host vectors (copies in and out). */
@@ -77,11 +78,12 @@ int sp_ell_dev_mvp_host(sp_ell_dev *a, const double *x, double *y);
  * on the uploaded matrix and keeps the fastest (cached per device, row width
  * and row-count octave).  A tuning knob; the result does not depend on it
  * beyond rounding.  A matrix whose rows 3a..3a+2 share one list of whole
- * nodes' columns (every assembled RVE), of 6,000 rows or more, is multiplied a warp per node instead
- * while no width is set here. */
+ * nodes' columns (every assembled RVE), of 6,000 rows or more, is multiplied a
+ * warp per node instead while no width is set here (and the device has room
+ * for its neighbour lists). */
 int sp_ell_dev_set_lanes(sp_ell_dev *a, int lanes);
-/* The lanes per row sp_ell_dev_mvp uses, the upload-time trial's time per
- * launch at 4, 8, 16 and 32 lanes (microseconds; trial_us may be NULL) and
+/* The lanes per row sp_ell_dev_mvp uses where it goes by rows, the
+ * upload-time trial's time per launch at 4, 8, 16 and 32 lanes (microseconds; trial_us may be NULL) and
  * whether the choice came from the autotuner's cache.  No counterpart in the
  * reference (its ell_mvp is a serial row loop, src/ell.c:127-141). */
 int sp_ell_dev_lanes(const sp_ell_dev *a, int *lanes, float *trial_us, int *from_cache);
@@ -227,8 +229,10 @@ typedef struct {
                         (below); SP_TUNE_OFF takes the fixed defaults (512 x 1
                         for the stencil, 512 x 2 for the assembled operator).  Stencil
                         solves at 512 x 1 run in element modes, in CTAs chosen by each
-                        RVE's size, where its mesh is in their range (2 to 32 layers, at
-                        most 1024 columns of elements).  A tuned
+                        RVE's size, where its mesh is in their range: 2 elements an axis
+                        or more, at most 32 layers and 1024 columns of elements; under
+                        periodic conditions 30 layers, 640 columns and p in one SM's
+                        shared memory (about 24^3 elements, in FP64 about 20^3).  A tuned
                         batch's results do not depend on the launch, but the shape -- and so
                         the last bits of the sums -- may depend on the batch's composition;
                         fix threads and ctas_per_sm for bit-identical results across batches */
@@ -259,8 +263,10 @@ int sp_batch_device_bytes(const sp_batch *b, size_t *bytes);
  * materials[nrve][4] = (E_matrix, nu_matrix, E_fiber, nu_fiber) (NULL: from
  * the descriptors).  Host arrays should be pinned for asynchronous copies. */
 int sp_batch_upload(sp_batch *b, const double *strains, const double *materials, void *stream);
-/* One persistent launch: every RVE is assembled (coloured scatter into its
- * ELL), solved for all load cases to rtol and volume-averaged. */
+/* Solves every RVE for all load cases to rtol and averages over its volume:
+ * one persistent launch, or with element modes one for each size class present,
+ * in parallel on streams joined to `stream` (SP_OP_ELL: each RVE's values are
+ * assembled in the launch). */
 int sp_batch_launch(sp_batch *b, void *stream);
 /* Queue the device->host copy of the results: stress[nrve][nrhs][6],
  * strain[nrve][nrhs][6] (either may be NULL), info[nrve] (may be NULL). */

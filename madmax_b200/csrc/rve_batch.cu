@@ -237,7 +237,7 @@ struct sp_batch_s {
 
 // The shape whose stencil solves run the element-mode kernel: the default and
 // the shape the autotuner compares the others with (4096 RVEs of n = 8..20
-// 332 ms in k_batch, 118 ms in element modes).
+// 335 ms in k_batch, 121 ms in element modes).
 static bool uses_modes(const Shape &s) {
   return s.threads == 512 && s.ctas == 1 && s.cluster == 1 && s.op != SP_OP_ELL;
 }

@@ -1,5 +1,6 @@
-// rve_modes_kernel.cuh -- the batched FP32 stencil solve, one load case of
-// one RVE per CTA at a time, on the element-mode operator (rve_modes.cuh).
+// rve_modes_kernel.cuh -- the batched stencil solve, in FP32 corrections or in
+// FP64, one load case of one RVE per CTA at a time, on the element-mode operator
+// (rve_modes.cuh).
 //
 // The load cases of an RVE are independent systems.  Solved one by one, the
 // search direction p and the product q = A p of an RVE of up to about 20^3
@@ -12,16 +13,19 @@
 // u = eps.x + w (here marched in element modes too), FP32 Jacobi-PCG
 // corrections as reliable updates, w += x in FP64, volume averages in FP64.
 //
-// What bounds it: the march's serial chain over the planes (a barrier and the
-// shared-memory exchange per plane) with its shuffles and packed FP32 work,
-// ~27,000 cycles an application at n = 20 against ~12,000 of issue slots (n = 16:
-// issue slots 48%, L1 data pipe 64% busy, DRAM idle).  Small
-// RVEs hide it with several CTAs per SM (classes at the end of this file), so
-// a class is as small as threads and shared memory allow.  Measured against
-// the block stencil with all load cases in one CTA: 4096 RVEs of n = 8..20
-// 332 -> 118 ms, 1 RVE of n = 24 with 6 load cases 42 -> 5.5 ms (6 SMs instead
-// of 1), periodic 256 RVEs of n = 9..17 34 -> 4.9 ms, FP64 192 RVEs of n = 8..16
-// 21 -> 4.7 ms, 74 RVEs of n = 32 (no vector on chip) 206 -> 63 ms.
+// The scalars that steer CG are products formed and added in FP64 (ModesType::
+// dot): in FP32 they left the range with small strains, lengths or moduli.
+//
+// What bounds it: the march's serial chain over the planes, a barrier and the
+// shared-memory exchange per plane, with its shuffles and packed FP32 work (592
+// RVEs of n = 16: issue slots 48%, L1 data pipe 60%, FP64 pipe 8% busy, DRAM
+// idle).  Small RVEs hide it with several CTAs per SM (classes at the end of
+// this file), so a class is as small as threads and shared memory allow.
+// Measured against the block stencil with all load cases in one CTA, solves to
+// 1e-10: 4096 RVEs of n = 8..20 335 -> 121 ms, 1 RVE of n = 24 with 6 load cases
+// 38.0 -> 5.9 ms (6 SMs instead of 1), periodic 256 RVEs of n = 9..17 34.6 -> 5.1
+// ms, FP64 192 RVEs of n = 8..16 21.9 -> 5.0 ms, 74 RVEs of n = 32 (no vector on
+// chip) 206 -> 63 ms.  (With the scalars in FP32: 117, 5.6, 5.0, 4.9 ms.)
 #pragma once
 
 #include "rve_batch_kernel.cuh"
@@ -642,7 +646,7 @@ __device__ __noinline__ int march_average(const double *w, int ph) {
       modes_below<PER>(T.f, left, down);
       const unsigned c3 = sh.col[T.f], c2 = sh.col[T.f + left], c1 = sh.col[T.f + down],
                      c0 = sh.col[T.f + left + down];
-  #pragma unroll 4
+#pragma unroll 4
       for (int pl = 0; pl < mz; pl++) {
         const unsigned b0 = (c0 >> pl) & 3u, b1 = (c1 >> pl) & 3u, b2 = (c2 >> pl) & 3u,
                        b3 = (c3 >> pl) & 3u;
@@ -650,10 +654,10 @@ __device__ __noinline__ int march_average(const double *w, int ph) {
         const int lower = (b0 & 1) + (b1 & 1) + (b2 & 1) + (b3 & 1);
         const double k[3] = {(double)(n0 + n2 - n1 - n3), (double)(n0 + n1 - n2 - n3),
                              (double)(2 * lower - (n0 + n1 + n2 + n3))};
-  #pragma unroll
+#pragma unroll
         for (int c = 0; c < 3; c++) {
           const double v = w[c * wl + pl * nface + T.f];
-  #pragma unroll
+#pragma unroll
           for (int d = 0; d < 3; d++) m[3 * c + d] = fma(k[d], v, m[3 * c + d]);
         }
       }
@@ -826,18 +830,18 @@ __device__ __noinline__ void update_w(const typename ModesType<V>::Mem *xg, doub
   for (int y0 = 0; y0 < sh.ney; y0 += sh.rows) {
     const ModesLane<PER> T(y0);
     if (!T.owner) continue;
-  #pragma unroll 1
+#pragma unroll 1
     for (int s = 0; s < h; s++) {
       const int i = s * nface + T.f;
       V x[3];
       double w0[3], w1[3];
-  #pragma unroll
+#pragma unroll
       for (int c = 0; c < 3; c++) {
         x[c] = ModesType<V>::ld(xg + (c * ntot + i));
         w0[c] = w[c * wl + i];
         w1[c] = s + h < mz ? w[c * wl + i + h * nface] : 0.0;
       }
-  #pragma unroll
+#pragma unroll
       for (int c = 0; c < 3; c++) {
         if constexpr (ModesType<V>::F64) {
           w[c * wl + i] = w0[c] + x[c];
@@ -962,7 +966,7 @@ __device__ __noinline__ void modes_setup(const double *len, const double *mat,
       for (int s = 0; s < sh.h; s++)
         mcnt()[s * nface + T.f] = (uint8_t)(count(s) | (F64 ? 0 : count(s + sh.h) << 4));
       const double X = (T.f % nex) * sh.hx[0], Y = (T.f / nex) * sh.hx[1];
-  #pragma unroll
+#pragma unroll
       for (int c = 0; c < 3; c++) {
         const double xy = sh.E[3 * c] * X + sh.E[3 * c + 1] * Y, ez = sh.E[3 * c + 2] * sh.hx[2];
         if (!PER)
