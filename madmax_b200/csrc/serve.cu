@@ -558,10 +558,9 @@ extern "C" void sp_server_opts_default(sp_server_opts *o) {
 }
 
 // `cls`: the element-mode class (in: the one the geometries allow; out: -1
-// where the budget leaves that loop fewer CTAs than the former one, whose
-// geometries hold one store instead of two: with the same CTAs the element
-// modes are the faster, with a few of them they are not).  What the former
-// loop does not fit is refused.
+// where the budget leaves that loop fewer CTAs than match the former one's
+// slots, whose geometries hold one store instead of two).  What the former loop
+// does not fit is refused.
 static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_opts *o, int nsm,
                          int *cls, int *slots, size_t *total) {
   size_t resident[2] = {0, 0}, plans = 0;  // of the former loop, of the element modes
@@ -608,7 +607,7 @@ static int server_layout(int ngeom, const sp_rve_desc *descs, const sp_server_op
   const size_t own = resident[1] + mslot.bytes();  // with the dispatcher's
   if (own < budget)
     m = fit(own, mslot.bytes(), kServeClasses[*cls].ctas, (long long)o->max_inflight * SERVE_NRHS);
-  if (m < 1 || m < *slots) {
+  if (m < 1 || m < kServeClasses[*cls].match * *slots) {
     *cls = -1;
     return SP_OK;
   }

@@ -96,6 +96,7 @@ struct ServeModes {
 // cases in flight per SM; the last class also serves the larger ones.
 struct ServeClass {
   int threads, ctas;
+  double match;  // CTAs that serve at least as much as a slot of the former loop
   void (*fn)(const ServeModes);
   // dynamic shared memory of a CTA (static data and the driver's share apart)
   int dyn() const {

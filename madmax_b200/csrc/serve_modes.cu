@@ -356,10 +356,15 @@ __global__ void __launch_bounds__(NT, MINB) k_serve_modes(const __grid_constant_
 }
 
 // 128 registers a thread at every class; the shared memory of a CTA is the
-// SM's over its CTAs, so a class ends where p and q of a geometry no longer fit
-const ServeClass kServeClasses[SERVE_CLASSES] = {{64, 8, k_serve_modes<64, 8>},
-                                                 {160, 3, k_serve_modes<160, 3>},
-                                                 {256, 2, k_serve_modes<256, 2>},
-                                                 {512, 1, k_serve_modes<512, 1>}};
+// SM's over its CTAs, so a class ends where p and q of a geometry no longer fit.
+// Requests a second that a CTA serves, few of them at once, solved and
+// predicted, against a slot of the former loop (512 threads): n = 6 1,092 and
+// 5,470 against 2,037 and 7,380; n = 12 285 and 3,430 against 312 and 3,020;
+// n = 16 167 and 2,670 against 111 and 1,650; n = 20 80 and 1,910 against 48 and
+// 925; n = 28 11.4 and 663 against 10.5 and 362.
+const ServeClass kServeClasses[SERVE_CLASSES] = {{64, 8, 2.0, k_serve_modes<64, 8>},
+                                                 {160, 3, 1.1, k_serve_modes<160, 3>},
+                                                 {256, 2, 1.0, k_serve_modes<256, 2>},
+                                                 {512, 1, 1.0, k_serve_modes<512, 1>}};
 
 }  // namespace sp

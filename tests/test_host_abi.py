@@ -262,7 +262,8 @@ def test_solvers_header_includes_slepc_under_dslepc(tmp_path):
     assert no.returncode != 0 and "EPS" in no.stderr
 
 
-@pytest.mark.parametrize("sizes", [(8, 12, 16, 20), (6,) * 50, (12,) * 400, (24, 32)])
+@pytest.mark.parametrize("sizes", [(8, 12, 16, 20), (6,) * 50, (6,) * 1500, (12,) * 400,
+                                   (24, 32)])
 def test_tight_budgets_keep_the_slots_of_the_former_loop(sizes):
     """The element-mode loop holds two stores a geometry, the former loop one.
     Where the budget leaves it fewer CTAs than the former loop's request slots,
@@ -287,6 +288,8 @@ def test_tight_budgets_keep_the_slots_of_the_former_loop(sizes):
         rc, total = plan(hbm_budget=budget)
         assert rc == 0
         if total != old + (slots + 1) * oslot:
-            assert total <= budget and (total - new) // nslot - 1 >= slots, slots
+            # (a CTA of the class of n = 6 serves half as much as a slot)
+            least = 2 * slots if max(sizes) <= 7 else slots
+            assert total <= budget and (total - new) // nslot - 1 >= least, slots
     assert plan(hbm_budget=old + oslot - 1)[0] == mb.SP_ERR_BUDGET
     assert plan()[1] >= new + 148 * nslot
